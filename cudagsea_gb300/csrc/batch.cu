@@ -10,10 +10,11 @@
 //      family when all instances share a metric); in the plain form one
 //      launch per metric and kernel path (exact, or packed with 4 or 8
 //      permutations per thread);
-//   3. the sort: one launch per register-resident class (ITEMS keys per
-//      thread, one CTA or a two-CTA cluster per permutation); instances
-//      beyond the register forms (G > 40,960 fp32 / 20,480 fp64) sort on
-//      their own;
+//   3. the sort: one launch per bucket-sort class, then one per radix class
+//      (keys per thread, one CTA or a two-CTA cluster per permutation) for
+//      the permutations the bucket sort declined; instances beyond the
+//      register radix forms (G > 40,960 fp32 / 20,480 fp64) sort on their
+//      own;
 //   4. one persistent enrichment launch per size class (the bitmap words per
 //      lane of the register procedure, fixed by G): its CTAs pull
 //      (instance, permutation) items from a global counter, heaviest
@@ -70,7 +71,8 @@ struct gsea_batch_s {
     std::vector<Multi<gsea::ChosenTask>> chosen;
     std::vector<Multi<gsea::MetricTask<float>>> metric32;   // plain form
     std::vector<Multi<gsea::MetricTask<double>>> metric64;
-    std::vector<Multi<gsea::SortTask>> sorts;
+    std::vector<Multi<gsea::SortTask>> bucket_sorts;  // every instance's permutations first ...
+    std::vector<Multi<gsea::SortTask>> sorts;         // ... then those the bucket sorts declined
     std::vector<int64_t> solo_sort;   // instances sorted on their own (tiled sort)
     Multi<gsea::StatsTask<float>> stats32;
     Multi<gsea::StatsTask<double>> stats64;
@@ -121,6 +123,8 @@ void drop_classes(gsea_batch_s* b) {
     b->metric32.clear();
     for (auto& m : b->metric64) free_multi(m);
     b->metric64.clear();
+    for (auto& m : b->bucket_sorts) free_multi(m);
+    b->bucket_sorts.clear();
     for (auto& m : b->sorts) free_multi(m);
     b->sorts.clear();
     b->solo_sort.clear();
@@ -139,7 +143,7 @@ std::vector<Multi<gsea::MetricTask<T>>>& metric_groups(gsea_batch_s* b) {
 template <class T>
 int build_multi(gsea_batch_s* b, Multi<gsea::StatsTask<T>>& stats) {
     const bool fp64 = b->precision == 64;
-    std::map<int, size_t> chosen_at, sort_at, metric_at;
+    std::map<int, size_t> chosen_at, sort_at, bucket_at, metric_at;
     auto& metrics = metric_groups<T>(b);
     for (int64_t i = 0; i < (int64_t)b->plans.size(); i++) {
         gsea_plan_s* p = b->plans[i];
@@ -213,13 +217,20 @@ int build_multi(gsea_batch_s* b, Multi<gsea::StatsTask<T>>& stats) {
             st.G = (int)c.num_genes;
             st.num_perms = (int)c.num_perms;
             st.descending = c.ascending ? 0 : 1;
-            auto it = sort_at.find(cls);
-            if (it == sort_at.end()) {
-                it = sort_at.emplace(cls, b->sorts.size()).first;
-                b->sorts.emplace_back();
-                b->sorts.back().key = cls;
-            }
-            b->sorts[it->second].h.push_back(st);
+            st.cap = gsea::sort_bucket_cap(st.G);
+            st.hard = static_cast<uint8_t*>(p->sort_scratch) +
+                      (p->sort_scratch_bytes - gsea::sort_mark_bytes(st.num_perms));
+            auto add = [&](std::vector<Multi<gsea::SortTask>>& to, std::map<int, size_t>& at, int key) {
+                auto it = at.find(key);
+                if (it == at.end()) {
+                    it = at.emplace(key, to.size()).first;
+                    to.emplace_back();
+                    to.back().key = key;
+                }
+                to[it->second].h.push_back(st);
+            };
+            add(b->bucket_sorts, bucket_at, gsea::sort_bucket_multi_class(st.G));
+            add(b->sorts, sort_at, cls);
         }
         const int rows = gsea::stats_multi_rows<T>((int)c.num_sets, c.num_perms);
         if (rows <= 0) {
@@ -239,6 +250,8 @@ int build_multi(gsea_batch_s* b, Multi<gsea::StatsTask<T>>& stats) {
     for (auto& m : b->chosen)
         if (e == cudaSuccess) e = upload_multi(m);
     for (auto& m : metrics)
+        if (e == cudaSuccess) e = upload_multi(m);
+    for (auto& m : b->bucket_sorts)
         if (e == cudaSuccess) e = upload_multi(m);
     for (auto& m : b->sorts)
         if (e == cudaSuccess) e = upload_multi(m);
@@ -354,12 +367,15 @@ int record(gsea_batch_s* b) {
     };
     if ((rc = fork(ev[0]))) return rc;
     size_t lane = 0;
-    for (auto& m : b->sorts)
-        GSEA_CUDA(gsea::launch_sort_multi(m.d, (int)m.h.size(), m.key, fp64, b->streams[lane++ % ns]),
+    for (auto& m : b->bucket_sorts)
+        GSEA_CUDA(gsea::launch_sort_bucket_multi(m.d, m.h.data(), (int)m.h.size(), m.key, fp64,
+                                                 b->streams[lane++ % ns]),
                   "batched sort");
     for (int64_t i : b->solo_sort)
         if ((rc = gsea::plan_run_sort(b->plans[i], b->streams[lane++ % ns]))) return rc;
     if ((rc = join(ev + 1))) return rc;
+    for (auto& m : b->sorts)
+        GSEA_CUDA(gsea::launch_sort_multi(m.d, (int)m.h.size(), m.key, fp64, st), "batched sort");
     if ((rc = fork(ev[ns + 1]))) return rc;
     for (size_t ci = 0; ci < b->classes.size(); ci++) {
         const auto it = b->es_tuning.find(b->classes[ci].wpl);

@@ -46,11 +46,25 @@ template <class T> __device__ __forceinline__ T cuabs(T x) { return x < T(0) ? -
 // Radix order of IEEE keys: unsigned ascending order of radix_bits(x) equals
 // ascending value order with -0 < +0 and NaNs at the two ends, which is the
 // order CUB's radix sort gives the reference GPU path (batched_sort.cuh:144).
+// The bits are taken by a move the compiler does not look through: where the
+// value is used as a number too, it rewrites "sign bit set" as a negated
+// absolute value in floating point, which gives a NaN another sign (seen with
+// doubles: the key of a NaN differed from that of an equal NaN).
+__device__ __forceinline__ uint32_t bits_of(float f) {
+    uint32_t u;
+    asm("mov.b32 %0, %1;" : "=r"(u) : "f"(f));
+    return u;
+}
+__device__ __forceinline__ unsigned long long bits_of(double f) {
+    unsigned long long u;
+    asm("mov.b64 %0, %1;" : "=l"(u) : "d"(f));
+    return u;
+}
 template <class T> struct RadixKey;
 template <> struct RadixKey<float> {
     using U = uint32_t;
     static __device__ __forceinline__ U from(float f, bool descending) {
-        U u = __float_as_uint(f);
+        U u = bits_of(f);
         u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
         return descending ? ~u : u;
     }
@@ -58,7 +72,7 @@ template <> struct RadixKey<float> {
 template <> struct RadixKey<double> {
     using U = unsigned long long;
     static __device__ __forceinline__ U from(double f, bool descending) {
-        U u = (U)__double_as_longlong(f);
+        U u = bits_of(f);
         u = (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
         return descending ? ~u : u;
     }

@@ -1,4 +1,8 @@
-// k_sort.cu -- per-permutation stable ranking of genes by metric.
+// k_sort.cu -- per-permutation stable ranking of genes by metric: the
+// dispatch and the radix sorts.  Up to 65,535 genes the bucket sort of
+// k_sort_bucket.cu runs first and the radix sorts here take the permutations
+// it declined (`only`: one byte per permutation; a CTA none of whose
+// permutations is marked leaves after one look).
 //
 // Replaces pathway_sort_gpu (src/include/batched_sort.cuh:91-269), which runs
 // CUB's DeviceSegmentedRadixSort in descending order on (metric, gene id)
@@ -142,6 +146,16 @@ __device__ __forceinline__ void tile_offsets(uint32_t (*cnt)[256], uint32_t (*qs
     __syncthreads();
 }
 
+// none of the permutations first, first + stride, ... is marked in `only`
+// (the same answer in every thread; a null list marks all of them)
+__device__ __forceinline__ bool none_marked(const uint8_t* __restrict__ only, int first, int stride, int num_perms) {
+    if (!only) return false;
+    int any = 0;
+    for (int64_t p = first + (int64_t)threadIdx.x * stride; p < num_perms; p += (int64_t)kThreads * stride)
+        any |= only[p];
+    return !__syncthreads_or(any);
+}
+
 // ---------------------------------------------------------------------------
 // Digit counters of the register sort: 16 bits each (a warp counts at most
 // 32*ITEMS <= 640 items of a digit, a scanned offset is below TILE <= 20,480),
@@ -160,7 +174,8 @@ __device__ __forceinline__ uint32_t cnt16_add(uint32_t* words, uint32_t dig, uin
 template <class T, class RankT, int ITEMS>
 __device__ __forceinline__ void
 sort_regs_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perms, bool descending,
-               RankT* __restrict__ ranks, T* __restrict__ sorted_abs, uint32_t* __restrict__ order) {
+               RankT* __restrict__ ranks, T* __restrict__ sorted_abs, uint32_t* __restrict__ order,
+               const uint8_t* __restrict__ only) {
     using U = typename RadixKey<T>::U;
     static_assert(sizeof(U) == 4, "register sort: fp32 keys");
     constexpr int TILE = kThreads * ITEMS;
@@ -172,6 +187,7 @@ sort_regs_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perms,
     uint32_t* warp_sums = tot + 256;
     uint32_t* flag = warp_sums + 8;
 
+    if (none_marked(only, bx, gx, num_perms)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t lt = lanemask_lt();
     const int my0 = warp * 32 * ITEMS + lane;  // slot of item i: my0 + 32*i
@@ -180,6 +196,7 @@ sort_regs_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perms,
     __syncthreads();
 
     for (int p = bx; p < num_perms; p += gx) {
+        if (only && !only[p]) continue;
         const T* kp = keys + (int64_t)p * G;
         U key[ITEMS];
         uint32_t val[ITEMS];
@@ -275,8 +292,10 @@ sort_regs_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perms,
 template <class T, class RankT, int ITEMS>
 __global__ void __launch_bounds__(kThreads, 1)
 sort_regs_kernel(const T* __restrict__ keys, int G, int num_perms, bool descending,
-                 RankT* __restrict__ ranks, T* __restrict__ sorted_abs, uint32_t* __restrict__ order) {
-    sort_regs_body<T, RankT, ITEMS>(blockIdx.x, gridDim.x, keys, G, num_perms, descending, ranks, sorted_abs, order);
+                 RankT* __restrict__ ranks, T* __restrict__ sorted_abs, uint32_t* __restrict__ order,
+                 const uint8_t* __restrict__ only) {
+    sort_regs_body<T, RankT, ITEMS>(blockIdx.x, gridDim.x, keys, G, num_perms, descending, ranks, sorted_abs, order,
+                                    only);
 }
 
 // every instance of a batch (same ITEMS class) at once: blockIdx.z = the
@@ -286,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) sort_regs_multi(const SortTask* _
     const SortTask& t = tasks[blockIdx.z];
     sort_regs_body<T, RankT, ITEMS>(blockIdx.x, gridDim.x, static_cast<const T*>(t.keys), t.G, t.num_perms,
                                     t.descending != 0, static_cast<RankT*>(t.ranks), static_cast<T*>(t.sorted),
-                                    t.order);
+                                    t.order, t.hard);
 }
 
 template <class T, int ITEMS>
@@ -314,7 +333,8 @@ constexpr bool cluster_packed() { return sizeof(typename RadixKey<T>::U) == 4 &&
 template <class T, class RankT, int ITEMS, int CL>
 __device__ __forceinline__ void
 sort_cluster_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perms, bool descending,
-                  RankT* __restrict__ ranks, T* __restrict__ sorted_abs, uint32_t* __restrict__ order) {
+                  RankT* __restrict__ ranks, T* __restrict__ sorted_abs, uint32_t* __restrict__ order,
+                  const uint8_t* __restrict__ only) {
     using U = typename RadixKey<T>::U;
     constexpr bool PACK = cluster_packed<T, ITEMS>();
     using E = typename std::conditional<PACK, unsigned long long, U>::type;  // exchange slot
@@ -338,7 +358,9 @@ sort_cluster_body(int bx, int gx, const T* __restrict__ keys, int G, int num_per
     const int first = rank * TILE;              // global position of slot 0
     const int clusters = gx / CL;
 
+    if (none_marked(only, bx / CL, clusters, num_perms)) return;  // the same in both CTAs
     for (int p = bx / CL; p < num_perms; p += clusters) {
+        if (only && !only[p]) continue;
         const T* kp = keys + (int64_t)p * G;
         U key[ITEMS];
         uint32_t val[ITEMS];
@@ -470,9 +492,10 @@ sort_cluster_body(int bx, int gx, const T* __restrict__ keys, int G, int num_per
 template <class T, class RankT, int ITEMS, int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kThreads, 1)
 sort_cluster_kernel(const T* __restrict__ keys, int G, int num_perms, bool descending,
-                    RankT* __restrict__ ranks, T* __restrict__ sorted_abs, uint32_t* __restrict__ order) {
+                    RankT* __restrict__ ranks, T* __restrict__ sorted_abs, uint32_t* __restrict__ order,
+                    const uint8_t* __restrict__ only) {
     sort_cluster_body<T, RankT, ITEMS, CL>(blockIdx.x, gridDim.x, keys, G, num_perms, descending, ranks, sorted_abs,
-                                           order);
+                                           order, only);
 }
 
 template <class T, class RankT, int ITEMS, int CL>
@@ -481,7 +504,7 @@ sort_cluster_multi(const SortTask* __restrict__ tasks) {
     const SortTask& t = tasks[blockIdx.z];
     sort_cluster_body<T, RankT, ITEMS, CL>(blockIdx.x, gridDim.x, static_cast<const T*>(t.keys), t.G, t.num_perms,
                                            t.descending != 0, static_cast<RankT*>(t.ranks), static_cast<T*>(t.sorted),
-                                           t.order);
+                                           t.order, t.hard);
 }
 
 template <class T, int ITEMS>
@@ -540,7 +563,8 @@ template <class T, class RankT>
 __global__ void __launch_bounds__(kThreads, 1)
 sort_tiled_kernel(const T* __restrict__ keys, int G, int num_perms, bool descending,
                   RankT* __restrict__ ranks, T* __restrict__ sorted_abs, uint32_t* __restrict__ order,
-                  unsigned char* __restrict__ scratch, bool stage_ranks, int* __restrict__ error_flag) {
+                  unsigned char* __restrict__ scratch, bool stage_ranks, int* __restrict__ error_flag,
+                  const uint8_t* __restrict__ only) {
     using U = typename RadixKey<T>::U;
     constexpr int NPASS = (int)sizeof(U);
     // stage buffers [2][kTile] keys and [2][kTile] gene ids; after the
@@ -558,6 +582,7 @@ sort_tiled_kernel(const T* __restrict__ keys, int G, int num_perms, bool descend
     __shared__ int failed;
     __shared__ __align__(8) unsigned long long bar[kStages];
 
+    if (none_marked(only, blockIdx.x, gridDim.x, num_perms)) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t lt = lanemask_lt();
     const int Gp = tiled_row(G);
@@ -573,6 +598,7 @@ sort_tiled_kernel(const T* __restrict__ keys, int G, int num_perms, bool descend
     const int ntiles = (G + kTile - 1) / kTile;
 
     for (int p = blockIdx.x; p < num_perms; p += gridDim.x) {
+        if (only && !only[p]) continue;
         int a_off = 0;  // buffer A = rows at a_off, buffer B = rows at Gp - a_off
         bool ident = true;  // buffer A's gene ids are the identity (not yet written)
         const T* kp = keys + (int64_t)p * G;
@@ -721,20 +747,22 @@ int num_sms() {
 }
 
 template <class T, class RankT, int ITEMS>
-cudaError_t launch_regs(const T* keys, int G, int P, bool desc, const SortBuffers& o, cudaStream_t st) {
+cudaError_t launch_regs(const T* keys, int G, int P, bool desc, const SortBuffers& o, const uint8_t* only,
+                        cudaStream_t st) {
     const size_t smem = regs_smem_bytes<T, ITEMS>();
     auto kern = sort_regs_kernel<T, RankT, ITEMS>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int grid = P < 4 * num_sms() ? P : 4 * num_sms();
-    kern<<<grid, kThreads, smem, st>>>(keys, G, P, desc, static_cast<RankT*>(o.ranks),
-                                       static_cast<T*>(o.sorted_abs), o.order);
+    const int fill = (only ? 1 : 4) * num_sms();  // after the bucket sort there is seldom anything left
+    kern<<<P < fill ? P : fill, kThreads, smem, st>>>(keys, G, P, desc, static_cast<RankT*>(o.ranks),
+                                                      static_cast<T*>(o.sorted_abs), o.order, only);
     launches_add(1);
     return cudaGetLastError();
 }
 
 template <class T, class RankT, int ITEMS, int CL>
-cudaError_t launch_cluster(const T* keys, int G, int P, bool desc, const SortBuffers& o, cudaStream_t st) {
+cudaError_t launch_cluster(const T* keys, int G, int P, bool desc, const SortBuffers& o, const uint8_t* only,
+                           cudaStream_t st) {
     const size_t smem = cluster_smem_bytes<T, ITEMS>();
     auto kern = sort_cluster_kernel<T, RankT, ITEMS, CL>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -748,7 +776,7 @@ cudaError_t launch_cluster(const T* keys, int G, int P, bool desc, const SortBuf
     const int groups = num_sms() * per_sm / CL > 0 ? num_sms() * per_sm / CL : 1;
     const int clusters = P < groups ? P : groups;
     kern<<<CL * clusters, kThreads, smem, st>>>(keys, G, P, desc, static_cast<RankT*>(o.ranks),
-                                                static_cast<T*>(o.sorted_abs), o.order);
+                                                static_cast<T*>(o.sorted_abs), o.order, only);
     launches_add(1);
     return cudaGetLastError();
 }
@@ -760,34 +788,33 @@ template <class T>
 constexpr int regs_max_genes() { return sizeof(T) == 4 ? 2 * kThreads * 20 : 2 * kThreads * 10; }
 
 template <class T, class RankT>
-cudaError_t launch_sort_t(const T* keys, int G, int P, bool desc, const SortBuffers& o, cudaStream_t st) {
-    if (o.variant == 1 && G > regs_max_genes<T>()) return cudaErrorInvalidValue;
+cudaError_t launch_radix(const T* keys, int G, int P, bool desc, const SortBuffers& o, const uint8_t* only,
+                         cudaStream_t st) {
     if constexpr (sizeof(T) == 8) {
         // fp64: the cluster form holds the segment in registers (keys and
         // gene ids exchanged separately); one CTA up to 10,240 genes, a
         // two-CTA cluster beyond
         if (o.variant != 2) {
-            if (G <= kThreads * 4) return launch_cluster<T, RankT, 4, 1>(keys, G, P, desc, o, st);
-            if (G <= kThreads * 10) return launch_cluster<T, RankT, 10, 1>(keys, G, P, desc, o, st);
-            if (G <= 2 * kThreads * 10) return launch_cluster<T, RankT, 10, 2>(keys, G, P, desc, o, st);
+            if (G <= kThreads * 4) return launch_cluster<T, RankT, 4, 1>(keys, G, P, desc, o, only, st);
+            if (G <= kThreads * 10) return launch_cluster<T, RankT, 10, 1>(keys, G, P, desc, o, only, st);
+            if (G <= 2 * kThreads * 10) return launch_cluster<T, RankT, 10, 2>(keys, G, P, desc, o, only, st);
         }
     }
     if constexpr (sizeof(T) == 4) {
       if (o.variant != 2) {
-        if (G <= kThreads * 4) return launch_regs<T, RankT, 4>(keys, G, P, desc, o, st);
-        if (G <= kThreads * 8) return launch_regs<T, RankT, 8>(keys, G, P, desc, o, st);
-        if (G <= kThreads * 12) return launch_regs<T, RankT, 12>(keys, G, P, desc, o, st);
-        if (G <= kThreads * 16) return launch_regs<T, RankT, 16>(keys, G, P, desc, o, st);
-        if (G <= kThreads * 20) return launch_regs<T, RankT, 20>(keys, G, P, desc, o, st);
+        if (G <= kThreads * 4) return launch_regs<T, RankT, 4>(keys, G, P, desc, o, only, st);
+        if (G <= kThreads * 8) return launch_regs<T, RankT, 8>(keys, G, P, desc, o, only, st);
+        if (G <= kThreads * 12) return launch_regs<T, RankT, 12>(keys, G, P, desc, o, only, st);
+        if (G <= kThreads * 16) return launch_regs<T, RankT, 16>(keys, G, P, desc, o, only, st);
+        if (G <= kThreads * 20) return launch_regs<T, RankT, 20>(keys, G, P, desc, o, only, st);
         // two-CTA clusters: a four-CTA cluster ran ~2.4x slower per SM
         // (four-way barriers, scatters to three peers, GPC packing)
-        if (G <= 2 * kThreads * 16) return launch_cluster<T, RankT, 16, 2>(keys, G, P, desc, o, st);
-        if (G <= 2 * kThreads * 20) return launch_cluster<T, RankT, 20, 2>(keys, G, P, desc, o, st);
+        if (G <= 2 * kThreads * 16) return launch_cluster<T, RankT, 16, 2>(keys, G, P, desc, o, only, st);
+        if (G <= 2 * kThreads * 20) return launch_cluster<T, RankT, 20, 2>(keys, G, P, desc, o, only, st);
       }
     }
     using U = typename RadixKey<T>::U;
     const int grid = P < num_sms() ? P : num_sms();
-    if (o.scratch_bytes < sort_scratch_bytes<T>(G, P)) return cudaErrorInvalidValue;
     // the bulk copies read the scratch rows from 16-byte boundaries
     if (reinterpret_cast<uintptr_t>(o.scratch) & 15u) return cudaErrorInvalidValue;
     // stage the ranks by gene in shared memory (over the stage buffers) when
@@ -800,9 +827,26 @@ cudaError_t launch_sort_t(const T* keys, int G, int P, bool desc, const SortBuff
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
     kern<<<grid, kThreads, dyn, st>>>(keys, G, P, desc, static_cast<RankT*>(o.ranks), static_cast<T*>(o.sorted_abs),
-                                      o.order, static_cast<unsigned char*>(o.scratch), stage, o.error_flag);
+                                      o.order, static_cast<unsigned char*>(o.scratch), stage, o.error_flag, only);
     launches_add(1);
     return cudaGetLastError();
+}
+
+template <class T, class RankT>
+cudaError_t launch_sort_t(const T* keys, int G, int P, bool desc, SortBuffers o, cudaStream_t st) {
+    if (o.variant == 1 && G > regs_max_genes<T>()) return cudaErrorInvalidValue;
+    if (o.scratch_bytes < sort_scratch_bytes<T>(G, P)) return cudaErrorInvalidValue;
+    const uint8_t* only = nullptr;
+    if constexpr (sizeof(RankT) == 2) {
+        if (o.variant != 2 && sort_bucket_class(G) != 0) {
+            // one mark per permutation, at the end of the scratch
+            o.hard = static_cast<uint8_t*>(o.scratch) + (o.scratch_bytes - sort_mark_bytes(P));
+            const cudaError_t e = launch_sort_bucket<T>(keys, G, P, desc, o, st);
+            if (e != cudaSuccess) return e;
+            only = o.hard;
+        }
+    }
+    return launch_radix<T, RankT>(keys, G, P, desc, o, only, st);
 }
 
 template <class T, class RankT, int ITEMS>
@@ -811,7 +855,7 @@ cudaError_t launch_regs_multi(const SortTask* d, int n, cudaStream_t st) {
     auto kern = sort_regs_multi<T, RankT, ITEMS>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int per = (2 * num_sms() + n - 1) / n;  // CTAs per instance: about two waves over the SMs in all
+    const int per = (num_sms() + n - 1) / n;  // CTAs per instance: about one wave over the SMs in all
     kern<<<dim3((unsigned)(per > 0 ? per : 1), 1, (unsigned)n), kThreads, smem, st>>>(d);
     launches_add(1);
     return cudaGetLastError();
@@ -823,7 +867,7 @@ cudaError_t launch_cluster_multi(const SortTask* d, int n, cudaStream_t st) {
     auto kern = sort_cluster_multi<T, RankT, ITEMS, CL>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int per = (2 * num_sms() / CL + n - 1) / n;  // clusters per instance
+    const int per = (num_sms() / CL + n - 1) / n;  // clusters per instance
     kern<<<dim3((unsigned)(CL * (per > 0 ? per : 1)), 1, (unsigned)n), kThreads, smem, st>>>(d);
     launches_add(1);
     return cudaGetLastError();
@@ -831,16 +875,16 @@ cudaError_t launch_cluster_multi(const SortTask* d, int n, cudaStream_t st) {
 
 }  // namespace
 
+// radix sorts of a batch (what its bucket sorts declined): few classes, a
+// batch launches each of them
 int sort_multi_class(int G, bool fp64) {
-    if (G <= 0 || G > 65536) return 0;
+    if (G <= 0 || G > 65535) return 0;
     if (!fp64) {
-        for (int items : {4, 8, 12, 16, 20})
-            if (G <= kThreads * items) return items;
-        if (G <= 2 * kThreads * 16) return 116;
+        if (G <= kThreads * 8) return 8;
+        if (G <= kThreads * 20) return 20;
         if (G <= 2 * kThreads * 20) return 120;
         return 0;
     }
-    if (G <= kThreads * 4) return 204;
     if (G <= kThreads * 10) return 210;
     if (G <= 2 * kThreads * 10) return 310;
     return 0;
@@ -852,30 +896,27 @@ cudaError_t launch_sort_multi(const SortTask* d_tasks, int n, int cls, bool fp64
     using R = uint16_t;  // batch instances have at most 65,536 genes
     if (!fp64) {
         switch (cls) {
-            case 4: return launch_regs_multi<float, R, 4>(d_tasks, n, st);
             case 8: return launch_regs_multi<float, R, 8>(d_tasks, n, st);
-            case 12: return launch_regs_multi<float, R, 12>(d_tasks, n, st);
-            case 16: return launch_regs_multi<float, R, 16>(d_tasks, n, st);
             case 20: return launch_regs_multi<float, R, 20>(d_tasks, n, st);
-            case 116: return launch_cluster_multi<float, R, 16, 2>(d_tasks, n, st);
             case 120: return launch_cluster_multi<float, R, 20, 2>(d_tasks, n, st);
             default: return cudaErrorInvalidValue;
         }
     }
     switch (cls) {
-        case 204: return launch_cluster_multi<double, R, 4, 1>(d_tasks, n, st);
         case 210: return launch_cluster_multi<double, R, 10, 1>(d_tasks, n, st);
         case 310: return launch_cluster_multi<double, R, 10, 2>(d_tasks, n, st);
         default: return cudaErrorInvalidValue;
     }
 }
 
+size_t sort_mark_bytes(int num_perms) { return ((size_t)num_perms + 15) & ~(size_t)15; }
+
 template <class T>
 size_t sort_scratch_bytes(int G, int num_perms) {
     using U = typename RadixKey<T>::U;
     // sized for the tiled variant, which any G may be tuned to
     const int grid = num_perms < num_sms() ? num_perms : num_sms();
-    return tiled_cta_bytes<U>(G) * (size_t)(grid > 0 ? grid : 1);
+    return tiled_cta_bytes<U>(G) * (size_t)(grid > 0 ? grid : 1) + sort_mark_bytes(num_perms);
 }
 template size_t sort_scratch_bytes<float>(int, int);
 template size_t sort_scratch_bytes<double>(int, int);

@@ -54,10 +54,11 @@ struct SortBuffers {
     bool ranks16;
     void* sorted_abs;     // T*
     uint32_t* order;      // optional
-    void* scratch;        // per-CTA ping-pong buffers for the tiled variant
+    void* scratch;        // per-CTA ping-pong buffers for the tiled variant, one mark per permutation
     size_t scratch_bytes;
-    int variant = 0;      // 0 automatic, 1 register radix sort (fp32, G <= 40,960; two-CTA clusters above 20,480), 2 tiled
+    int variant = 0;      // 0 automatic, 1 on-chip sorts (bucket, then register radix; fp32 G <= 40,960, fp64 G <= 20,480), 2 tiled
     int* error_flag = nullptr;  // set to 1 when a bounded wait of the tiled sort expires
+    uint8_t* hard = nullptr;    // set by launch_sort: permutations the bucket sort left to the radix sort
 };
 template <class T>
 size_t sort_scratch_bytes(int G, int num_perms);
@@ -129,21 +130,38 @@ template <class T>
 cudaError_t launch_stats_ragged(const T* es, int K, int64_t ld, const int64_t* counts, int64_t p_fwer, T* stats,
                                 void* scratch, cudaStream_t st, int64_t hist_cols = 0);
 
-// Sorts of many instances at once (batched form): all instances of one
+// The bucket sort (k_sort_bucket.cu): class of G genes (0: none; 16-bit ranks
+// only), and the launch, which marks in out.hard the permutations it leaves
+// to the radix sorts.
+int sort_bucket_class(int G);
+int sort_bucket_cap(int G);   // slots a permutation is given
+size_t sort_mark_bytes(int num_perms);
+template <class T>
+cudaError_t launch_sort_bucket(const T* keys, int G, int num_perms, bool descending, const SortBuffers& out,
+                               cudaStream_t st);
+
+// Sorts of many instances at once (batched form): first the bucket sort of
+// all instances of one class (sort_bucket_multi_class), then, for the
+// permutations marked in `hard`, the radix sort of all instances of one
 // register-resident class (sort_multi_class of their G and precision; 0: the
-// class has no multi form, the instance takes its solo launch_sort), one
-// launch, blockIdx.z = instance; ranks (16-bit), weights and order those of
-// the solo sort.
+// class has no multi form, the instance takes its solo launch_sort); one
+// launch each, blockIdx.z = instance; ranks (16-bit), weights and order those
+// of the solo sort.
 struct SortTask {
     const void* keys;   // [P][G] T
     void* ranks;        // [P][G] uint16
     void* sorted;       // [P][G] T
     uint32_t* order;    // [P][G] or null
+    uint8_t* hard;      // [P] permutations left to the radix sort
     int G;
     int num_perms;
     int descending;
+    int cap;            // sort_bucket_cap(G)
 };
 int sort_multi_class(int G, bool fp64);
+int sort_bucket_multi_class(int G);
+cudaError_t launch_sort_bucket_multi(const SortTask* d_tasks, const SortTask* h_tasks, int n, int cls, bool fp64,
+                                     cudaStream_t st);
 cudaError_t launch_sort_multi(const SortTask* d_tasks, int n, int cls, bool fp64, cudaStream_t st);
 
 // Label permutations of many instances at once (batched form), blockIdx.z =

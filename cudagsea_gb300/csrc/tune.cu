@@ -107,7 +107,9 @@ int autotune_t(gsea_plan_s* p, int64_t n64, unsigned stages, gsea_tuning* best_o
     sb.scratch_bytes = p->sort_scratch_bytes;
     sb.error_flag = p->dev_error;
     float sbest = 1e30f;
-    std::vector<int> sc = {1, 2};
+    // beyond the register radix sorts (variant 1) the automatic choice is the
+    // bucket sort with the tiled one behind it
+    std::vector<int> sc = {G <= (c.precision == 64 ? 20480 : 40960) ? 1 : 0, 2};
     if (!(stages & kSort)) sc = {best.sort_variant};
     for (int v : sc) {
         sb.variant = v;

@@ -279,9 +279,11 @@ typedef struct gsea_tuning {
     int32_t chosen_tile;  /* tensor-core form: permutations per tile, 128 (the automatic choice: one
                              persistent CTA per SM walking the tiles, the copies, MMAs and
                              epilogue on separate warps) or 256 (one tile per CTA) */
-    int32_t sort_variant; /* 1 register radix sort (fp32, G <= 40,960: one CTA up to 20,480, a two-CTA
+    int32_t sort_variant; /* 1 on-chip sorts: a bucket sort, and for the permutations it declines the
+                             register radix sort (fp32, G <= 40,960: one CTA up to 20,480, a two-CTA
                              cluster exchanging through distributed shared memory beyond; fp64,
-                             G <= 20,480: one CTA up to 10,240, a two-CTA cluster beyond), 2 tiled */
+                             G <= 20,480: one CTA up to 10,240, a two-CTA cluster beyond), 2 tiled;
+                             0: the bucket sort up to 65,535 genes with 1 or 2 behind it */
     int32_t es_warps;     /* warps per CTA of the enrichment kernel: 8, 16, 24 or 32 (24: with
                              es_stage 2 or 3 only) */
     int32_t es_stage;     /* 1 stage the permutation's ranks and weights in shared memory, 2 its ranks
