@@ -293,8 +293,7 @@ int build_classes(gsea_batch_s* b) {
             gsea::EsTask<T> t;
             t.ranks = p->ranks;
             t.sorted = static_cast<const T*>(p->sorted);
-            t.off = p->set_off;
-            t.genes = p->set_genes;
+            t.sets = gsea::plan_sets(p);
             t.order = p->set_order;
             t.decay = static_cast<const T*>(p->decay);
             t.es = static_cast<T*>(p->es);

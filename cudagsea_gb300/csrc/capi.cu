@@ -97,7 +97,7 @@ int mark(gsea_plan_s* p, int stage, cudaStream_t st) {
 }
 
 void free_plan_buffers(gsea_plan_s* p) {
-    void* bufs[] = {p->exprs, p->labels, p->set_off, p->set_genes, p->set_order, p->masks, p->fast_ok, p->decay, p->gene_mu,
+    void* bufs[] = {p->exprs, p->labels, p->set_off, p->set_genes, p->set_rec, p->set_list, p->set_order, p->masks, p->fast_ok, p->decay, p->gene_mu,
                     p->gene_t1, p->gene_t2, p->opA1, p->opA2, p->opB, p->dev_error, p->keys,
                     p->ranks, p->sorted, p->order, p->sort_scratch, p->es, p->stats, p->stats_scratch,
                     p->moments, p->active, p->counts, p->exceed, p->sumabs, p->qlow, p->feat, p->pred,
@@ -107,6 +107,8 @@ void free_plan_buffers(gsea_plan_s* p) {
     p->exprs = p->labels = nullptr;
     p->set_off = nullptr;
     p->set_genes = nullptr;
+    p->set_rec = nullptr;
+    p->set_list = nullptr;
     p->set_order = nullptr;
     p->masks = nullptr;
     p->fast_ok = nullptr;
@@ -173,11 +175,15 @@ int upload_sets(gsea_plan_s* p, const int64_t* off, const int32_t* genes, cudaSt
     for (int64_t k = 0; k < K; k++)
         if (off[k + 1] < off[k]) return fail(GSEA_ERR_INVALID_INPUT, "set_offsets must be non-decreasing");
     const int64_t nnz = off[K];
-    if (nnz > p->nnz_cap) {
+    if (nnz > p->nnz_cap || (p->ranks16 && !p->set_list)) {
         drop_graph(p);  // the captured launches point at the old buffer
         if (p->set_genes) cudaFree(p->set_genes);
         p->set_genes = nullptr;
+        if (p->set_list) cudaFree(p->set_list);
+        p->set_list = nullptr;
+        p->nnz_cap = 0;
         int rc = dev_alloc(&p->set_genes, sizeof(int32_t) * (size_t)nnz, "set genes");
+        if (!rc && p->ranks16) rc = dev_alloc(&p->set_list, gsea::es_list_bytes(K, nnz), "set lists");
         if (rc) return rc;
         p->nnz_cap = nnz;
     }
@@ -219,14 +225,19 @@ int count_labels(gsea_plan_s* p, const uint8_t* labels) {
 }
 
 // device-side preparation of freshly uploaded inputs, on `st`: the check of
-// the expression table (sets p->fast_ok) and, for the chosen form, the split
-// tensor-core operands
+// the expression table (sets p->fast_ok), the sets' marking lists and, for
+// the chosen form, the split tensor-core operands
 int check_inputs(gsea_plan_s* p, cudaStream_t st) {
     const int64_t n = p->cfg.num_genes * p->cfg.num_samples;
     cudaError_t e = p->cfg.precision == 64
                         ? gsea::launch_finite_check<double>(static_cast<const double*>(p->exprs), n, p->fast_ok, st)
                         : gsea::launch_finite_check<float>(static_cast<const float*>(p->exprs), n, p->fast_ok, st);
     if (e != cudaSuccess) return cuda_fail(e, "input check kernel");
+    if (p->ranks16 && p->set_list) {
+        e = gsea::launch_es_lists(p->set_off, p->set_genes, (int)p->cfg.num_sets, (int)p->cfg.num_genes, p->set_rec,
+                                  p->set_list, st);
+        if (e != cudaSuccess) return cuda_fail(e, "set list kernel");
+    }
     if (p->cfg.form != GSEA_FORM_PLAIN) {
         e = gsea::launch_chosen_prepare<float>(static_cast<const float*>(p->exprs), (int)p->cfg.num_genes,
                                                (int)p->cfg.num_samples, p->gene_mu, p->gene_t1, p->gene_t2, p->opA1,
@@ -289,8 +300,8 @@ int run_range_t(gsea_plan_s* p, cudaStream_t st, int64_t lo, int64_t hi, const i
                   "sort kernel");
         if ((rc = mark(p, 2, st))) return rc;
         if (!with_es) continue;
-        GSEA_CUDA(gsea::launch_es<T>(p->ranks, p->ranks16, static_cast<const T*>(p->sorted), G, nb, p->set_off,
-                                     p->set_genes, set_list, static_cast<const T*>(p->decay), n_sets,
+        GSEA_CUDA(gsea::launch_es<T>(p->ranks, p->ranks16, static_cast<const T*>(p->sorted), G, nb,
+                                     gsea::plan_sets(p), set_list, static_cast<const T*>(p->decay), n_sets,
                                      static_cast<T*>(p->es), P, b0, st, et, n_dev),
                   "enrichment kernel");
         if ((rc = mark(p, 3, st))) return rc;
@@ -372,6 +383,7 @@ int plan_run_range(gsea_plan_s* p, cudaStream_t st, int64_t lo, int64_t hi, cons
     return p->cfg.precision == 64 ? run_range_t<double>(p, st, lo, hi, set_list, n_sets, true, n_dev)
                                   : run_range_t<float>(p, st, lo, hi, set_list, n_sets, true, n_dev);
 }
+EsSets plan_sets(const gsea_plan_s* p) { return EsSets{p->set_off, p->set_genes, p->set_rec, p->set_list}; }
 int plan_dev_alloc(void** ptr, size_t bytes, const char* what) { return dev_alloc(ptr, bytes, what); }
 void plan_drop_graph(gsea_plan_s* p) { drop_graph(p); }
 int plan_check_error(gsea_plan_s* p) { return p->cfg.form != GSEA_FORM_PLAIN ? check_device_error(p) : GSEA_OK; }
@@ -558,6 +570,7 @@ int gsea_plan_create(const gsea_config* cfg, gsea_plan* out) {
         (rc = dev_alloc(&p->labels, (size_t)S, "labels")) ||
         (rc = dev_alloc(&p->set_off, sizeof(int64_t) * (K + 1), "set offsets")) ||
         (rc = dev_alloc(&p->set_order, sizeof(int32_t) * K, "set order")) ||
+        (p->ranks16 && (rc = dev_alloc(&p->set_rec, sizeof(int2) * K, "set records"))) ||
         (rc = dev_alloc(&p->masks, 4 * (size_t)p->words * pb, "label masks")) ||
         (rc = dev_alloc(&p->fast_ok, sizeof(int), "input flags")) ||
         (rc = dev_alloc(&p->decay, T * ((size_t)G + 1), "decay table")) ||

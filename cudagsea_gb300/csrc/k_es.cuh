@@ -25,21 +25,37 @@
 //     every position in shared memory (or, when the bitmaps of large G leave
 //     no room, the ranks only, the weights then read through L1 / L2);
 //   * a warp takes the next set from a CTA-wide counter (largest sets first),
-//     marks its members' ranks in a per-warp bitmap (duplicates collapse) and
-//     sums the weights of the marked ranks (N_R);
+//     marks its members' ranks in a per-warp bitmap and sums the weights of
+//     the marked ranks (N_R).  The members come from lists laid out at upload
+//     (es_lists_kernel): 16-bit gene ids, a lane's four members of a group of
+//     128 in one 8-byte load, no bounds or duplicate checks left to make;
 //   * each lane owns a contiguous range of bitmap words: their popcounts and
 //     one warp scan give the global index of the lane's first hit, and the
 //     lane walks its hits once, in rank order, with a lane-local prefix of the
 //     weights; its largest and smallest candidates are shifted afterwards by
 //     the weight of the hits before the lane (a second warp scan);
-//   * a warp reduction picks the winner.
+//   * two integer warp reductions give the largest and the smallest value.
 //   With 32-bit ranks (G > 65,536) a general procedure walks each lane's
 //   word range twice from shared memory instead.
 //
 // Rounding: fp32 sums are compensated (Kahan in a lane, float-float across
 // lanes), so the fp32 ES stay within a few ulp of the reference's Kahan
-// running sum (the shift adds one rounding); the fp64 path is double
-// throughout.
+// running sum (the shift adds one rounding).  fp64: the walk runs in fp32 and
+// only finds where the extremum is; the score there is then evaluated from
+// double sums over the set's members.  Where fp32 cannot tell which hit (or
+// which sign) wins, the set is walked again in double throughout.
+//
+// What bounds it: issue slots (1,000 sets x 1,000 permutations at 20,000
+// genes, fp32).  The walk is the largest part, 14 trips of the longest lane
+// for 8 hits per lane, so the trips carry as little as possible: bitmap words
+// hold the lowest rank in their top bit (one leading-zero count finds it, no
+// bit reversal), positions and miss counts are kept times four (byte offsets
+// of the weights; the decay is divided by four, exactly), the miss count
+// becomes a float by an addition instead of a conversion, the extrema carry
+// no positions and the words are cleared afterwards, 16 bytes at a time.
+// Positions decide a score only when the largest and the smallest value have
+// the same magnitude: such a set, and one whose weights are not finite, takes
+// the procedure with positions (set_score_positions).
 #pragma once
 #include <climits>
 #include <type_traits>
@@ -120,20 +136,12 @@ __device__ __forceinline__ void consider(T val, int pos, T& best, int& bpos) {
 }
 
 // ---------------------------------------------------------------------------
-// Per-set procedures.  Both run on one warp with the set's member ranks marked
-// in the warp's bitmap `bm` (G bits) and leave the bitmap all zero.
+// Per-set procedures.  All run on one warp with the set's member ranks marked
+// in the warp's bitmap `bm` (G bits): rank r in word r / 32.  The direct
+// procedures (G <= 1024*WPL) keep rank r in bit 31 - r % 32, and their words
+// are cleared by clear_words; the general one keeps it in bit r % 32 and
+// leaves the bitmap all zero.
 
-// Direct procedure (G <= 1024*WPL): the lane's bitmap words (WPL, a multiple
-// of 4, loaded as 16-byte vectors) give its hit count and a mask of its
-// nonzero words; a warp scan of the counts gives the global index of each
-// lane's first hit.  Every lane then walks its own hits once, in rank order,
-// with a lane-local compensated prefix of the weights, and keeps its largest
-// value after a hit and smallest value before one; the weight of the hits in
-// the lanes before it (a second warp scan, after the walk) shifts both by a
-// constant, which leaves their positions unchanged.  The set's total weight
-// `Wt` (every lane) comes from the marking.  Each word is cleared as it is
-// read.  `w0` = lane*WPL: the lane's first word, 16-byte aligned inside the
-// warp's region of WPL*32 words (bits at positions >= G are never set).
 // order-preserving signed 64-bit key of a double (an involution): the
 // integer order of the keys is the numeric order of non-NaN doubles, -0
 // below +0
@@ -145,95 +153,174 @@ __device__ __forceinline__ double okey_value(long long k) {
     return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
 }
 
-// One lane's walk over its hits in rank order (the direct procedure below):
-// its largest value after a hit (mx at pmx) and smallest before one (mn at
-// pmn) with the lane-local prefix Wl.  IKEY (doubles whose candidates are all
-// finite): the running extrema are compared as integer keys, on the integer
-// pipe instead of the FP64 pipe that bounds the FP64 kernel -- the same
-// results, since the keys order finite doubles as they compare except -0 /
-// +0, and a zero never decides a score (only a positive maximum or a
-// negative minimum counts).
-template <class T, int WPL, bool IKEY, class Mask>
-__device__ __forceinline__ void walk_hits(uint32_t* bm, int w0, Mask nzm, int cnt, int excl, const T* wt, T inv,
-                                          T d, Acc<T>& Wl, T& mx, int& pmx, T& mn, int& pmn) {
-    uint32_t cur = 0u;
-    int wi = 0;
-    long long kmx = 0, kmn = 0;
-    if constexpr (IKEY) {
-        kmx = okey(mx);
-        kmn = okey(mn);
-    }
-    for (int t = 0; t < cnt; t++) {
-        if (cur == 0u) {  // next nonzero word of the lane
-            wi = (WPL > 32 ? __ffsll((long long)nzm) : __ffs((int)nzm)) - 1;
-            nzm &= nzm - 1;
-            cur = bm[w0 + wi];
-            bm[w0 + wi] = 0u;
-        }
-        const int bit = __ffs(cur) - 1;
-        cur &= cur - 1;
-        const int r = ((w0 + wi) << 5) + bit;
-        const T md = -(T)(r - (excl + t)) * d;  // misses before this hit, times the decay
-        const T before = t > 0 ? Wl.scaled_plus(inv, md) : md;
-        Wl.add(wt[r]);
-        const T after = Wl.scaled_plus(inv, md);
-        if constexpr (IKEY) {
-            const long long kb = okey(before), ka = okey(after);
-            if (kb < kmn) { kmn = kb; pmn = r - 1; }
-            if (ka > kmx) { kmx = ka; pmx = r; }
-        } else {
-            if (before < mn) { mn = before; pmn = r - 1; }
-            if (after > mx) { mx = after; pmx = r; }
-        }
-    }
-    if constexpr (IKEY) {
-        mx = okey_value(kmx);
-        mn = okey_value(kmn);
-    }
+// A lane's words are read and cleared 16 bytes at a time, eight lanes at
+// once: where the lanes' regions lie a multiple of 64 or 128 bytes apart (WPL
+// 16, 32, 48, 64) they meet in the same banks (4- and 8-way; two thirds of
+// the time of a set at 60,000 genes), so those regions are 16 bytes longer.
+template <int WPL>
+__host__ __device__ constexpr int lane_stride() { return WPL > 0 && WPL % 16 == 0 ? WPL + 4 : WPL; }
+// the bitmap word of rank r
+template <int WPL>
+__device__ __forceinline__ uint32_t* rank_word(uint32_t* bm, uint32_t r) {
+    const uint32_t w = r >> 5;
+    return bm + (lane_stride<WPL>() == WPL ? w : w + 4u * (w / (uint32_t)(WPL > 0 ? WPL : 1)));
 }
 
-template <class T, int WPL>
-__device__ __forceinline__ T set_score_direct(uint32_t* bm, int w0, const T* wt, const T* __restrict__ decay, int G,
-                                              int lane, const Acc<T>& Wt) {
-    using Mask = typename std::conditional<(WPL > 32), unsigned long long, uint32_t>::type;
-    Mask nzm = 0;  // bit i: word w0 + i holds hits
+// bit i from the top of a word, and the place from the top of a word's
+// highest bit (nonzero words: one instruction, where a count of leading zeros
+// also has to answer for zero)
+__device__ __forceinline__ uint32_t top_bit(int i) { return 0x80000000u >> i; }
+__device__ __forceinline__ int top_place(uint32_t v) {
+    int i;
+    asm("bfind.shiftamt.u32 %0, %1;" : "=r"(i) : "r"(v));
+    return i;
+}
+
+// A lane's share of the bitmap: words w0 .. w0 + WPL - 1 (w0 = lane*WPL).
+// nz marks its nonzero words, word i in bit 31 - i (words from 32 on in nz2).
+template <int WPL>
+struct LaneWords {
+    uint32_t nz = 0u, nz2 = 0u;
     int cnt = 0;
+    __device__ __forceinline__ explicit LaneWords(const uint32_t* bmw) {
 #pragma unroll
-    for (int i = 0; i < WPL; i += 4) {
-        const uint4 v = *reinterpret_cast<const uint4*>(bm + w0 + i);
-        cnt += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
-        nzm |= (Mask)(((v.x != 0u) ? 1u : 0u) | ((v.y != 0u) ? 2u : 0u) | ((v.z != 0u) ? 4u : 0u) |
-                      ((v.w != 0u) ? 8u : 0u)) << i;
+        for (int i = 0; i < WPL; i += 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(bmw + i);
+            // four counts (at most 32 each) in the bytes of a word: summed at
+            // once, and turned into four marks (bit 7 of a byte plus 127 says
+            // the count is not zero; the product gathers bits 7, 15, 23, 31)
+            const uint32_t c = ((uint32_t)__popc(v.x) << 24) + ((uint32_t)__popc(v.y) << 16) +
+                               ((uint32_t)__popc(v.z) << 8) + (uint32_t)__popc(v.w);
+            cnt = (int)__dp4a(c, 0x01010101u, (uint32_t)cnt);
+            const uint32_t m = ((((c + 0x7f7f7f7fu) & 0x80808080u) * 0x204081u) & 0xf0000000u) >> (i & 31);
+            if (i < 32) nz |= m; else nz2 |= m;
+        }
     }
+};
+template <int WPL>
+__device__ __forceinline__ void clear_words(uint32_t* bmw) {
+#pragma unroll
+    for (int i = 0; i < WPL; i += 4) *reinterpret_cast<uint4*>(bmw + i) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// the lane's hits in rank order: next() gives four times the rank.  The step
+// to the lane's next nonzero word (taken by some lane at nearly every hit) is
+// predicated instead of branched around.
+template <int WPL>
+struct HitWalk {
+    uint32_t bmw;  // shared-memory address of the lane's words
+    uint32_t nz, nz2, cur = 0u;
+    uint32_t word4 = 0u, lane4;  // four times the rank of the word's top bit / of the lane's first
+    __device__ __forceinline__ HitWalk(const uint32_t* words, int w0, const LaneWords<WPL>& w)
+        : bmw((uint32_t)__cvta_generic_to_shared(words)), nz(w.nz), nz2(w.nz2), lane4((uint32_t)w0 << 7) {}
+    __device__ __forceinline__ uint32_t next() {
+        if (WPL > 32 && (cur | nz) == 0u) {
+            nz = nz2;
+            bmw += 32u * 4u;
+            lane4 += 32u << 7;
+        }
+        // reads words no one changes during the walk: no memory clobber
+        asm(
+            "{\n"
+            " .reg .pred p;\n"
+            " .reg .u32 i, t, a;\n"
+            " setp.eq.u32 p, %0, 0;\n"
+            " @p bfind.shiftamt.u32 i, %1;\n"
+            " @p shr.u32 t, 0x80000000, i;\n"
+            " @p xor.b32 %1, %1, t;\n"
+            " @p mad.lo.u32 a, i, 4, %3;\n"
+            " @p ld.shared.u32 %0, [a];\n"
+            " @p mad.lo.u32 %2, i, 128, %4;\n"
+            "}"
+            : "+r"(cur), "+r"(nz), "+r"(word4)
+            : "r"(bmw), "r"(lane4));
+        const int bit = top_place(cur);
+        cur ^= top_bit(bit);
+        return word4 + ((uint32_t)bit << 2);
+    }
+};
+
+template <class T>
+__device__ __forceinline__ T weight_at(const T* wt, uint32_t r4) {
+    return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(wt) + (size_t)r4 * (sizeof(T) / 4));
+}
+
+// exclusive count of the hits in the lanes before, and their total n
+__device__ __forceinline__ int hits_before(int cnt, int lane, int& n) {
     int incl = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(kFullMask, incl, o);
         if (lane >= o) incl += y;
     }
-    const int n = __shfl_sync(kFullMask, incl, 31);
-    const int excl = incl - cnt;  // hits in the lanes before
-    const T inv = n > 0 ? T(1) / Wt.value() : T(0);
-    const T d = decay[n];
-    Acc<T> Wl;  // weight of this lane's hits so far
-    T mx = -CUDART_INF, mn = CUDART_INF;
-    int pmx = -1, pmn = -1;
-    if constexpr (std::is_same<T, double>::value) {
-        if (isfinite(Wt.value()) && isfinite(inv))  // warp-uniform: every candidate is finite
-            walk_hits<T, WPL, true>(bm, w0, nzm, cnt, excl, wt, inv, d, Wl, mx, pmx, mn, pmn);
-        else
-            walk_hits<T, WPL, false>(bm, w0, nzm, cnt, excl, wt, inv, d, Wl, mx, pmx, mn, pmn);
-    } else {
-        walk_hits<T, WPL, false>(bm, w0, nzm, cnt, excl, wt, inv, d, Wl, mx, pmx, mn, pmn);
-    }
+    n = __shfl_sync(kFullMask, incl, 31);
+    return incl - cnt;
+}
+// weight of the hits in the lanes before, times inv (0 where there is none)
+template <class T>
+__device__ __forceinline__ T weight_before(const Acc<T>& Wl, int excl, T inv, int lane) {
     Acc<T> W_incl = Wl;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const Acc<T> y = W_incl.shfl_up(o);
         if (lane >= o) W_incl.merge(y);
     }
-    const Acc<T> W_pre = W_incl.shfl_up(1);  // weight of the hits before this lane's
-    const T shift = excl > 0 ? W_pre.scaled_plus(inv, T(0)) : T(0);
+    const Acc<T> W_pre = W_incl.shfl_up(1);
+    return excl > 0 ? W_pre.scaled_plus(inv, T(0)) : T(0);
+}
+
+// Procedure with positions (any weights): every lane walks its hits once and
+// keeps its largest value after a hit (mx at pmx) and smallest before one (mn
+// at pmn) with the lane-local prefix Wl; the weight of the lanes before
+// shifts both by a constant, which leaves their positions unchanged.  The
+// set's total weight Wt (every lane) comes from the marking.  fp64 with
+// finite candidates compares them as integer keys, on the integer pipe
+// instead of the FP64 pipe (the keys order finite doubles as they compare
+// except -0 / +0, and a zero never decides a score).
+template <class T, int WPL>
+__device__ __forceinline__ T set_score_positions(const uint32_t* bmw, int w0, const T* wt,
+                                                 const T* __restrict__ decay, int G, int lane, const Acc<T>& Wt) {
+    const LaneWords<WPL> words(bmw);
+    int n;
+    const int excl = hits_before(words.cnt, lane, n);
+    const T inv = n > 0 ? T(1) / Wt.value() : T(0);
+    const T d = decay[n];
+    Acc<T> Wl;
+    T mx = -CUDART_INF, mn = CUDART_INF;
+    int pmx = -1, pmn = -1;
+    bool ikey = false;
+    long long kmx = 0, kmn = 0;
+    if constexpr (std::is_same<T, double>::value) {
+        ikey = isfinite(Wt.value()) && isfinite(inv);  // every candidate is finite
+        kmx = okey(mx);
+        kmn = okey(mn);
+    }
+    HitWalk<WPL> hit(bmw, w0, words);
+    for (int t = 0; t < words.cnt; t++) {
+        const uint32_t r4 = hit.next();
+        const int r = (int)(r4 >> 2);
+        const T md = -(T)(r - (excl + t)) * d;  // misses before this hit, times the decay
+        const T before = t > 0 ? Wl.scaled_plus(inv, md) : md;
+        Wl.add(weight_at(wt, r4));
+        const T after = Wl.scaled_plus(inv, md);
+        if constexpr (std::is_same<T, double>::value) {
+            if (ikey) {
+                const long long kb = okey(before), ka = okey(after);
+                if (kb < kmn) { kmn = kb; pmn = r - 1; }
+                if (ka > kmx) { kmx = ka; pmx = r; }
+                continue;
+            }
+        }
+        if (before < mn) { mn = before; pmn = r - 1; }
+        if (after > mx) { mx = after; pmx = r; }
+    }
+    if constexpr (std::is_same<T, double>::value) {
+        if (ikey) {
+            mx = okey_value(kmx);
+            mn = okey_value(kmn);
+        }
+    }
+    const T shift = weight_before<T>(Wl, excl, inv, lane);
     mx += shift;
     mn += shift;
     if (lane == 31) {  // end of the list, after the trailing misses
@@ -255,6 +342,66 @@ __device__ __forceinline__ T set_score_direct(uint32_t* bm, int w0, const T* wt,
         consider<T>(ob, op, best, bpos);
     }
     return best;
+}
+
+template <int WPL>  // out of line: seldom taken
+__device__ __noinline__ float set_score_positions_f32(const uint32_t* bmw, int w0, const float* wt,
+                                                      const float* __restrict__ decay, int G, int lane,
+                                                      Acc<float> Wt) {
+    return set_score_positions<float, WPL>(bmw, w0, wt, decay, G, lane, Wt);
+}
+
+// largest positive / most negative value over the warp as bits of their
+// magnitudes (0 where there is none): non-negative floats order as integers
+__device__ __forceinline__ uint32_t warp_top(float v) {
+    return __reduce_max_sync(kFullMask, __float_as_uint(fmaxf(v, 0.f)));
+}
+
+// fp32, direct procedure: the values of set_score_positions without the
+// positions, which decide nothing unless the two extrema tie in magnitude.
+// Every operation on the values is the same, so the scores are the same bits:
+// the miss count times four is exact and so is d / 4, and with hi = lo = 0
+// the first hit's `before` is md itself for a finite inv.
+template <int WPL>
+__device__ __forceinline__ float set_score_direct(const uint32_t* bmw, int w0, const float* wt,
+                                                  const float* __restrict__ decay, int G, int lane,
+                                                  const Acc<float>& Wt) {
+    const LaneWords<WPL> words(bmw);
+    int n;
+    const int excl = hits_before(words.cnt, lane, n);
+    const float inv = n > 0 ? 1.f / Wt.value() : 0.f;
+    const float d = decay[n];
+    if (__all_sync(kFullMask, isfinite(Wt.value()) && isfinite(inv))) {
+        const float d4 = 0.25f * d;
+        constexpr uint32_t kMagic = 0x4b000000u;  // 2^23: adding a count below 2^23 to its bits adds it to its value
+        uint32_t e4 = 4u * (uint32_t)excl - kMagic;
+        const uint32_t end4 = e4 + 4u * (uint32_t)words.cnt;
+        Acc<float> Wl;
+        float mx = -CUDART_INF_F, mn = CUDART_INF_F;
+        HitWalk<WPL> hit(bmw, w0, words);
+#pragma unroll 2  // the sums change registers at every hit: two hits need no moves
+        while (e4 != end4) {
+            const uint32_t r4 = hit.next();
+            const float m4 = __fadd_rn(__uint_as_float(r4 - e4), -8388608.f);  // misses before this hit, times 4
+            const float md = __fmul_rn(-m4, d4);
+            mn = fminf(mn, Wl.scaled_plus(inv, md));
+            Wl.add(weight_at(wt, r4));
+            mx = fmaxf(mx, Wl.scaled_plus(inv, md));
+            e4 += 4u;
+        }
+        const float shift = weight_before<float>(Wl, excl, inv, lane);
+        mx += shift;
+        mn += shift;
+        if (lane == 31) {  // end of the list, after the trailing misses
+            const float tail = -(float)(G - n) * d;
+            mn = fminf(mn, n > 0 ? Wt.scaled_plus(inv, tail) : tail);
+        }
+        const uint32_t up = warp_top(mx), down = warp_top(-mn);
+        if (up > down) return __uint_as_float(up);  // warp-uniform
+        if (down > up) return -__uint_as_float(down);
+        if (up == 0u) return 0.f;
+    }
+    return set_score_positions_f32<WPL>(bmw, w0, wt, decay, G, lane, Wt);
 }
 
 // General procedure (any G, any set size): each lane walks its own word range
@@ -325,6 +472,12 @@ __device__ __noinline__ T set_score_walk(uint32_t* bm, int w0, int w1, const T* 
     return best;
 }
 
+// a member's rank in the direct procedures' bitmap: bit 31 - r % 32
+template <int WPL>
+__device__ __forceinline__ void mark(uint32_t* bm, uint32_t r) {
+    atomicOr(rank_word<WPL>(bm, r), __funnelshift_r(0x80000000u, 0u, r));
+}
+
 // One permutation on the calling CTA: stage its ranks and weights (STAGE 1),
 // its ranks only (STAGE 2, the weights then gathered through L1 / L2), its
 // weights only (STAGE 3, the ranks gathered) or nothing (STAGE 0),
@@ -335,8 +488,7 @@ __device__ __noinline__ T set_score_walk(uint32_t* bm, int w0, int w1, const T* 
 // s_w / s_rank: staging (STAGE), bm: this warp's zeroed bitmap region.
 // Begins and ends with the CTA in step (the staging may be reused after).
 template <class T, class RankT, int WARPS, int STAGE, int WPL>
-__device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G, const int64_t* __restrict__ set_off,
-                                            const int32_t* __restrict__ set_genes,
+__device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G, const EsSets sets,
                                             const int32_t* __restrict__ set_order, const T* __restrict__ decay, int K,
                                             T* __restrict__ es_col, int64_t es_stride, T* s_w, RankT* s_rank,
                                             uint32_t* bm, int* next_set, int part_lo = 0, int part_hi = 1,
@@ -366,39 +518,81 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
         }
         if (slot >= K) break;
         const int k = set_order ? set_order[slot] : slot;
-        const int64_t a = set_off[k];
-        const int m = (int)(set_off[k + 1] - a);  // a set lists fewer than 2^31 members
-        const int32_t* __restrict__ sg = set_genes + a;
-        // mark the members' ranks (duplicates and unknown ids fall away); the
-        // direct procedure also sums the weights of the newly marked ranks
-        Acc<T> Wm;
-        for (int base = 0; base < m; base += 128) {
-            int g[4];
+        T score;
+        if constexpr (WPL > 0) {
+            Acc<T> Wm;
+            const int2 rec = __ldg(sets.rec + k);  // first group of the set's list, members
+            if (rec.y >= 0) {
+                const uint2* __restrict__ list = sets.list + (int64_t)rec.x * 32 + lane;
+                const int full = rec.y >> 7, rem = rec.y & 127;
+#pragma unroll 1
+                for (int i = 0; i < full; i++, list += 32) {
+                    const uint2 q = __ldg(list);
+                    const uint32_t r0 = rk[q.x & 0xffffu], r1 = rk[q.x >> 16];
+                    const uint32_t r2 = rk[q.y & 0xffffu], r3 = rk[q.y >> 16];
+                    const T a0 = wt[r0], a1 = wt[r1], a2 = wt[r2], a3 = wt[r3];
+                    mark<WPL>(bm, r0);
+                    mark<WPL>(bm, r1);
+                    mark<WPL>(bm, r2);
+                    mark<WPL>(bm, r3);
+                    Wm.add(a0);
+                    Wm.add(a1);
+                    Wm.add(a2);
+                    Wm.add(a3);
+                }
+                if (rem) {
+                    const uint2 q = __ldg(list);
+                    const uint32_t g[4] = {q.x & 0xffffu, q.x >> 16, q.y & 0xffffu, q.y >> 16};
+                    uint32_t r[4];
+                    T a[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int idx = base + lane + 32 * i;
-                g[i] = idx < m ? __ldg(sg + idx) : -1;
-            }
+                    for (int i = 0; i < 4; i++) {  // the unused entries of a list are gene 0
+                        r[i] = rk[g[i]];
+                        a[i] = wt[r[i]];
+                    }
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                if (g[i] >= 0 && g[i] < G) {
-                    const uint32_t r = (uint32_t)rk[g[i]];
-                    const uint32_t bit = 1u << (r & 31);
-                    if (WPL > 0) {
-                        if (!(atomicOr(&bm[r >> 5], bit) & bit)) Wm.add(wt[r]);
-                    } else {
-                        atomicOr(&bm[r >> 5], bit);
+                    for (int i = 0; i < 4; i++) {
+                        if (lane + 32 * i < rem) {
+                            mark<WPL>(bm, r[i]);
+                            Wm.add(a[i]);
+                        }
+                    }
+                }
+            } else {
+                // duplicates or unknown ids: the caller's list, each member checked
+                const int64_t a = sets.off[k];
+                const int m = (int)(sets.off[k + 1] - a);  // a set lists fewer than 2^31 members
+                for (int idx = lane; idx < m; idx += 32) {
+                    const int g = __ldg(sets.genes + a + idx);
+                    if (g >= 0 && g < G) {
+                        const uint32_t r = rk[g];
+                        const uint32_t bit = __funnelshift_r(0x80000000u, 0u, r);
+                        if (!(atomicOr(rank_word<WPL>(bm, r), bit) & bit)) Wm.add(wt[r]);
                     }
                 }
             }
-        }
-        __syncwarp();
-        T score;
-        if (WPL > 0) {
+            __syncwarp();
 #pragma unroll
             for (int o = 16; o >= 1; o >>= 1) Wm.merge(Wm.shfl_xor(o));  // the set's weight, every lane
-            score = set_score_direct<T, (WPL > 0 ? WPL : 4)>(bm, lane * WPL, wt, decay, G, lane, Wm);
+            uint32_t* const bmw = bm + lane * lane_stride<WPL>();
+            if constexpr (std::is_same<T, float>::value) {
+                score = set_score_direct<WPL>(bmw, lane * WPL, wt, decay, G, lane, Wm);
+            } else {
+                score = set_score_positions<T, WPL>(bmw, lane * WPL, wt, decay, G, lane, Wm);
+            }
+            clear_words<WPL>(bmw);
         } else {
+            // mark the members' ranks (duplicates and unknown ids fall away)
+            const int64_t a = sets.off[k];
+            const int m = (int)(sets.off[k + 1] - a);
+            for (int idx = lane; idx < m; idx += 32) {
+                const int g = __ldg(sets.genes + a + idx);
+                if (g >= 0 && g < G) {
+                    const uint32_t r = (uint32_t)rk[g];
+                    atomicOr(&bm[r >> 5], 1u << (r & 31));
+                }
+            }
+            __syncwarp();
             score = set_score_walk<T>(bm, w0, w1, wt, decay, G, lane);
         }
         if (lane == 0) es_col[(int64_t)k * es_stride] = score;
@@ -432,15 +626,14 @@ __device__ __forceinline__ void es_smem_layout(unsigned char* smem, int G, int r
 template <class T, class RankT, int WARPS, int STAGE, int WPL>
 __global__ void __launch_bounds__(WARPS * 32)
 es_kernel(const RankT* __restrict__ ranks, const T* __restrict__ sorted_abs, int G, int num_perms,
-          const int64_t* __restrict__ set_off, const int32_t* __restrict__ set_genes,
-          const int32_t* __restrict__ set_order, const T* __restrict__ decay, int K, T* __restrict__ es,
-          int64_t es_stride, int64_t col0, const int* __restrict__ K_dev) {
+          const EsSets sets, const int32_t* __restrict__ set_order, const T* __restrict__ decay, int K,
+          T* __restrict__ es, int64_t es_stride, int64_t col0, const int* __restrict__ K_dev) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int next_set;
     if (K_dev) K = min(K, *K_dev);  // a set list whose length a kernel decided
     if (K <= 0) return;
     const int words = (G + 31) >> 5;
-    const int region = WPL > 0 ? WPL * 32 : words;  // per-warp bitmap words
+    const int region = WPL > 0 ? lane_stride<WPL>() * 32 : words;  // per-warp bitmap words
     T* s_w;
     RankT* s_rank;
     uint32_t* bm;
@@ -451,9 +644,9 @@ es_kernel(const RankT* __restrict__ ranks, const T* __restrict__ sorted_abs, int
     const int full = num_perms / grid;
     for (int i = 0; i < full; i++) {
         const int p = blockIdx.x + i * grid;
-        es_one_perm<T, RankT, WARPS, STAGE, WPL>(ranks + (int64_t)p * G, sorted_abs + (int64_t)p * G, G, set_off,
-                                                  set_genes, set_order, decay, K, es + col0 + p, es_stride, s_w,
-                                                  s_rank, bm, &next_set);
+        es_one_perm<T, RankT, WARPS, STAGE, WPL>(ranks + (int64_t)p * G, sorted_abs + (int64_t)p * G, G, sets,
+                                                  set_order, decay, K, es + col0 + p, es_stride, s_w, s_rank, bm,
+                                                  &next_set);
     }
     // ... then the rem < gridDim.x left over, each cut into `parts` parts
     // (parts * rem a multiple of gridDim.x where K allows); every CTA takes an
@@ -473,9 +666,9 @@ es_kernel(const RankT* __restrict__ ranks, const T* __restrict__ sorted_abs, int
         const int64_t left = hi - lo;
         const int j1 = left < (int64_t)(parts - j0) ? j0 + (int)left : parts;
         const int p = full * grid + (int)q;
-        es_one_perm<T, RankT, WARPS, STAGE, WPL>(ranks + (int64_t)p * G, sorted_abs + (int64_t)p * G, G, set_off,
-                                                  set_genes, set_order, decay, K, es + col0 + p, es_stride, s_w,
-                                                  s_rank, bm, &next_set, j0, j1, parts);
+        es_one_perm<T, RankT, WARPS, STAGE, WPL>(ranks + (int64_t)p * G, sorted_abs + (int64_t)p * G, G, sets,
+                                                  set_order, decay, K, es + col0 + p, es_stride, s_w, s_rank, bm,
+                                                  &next_set, j0, j1, parts);
         lo += j1 - j0;
     }
 }
@@ -493,7 +686,7 @@ es_batch_kernel(const EsTask<T>* __restrict__ tasks, const int64_t* __restrict__
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int next_set;
     __shared__ long long s_item;
-    const int region = WPL > 0 ? WPL * 32 : (Gmax + 31) >> 5;
+    const int region = WPL > 0 ? lane_stride<WPL>() * 32 : (Gmax + 31) >> 5;
     T* s_w;
     RankT* s_rank;
     uint32_t* bm;
@@ -513,14 +706,15 @@ es_batch_kernel(const EsTask<T>* __restrict__ tasks, const int64_t* __restrict__
         const EsTask<T>& tk = tasks[lo];
         const int64_t p = item - (lo > 0 ? item_end[lo - 1] : 0);
         const RankT* rk = static_cast<const RankT*>(tk.ranks) + p * tk.G;
-        es_one_perm<T, RankT, WARPS, STAGE, WPL>(rk, tk.sorted + p * tk.G, tk.G, tk.off, tk.genes, tk.order,
-                                                  tk.decay, tk.K, tk.es + tk.col0 + p, tk.stride, s_w, s_rank, bm,
-                                                  &next_set);
+        es_one_perm<T, RankT, WARPS, STAGE, WPL>(rk, tk.sorted + p * tk.G, tk.G, tk.sets, tk.order, tk.decay, tk.K,
+                                                  tk.es + tk.col0 + p, tk.stride, s_w, s_rank, bm, &next_set);
     }
 }
 
-// words of a warp's bitmap region: WPL*32 for the register procedure
-inline int es_region_words(int G, int wpl) { return wpl > 0 ? wpl * 32 : (G + 31) >> 5; }
+// words of a warp's bitmap region
+inline int es_region_words(int G, int wpl) {
+    return wpl > 0 ? (wpl % 16 == 0 ? wpl + 4 : wpl) * 32 : (G + 31) >> 5;
+}
 
 inline int es_wpl(int G, bool ranks16) {
     const int need = (((G + 31) >> 5) + 31) >> 5;
@@ -537,9 +731,25 @@ size_t es_smem_bytes(int G) {
     return s + sizeof(uint32_t) * (size_t)region * WARPS;
 }
 
+// Whether a configuration may run.  The first pass over the candidates leaves
+// an unstaged one at least 64 KB of the SM's memory as L1: its gathers of
+// ranks and weights live there (60,000 genes, 304 x 500 scores: 24 warps
+// with 28 KB of L1 772 us, 16 warps with 92 KB 477; 45,000: 32 warps 731, 24
+// warps 380), so more warps are only worth it while the bitmaps stay below
+// 164 KB.
+inline bool es_fits(int warps, int stage, size_t smem, int wpl, size_t cap, bool leave_l1, const EsTuning& tune) {
+    constexpr size_t kLeavesL1 = 163 * 1024;
+    if (smem > cap) return false;
+    if ((stage >= 2 || warps == 24) && wpl < 24) return false;
+    if (stage == 1 && wpl >= 40) return false;
+    if (tune.warps && tune.warps != warps) return false;
+    if (tune.stage >= 0 && tune.stage != stage) return false;
+    return !(leave_l1 && stage == 0 && smem > kLeavesL1);
+}
+
 template <class T, class RankT, int WARPS, int STAGE, int WPL>
-cudaError_t launch_es_v(const RankT* ranks, const T* sorted_abs, int G, int P, const int64_t* off,
-                        const int32_t* genes, const int32_t* order, const T* decay, int K, T* es, int64_t stride,
+cudaError_t launch_es_v(const RankT* ranks, const T* sorted_abs, int G, int P, const EsSets& sets,
+                        const int32_t* order, const T* decay, int K, T* es, int64_t stride,
                         int64_t col0, int grid, cudaStream_t st, const int* K_dev) {
     const size_t smem = es_smem_bytes<T, RankT, WARPS, STAGE>(G);
     auto kern = es_kernel<T, RankT, WARPS, STAGE, WPL>;
@@ -550,59 +760,59 @@ cudaError_t launch_es_v(const RankT* ranks, const T* sorted_abs, int G, int P, c
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidValue;
     grid *= per_sm;
-    kern<<<grid, WARPS * 32, smem, st>>>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0,
+    kern<<<grid, WARPS * 32, smem, st>>>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0,
                                          K_dev);
     launches_add(1);
     return cudaGetLastError();
 }
 
 template <class T, class RankT, int WARPS, int STAGE>
-cudaError_t launch_es_w(const RankT* ranks, const T* sorted_abs, int G, int P, const int64_t* off,
-                        const int32_t* genes, const int32_t* order, const T* decay, int K, T* es, int64_t stride,
+cudaError_t launch_es_w(const RankT* ranks, const T* sorted_abs, int G, int P, const EsSets& sets,
+                        const int32_t* order, const T* decay, int K, T* es, int64_t stride,
                         int64_t col0, int grid, cudaStream_t st, const int* K_dev) {
     // words per lane for the register-resident list procedure (u16 positions);
     // 32-bit ranks (G > 65,536) always take the general procedure
     if constexpr (sizeof(RankT) == 4) {
         if (STAGE >= 2) return cudaErrorInvalidValue;
-        return launch_es_v<T, RankT, WARPS, STAGE, 0>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride,
+        return launch_es_v<T, RankT, WARPS, STAGE, 0>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride,
                                                       col0, grid, st, K_dev);
     } else if constexpr (STAGE >= 2 || WARPS == 24) {  // partial staging / 24 warps: the large-G classes
         switch (es_wpl(G, true)) {
-            case 24: return launch_es_v<T, RankT, WARPS, STAGE, 24>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 32: return launch_es_v<T, RankT, WARPS, STAGE, 32>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 40: return launch_es_v<T, RankT, WARPS, STAGE, 40>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 48: return launch_es_v<T, RankT, WARPS, STAGE, 48>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 64: return launch_es_v<T, RankT, WARPS, STAGE, 64>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 24: return launch_es_v<T, RankT, WARPS, STAGE, 24>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 32: return launch_es_v<T, RankT, WARPS, STAGE, 32>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 40: return launch_es_v<T, RankT, WARPS, STAGE, 40>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 48: return launch_es_v<T, RankT, WARPS, STAGE, 48>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 64: return launch_es_v<T, RankT, WARPS, STAGE, 64>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
             default: return cudaErrorInvalidValue;
         }
     } else {
         switch (es_wpl(G, true)) {
-            case 4: return launch_es_v<T, RankT, WARPS, STAGE, 4>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 8: return launch_es_v<T, RankT, WARPS, STAGE, 8>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 12: return launch_es_v<T, RankT, WARPS, STAGE, 12>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 16: return launch_es_v<T, RankT, WARPS, STAGE, 16>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 20: return launch_es_v<T, RankT, WARPS, STAGE, 20>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 24: return launch_es_v<T, RankT, WARPS, STAGE, 24>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
-            case 32: return launch_es_v<T, RankT, WARPS, STAGE, 32>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 4: return launch_es_v<T, RankT, WARPS, STAGE, 4>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 8: return launch_es_v<T, RankT, WARPS, STAGE, 8>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 12: return launch_es_v<T, RankT, WARPS, STAGE, 12>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 16: return launch_es_v<T, RankT, WARPS, STAGE, 16>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 20: return launch_es_v<T, RankT, WARPS, STAGE, 20>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 24: return launch_es_v<T, RankT, WARPS, STAGE, 24>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
+            case 32: return launch_es_v<T, RankT, WARPS, STAGE, 32>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
             case 40:  // the staging of ranks and weights never fits beside these regions
-                if constexpr (STAGE == 0) return launch_es_v<T, RankT, WARPS, 0, 40>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
+                if constexpr (STAGE == 0) return launch_es_v<T, RankT, WARPS, 0, 40>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
                 return cudaErrorInvalidValue;
             case 48:
-                if constexpr (STAGE == 0) return launch_es_v<T, RankT, WARPS, 0, 48>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
+                if constexpr (STAGE == 0) return launch_es_v<T, RankT, WARPS, 0, 48>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
                 return cudaErrorInvalidValue;
             case 64:
-                if constexpr (STAGE == 0) return launch_es_v<T, RankT, WARPS, 0, 64>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, K_dev);
+                if constexpr (STAGE == 0) return launch_es_v<T, RankT, WARPS, 0, 64>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
                 return cudaErrorInvalidValue;
             default: break;
         }
-        return launch_es_v<T, RankT, WARPS, STAGE, 0>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride,
+        return launch_es_v<T, RankT, WARPS, STAGE, 0>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride,
                                                       col0, grid, st, K_dev);
     }
 }
 
 template <class T, class RankT>
-cudaError_t launch_es_t(const RankT* ranks, const T* sorted_abs, int G, int P, const int64_t* off,
-                        const int32_t* genes, const int32_t* order, const T* decay, int K, T* es, int64_t stride,
+cudaError_t launch_es_t(const RankT* ranks, const T* sorted_abs, int G, int P, const EsSets& sets,
+                        const int32_t* order, const T* decay, int K, T* es, int64_t stride,
                         int64_t col0, EsTuning tune, cudaStream_t st, const int* K_dev) {
     int dev = 0, max_smem = 0, sms = 1;
     cudaGetDevice(&dev);
@@ -610,33 +820,28 @@ cudaError_t launch_es_t(const RankT* ranks, const T* sorted_abs, int G, int P, c
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t cap = (size_t)max_smem - 64;  // static shared counter
     const int grid = sms;  // times the resident CTAs per SM; the last round's permutations are split by sets
-    // candidates in the automatic order: 32 warps first (staging ranks and
-    // weights, then weights only, 24 warps with weights only, 32 with ranks
-    // only, 32 with none), then fewer warps -- warps count for more than
-    // staging (measured on 24,000-40,000 genes); the partial stagings are for
+    // candidates in the automatic order (es_fits): staging the weights first,
+    // 32 warps, then 24; then nothing staged.  The partial stagings are for
     // the large-G classes (24-64 bitmap words per lane)
     struct Cand { int warps; int stage; size_t smem; };
     const Cand cands[] = {{32, 1, es_smem_bytes<T, RankT, 32, 1>(G)},
                           {32, 3, es_smem_bytes<T, RankT, 32, 3>(G)},
                           {24, 3, es_smem_bytes<T, RankT, 24, 3>(G)},
-                          {32, 2, es_smem_bytes<T, RankT, 32, 2>(G)},
                           {32, 0, es_smem_bytes<T, RankT, 32, 0>(G)},
                           {24, 0, es_smem_bytes<T, RankT, 24, 0>(G)},
+                          {16, 0, es_smem_bytes<T, RankT, 16, 0>(G)},
+                          {32, 2, es_smem_bytes<T, RankT, 32, 2>(G)},
                           {16, 1, es_smem_bytes<T, RankT, 16, 1>(G)},
                           {24, 2, es_smem_bytes<T, RankT, 24, 2>(G)},
                           {16, 2, es_smem_bytes<T, RankT, 16, 2>(G)},
                           {8, 1, es_smem_bytes<T, RankT, 8, 1>(G)},
-                          {16, 0, es_smem_bytes<T, RankT, 16, 0>(G)},
                           {8, 0, es_smem_bytes<T, RankT, 8, 0>(G)}};
     const int wpl = es_wpl(G, sizeof(RankT) == 2);
+    for (int pass = 0; pass < 2; pass++)
     for (const Cand& c : cands) {
-        if (c.smem > cap) continue;
-        if ((c.stage >= 2 || c.warps == 24) && wpl < 24) continue;
-        if (c.stage == 1 && wpl >= 40) continue;
-        if (tune.warps && tune.warps != c.warps) continue;
-        if (tune.stage >= 0 && tune.stage != c.stage) continue;
+        if (!es_fits(c.warps, c.stage, c.smem, wpl, cap, pass == 0, tune)) continue;
 #define GSEA_ES(W, S) \
-    return launch_es_w<T, RankT, W, S>(ranks, sorted_abs, G, P, off, genes, order, decay, K, es, stride, col0, grid, st, \
+    return launch_es_w<T, RankT, W, S>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, \
                                        K_dev)
         if (c.warps == 32 && c.stage == 1) GSEA_ES(32, 1);
         if (c.warps == 16 && c.stage == 1) GSEA_ES(16, 1);
@@ -728,21 +933,18 @@ cudaError_t launch_es_batch(const EsTask<T>* tasks, const int64_t* item_end, int
     const Cand cands[] = {{32, 1, es_smem_bytes<T, uint16_t, 32, 1>(Gmax)},
                           {32, 3, es_smem_bytes<T, uint16_t, 32, 3>(Gmax)},
                           {24, 3, es_smem_bytes<T, uint16_t, 24, 3>(Gmax)},
-                          {32, 2, es_smem_bytes<T, uint16_t, 32, 2>(Gmax)},
                           {32, 0, es_smem_bytes<T, uint16_t, 32, 0>(Gmax)},
                           {24, 0, es_smem_bytes<T, uint16_t, 24, 0>(Gmax)},
+                          {16, 0, es_smem_bytes<T, uint16_t, 16, 0>(Gmax)},
+                          {32, 2, es_smem_bytes<T, uint16_t, 32, 2>(Gmax)},
                           {16, 1, es_smem_bytes<T, uint16_t, 16, 1>(Gmax)},
                           {24, 2, es_smem_bytes<T, uint16_t, 24, 2>(Gmax)},
                           {16, 2, es_smem_bytes<T, uint16_t, 16, 2>(Gmax)},
                           {8, 1, es_smem_bytes<T, uint16_t, 8, 1>(Gmax)},
-                          {16, 0, es_smem_bytes<T, uint16_t, 16, 0>(Gmax)},
                           {8, 0, es_smem_bytes<T, uint16_t, 8, 0>(Gmax)}};
+    for (int pass = 0; pass < 2; pass++)
     for (const Cand& c : cands) {
-        if (c.smem > cap) continue;
-        if ((c.stage >= 2 || c.warps == 24) && wpl < 24) continue;
-        if (c.stage == 1 && wpl >= 40) continue;
-        if (tune.warps && tune.warps != c.warps) continue;
-        if (tune.stage >= 0 && tune.stage != c.stage) continue;
+        if (!es_fits(c.warps, c.stage, c.smem, wpl, cap, pass == 0, tune)) continue;
 #define GSEA_ESB(W, S) return launch_es_batch_w<T, W, S>(tasks, item_end, ntasks, nitems, counter, Gmax, wpl, st)
         if (c.warps == 32 && c.stage == 1) GSEA_ESB(32, 1);
         if (c.warps == 16 && c.stage == 1) GSEA_ESB(16, 1);
@@ -763,15 +965,14 @@ cudaError_t launch_es_batch(const EsTask<T>* tasks, const int64_t* item_end, int
 
 template <class T>
 cudaError_t launch_es(const void* ranks, bool ranks16, const T* sorted_abs, int G, int num_perms,
-                      const int64_t* set_offsets, const int32_t* set_genes, const int32_t* set_order,
-                      const T* decay, int K, T* es, int64_t es_stride, int64_t perm_col0, cudaStream_t st,
+                      const EsSets& sets, const int32_t* set_order, const T* decay, int K, T* es, int64_t es_stride, int64_t perm_col0, cudaStream_t st,
                       EsTuning tune, const int* K_dev) {
     if (num_perms <= 0 || K <= 0) return cudaSuccess;
     if (ranks16)
-        return launch_es_t<T, uint16_t>(static_cast<const uint16_t*>(ranks), sorted_abs, G, num_perms, set_offsets,
-                                        set_genes, set_order, decay, K, es, es_stride, perm_col0, tune, st, K_dev);
-    return launch_es_t<T, uint32_t>(static_cast<const uint32_t*>(ranks), sorted_abs, G, num_perms, set_offsets,
-                                    set_genes, set_order, decay, K, es, es_stride, perm_col0, tune, st, K_dev);
+        return launch_es_t<T, uint16_t>(static_cast<const uint16_t*>(ranks), sorted_abs, G, num_perms, sets,
+                                        set_order, decay, K, es, es_stride, perm_col0, tune, st, K_dev);
+    return launch_es_t<T, uint32_t>(static_cast<const uint32_t*>(ranks), sorted_abs, G, num_perms, sets,
+                                    set_order, decay, K, es, es_stride, perm_col0, tune, st, K_dev);
 }
 
 // decay[n] = (T)(1.0 / (G - n)) for n < G, 0 for n = G: the miss step of a

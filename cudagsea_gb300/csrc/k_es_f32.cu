@@ -5,9 +5,65 @@ namespace gsea {
 
 int es_size_class(int G) { return es_wpl(G, G <= 65536); }
 
-template cudaError_t launch_es<float>(const void*, bool, const float*, int, int, const int64_t*, const int32_t*,
-                                      const int32_t*, const float*, int, float*, int64_t, int64_t, cudaStream_t,
-                                      EsTuning, const int*);
+namespace {
+// The sets' marking lists (EsSets): one warp per set writes its groups and
+// finds duplicates and unknown ids in a bitmap of the genes.  A set's list
+// starts at group floor(offset / 128) + k, which leaves every set room for
+// its last, partial group without a scan over the sets.
+constexpr int kListWarps = 4;
+__global__ void __launch_bounds__(32 * kListWarps)
+es_lists_kernel(const int64_t* __restrict__ off, const int32_t* __restrict__ genes, int K, int G,
+                int2* __restrict__ rec, uint2* __restrict__ list) {
+    extern __shared__ uint32_t seen[];  // [kListWarps][(G + 31) / 32]
+    const int words = (G + 31) >> 5;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t* const bm = seen + warp * words;
+    for (int w = lane; w < words; w += 32) bm[w] = 0u;
+    const int k = blockIdx.x * kListWarps + warp;
+    if (k >= K) return;  // the whole warp; no block barrier below
+    __syncwarp();
+    const int64_t a = off[k];
+    const int64_t m = off[k + 1] - a;
+    const int64_t first = a / 128 + k;
+    bool bad = m > INT_MAX || first > INT_MAX;
+    for (int64_t base = 0; base < m; base += 128) {
+        uint32_t e[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int64_t idx = base + 32 * i + lane;
+            e[i] = 0u;
+            if (idx < m) {
+                const int g = genes[a + idx];
+                if (g < 0 || g >= G) {
+                    bad = true;
+                } else {
+                    e[i] = (uint32_t)g;
+                    const uint32_t bit = 1u << (g & 31);
+                    if (atomicOr(&bm[g >> 5], bit) & bit) bad = true;
+                }
+            }
+        }
+        list[(first + base / 128) * 32 + lane] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
+    }
+    bad = __any_sync(kFullMask, bad);
+    if (lane == 0) rec[k] = make_int2(bad ? 0 : (int)first, bad ? -1 : (int)m);
+}
+}  // namespace
+
+size_t es_list_bytes(int64_t K, int64_t nnz) { return ((size_t)(nnz / 128 + K) + 1) * 128 * sizeof(uint16_t); }
+
+cudaError_t launch_es_lists(const int64_t* off, const int32_t* genes, int K, int G, int2* rec, uint2* list,
+                            cudaStream_t st) {
+    if (K <= 0) return cudaSuccess;
+    if (G > 65536) return cudaErrorInvalidValue;
+    const size_t smem = sizeof(uint32_t) * kListWarps * (size_t)((G + 31) / 32);
+    es_lists_kernel<<<(K + kListWarps - 1) / kListWarps, 32 * kListWarps, smem, st>>>(off, genes, K, G, rec, list);
+    launches_add(1);
+    return cudaGetLastError();
+}
+
+template cudaError_t launch_es<float>(const void*, bool, const float*, int, int, const EsSets&, const int32_t*,
+                                      const float*, int, float*, int64_t, int64_t, cudaStream_t, EsTuning, const int*);
 template cudaError_t launch_es_batch<float>(const EsTask<float>*, const int64_t*, int, int64_t, unsigned long long*,
                                             int, int, EsTuning, cudaStream_t);
 template cudaError_t launch_decay_table<float>(int, float*, cudaStream_t);

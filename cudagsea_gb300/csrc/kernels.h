@@ -79,10 +79,23 @@ struct EsTuning {
     int warps = 0;
     int stage = -1;
 };
+// The gene sets of a plan: the caller's CSR (offsets [K+1], genes) and the
+// lists the kernel marks from (launch_es_lists; G <= 65,536).  Set k's list
+// starts at group rec[k].x: groups of 128 16-bit gene ids, entry 4*lane + i
+// of a group the set's member 32*i + lane of it; rec[k].y members, or -1 when
+// the set lists a gene twice or an unknown id (the CSR is then read).
+struct EsSets {
+    const int64_t* off;
+    const int32_t* genes;
+    const int2* rec;
+    const uint2* list;
+};
+size_t es_list_bytes(int64_t K, int64_t nnz);
+cudaError_t launch_es_lists(const int64_t* off, const int32_t* genes, int K, int G, int2* rec, uint2* list,
+                            cudaStream_t st);
 template <class T>
 cudaError_t launch_es(const void* ranks, bool ranks16, const T* sorted_abs, int G, int num_perms,
-                      const int64_t* set_offsets, const int32_t* set_genes, const int32_t* set_order,
-                      const T* decay, int K, T* es, int64_t es_stride, int64_t perm_col0, cudaStream_t st,
+                      const EsSets& sets, const int32_t* set_order, const T* decay, int K, T* es, int64_t es_stride, int64_t perm_col0, cudaStream_t st,
                       EsTuning tune = EsTuning(), const int* K_dev = nullptr);
 // (K_dev: when not null, the number of sets is min(K, *K_dev), read on the
 // device -- a set list whose length a kernel decided)
@@ -96,8 +109,7 @@ template <class T>
 struct EsTask {
     const void* ranks;
     const T* sorted;
-    const int64_t* off;
-    const int32_t* genes;
+    EsSets sets;
     const int32_t* order;
     const T* decay;
     T* es;

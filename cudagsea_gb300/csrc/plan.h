@@ -51,6 +51,8 @@ struct gsea_plan_s {
     uint8_t* labels = nullptr;
     int64_t* set_off = nullptr;
     int32_t* set_genes = nullptr;
+    int2* set_rec = nullptr;           // marking lists of the sets (gsea::EsSets), G <= 65,536
+    uint2* set_list = nullptr;
     int32_t* set_order = nullptr;      // sets by decreasing size, for the ES kernel
     std::vector<int32_t> h_set_order;  // host staging of set_order
     std::vector<int64_t> h_set_size;   // members of each set (after mapping)
@@ -111,6 +113,8 @@ struct gsea_plan_s {
 };
 
 namespace gsea {
+struct EsSets;
+EsSets plan_sets(const gsea_plan_s* p);
 // Scores permutations [lo, hi) (global indices perm_offset + lo ...) of the
 // sets set_list[0..n_sets) into columns lo..hi-1 of the plan's ES matrix
 // (row stride num_perms).  No statistics.

@@ -131,8 +131,8 @@ int autotune_t(gsea_plan_s* p, int64_t n64, unsigned stages, gsea_tuning* best_o
             et.stage = stage;
             const float ms = time_best(
                 [&]() {
-                    return gsea::launch_es<T>(p->ranks, p->ranks16, static_cast<const T*>(p->sorted), G, n, p->set_off,
-                                              p->set_genes, p->set_order, static_cast<const T*>(p->decay), K,
+                    return gsea::launch_es<T>(p->ranks, p->ranks16, static_cast<const T*>(p->sorted), G, n,
+                                              gsea::plan_sets(p), p->set_order, static_cast<const T*>(p->decay), K,
                                               static_cast<T*>(p->es), c.num_perms, 0, st, et);
                 },
                 st, t);
