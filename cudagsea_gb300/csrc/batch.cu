@@ -8,8 +8,7 @@
 //   2. the metric: in the tensor-core form one launch each of the label
 //      operand and the tcgen05 class statistics per metric family (one
 //      family when all instances share a metric); in the plain form one
-//      launch per metric and kernel path (exact, or packed with 4 or 8
-//      permutations per thread);
+//      launch per metric (and rounds of a warp, as tuned);
 //   3. the sort: one launch per bucket-sort class, then one per radix class
 //      (keys per thread, one CTA or a two-CTA cluster per permutation) for
 //      the permutations the bucket sort declined; instances beyond the
@@ -195,8 +194,7 @@ int build_multi(gsea_batch_s* b, Multi<gsea::StatsTask<T>>& stats) {
             mt.num_perms = (int)p->pb;
             mt.nA = (T)p->nA;
             mt.nB = (T)p->nB;
-            const int key = gsea::metric_multi_key<T>(c.metric, mt.S, mt.words, p->fast_ok != nullptr,
-                                                      p->tuning.metric_pb);
+            const int key = gsea::metric_multi_key<T>(c.metric, p->tuning.metric_pb);
             auto it = metric_at.find(key);
             if (it == metric_at.end()) {
                 it = metric_at.emplace(key, metrics.size()).first;

@@ -15,15 +15,24 @@
 // accumulators use their default biased=true).  Every product is rounded
 // before it is added (Exact<T>), matching the reference's CPU arithmetic.
 //
-// Work decomposition (GB300): a thread owns one gene and PB permutations.
-// Each expression value x[s][g] is loaded once per PB permutations (coalesced
-// across the genes of a warp, patient-major table) and the class bit of each
-// permutation is a warp-uniform bit of a shared-memory mask word, so the
-// class selection never diverges.
+// Work decomposition (GB300).  The class of a sample is the same for every
+// gene, so a warp owns a few permutations and its lanes the genes: the class
+// bits of the samples select one of sixteen code paths (one indirect branch,
+// never divergent), and a path updates each permutation's statistics of the
+// sample's own class and nothing else -- no selects, no arithmetic with 0/1
+// weights on the other class.  That halves the FP32 work of the selecting
+// form for the two-pass metrics (4 operations per gene, sample and
+// permutation instead of 8); the FP64 work is the operations themselves.
+// fp32 lanes hold their genes as pairs, updated by the paired FP32
+// instructions.  The warps of a block share a tile of the expression table,
+// copied to shared memory 32 samples at a time (cp.async, two buffers), so
+// the table is read from L2 once per block of 16 (fp32) or 32 permutations
+// and pass.
 #pragma once
 #include <algorithm>
 #include <type_traits>
 
+#include "bulk.cuh"
 #include "common.cuh"
 #include "kernels.h"
 
@@ -32,13 +41,42 @@ namespace gsea {
 enum AccKind { ACC_NAIVE, ACC_KAHAN, ACC_ONEPASS, ACC_TWOPASS, ACC_KNUTH, ACC_OVERKILL };
 enum CombKind { COMB_DIFF, COMB_RATIO, COMB_LOG2, COMB_S2N, COMB_TTEST };
 
-template <class T, int COMB>
-__device__ __forceinline__ T combine(T mA, T vA, T nA, T mB, T vB, T nB) {
+// Division by a class size: the correctly rounded quotient from the rounded
+// reciprocal and one exact remainder (Markstein's method; a quotient by an
+// integer below 2^13 is never close enough to a rounding boundary for the
+// remainder's correction to decide it wrongly).  Values whose remainder could
+// leave the normal range are divided by the general operation.
+template <class T>
+struct ClassSize {
+    T n;
+    __device__ __forceinline__ explicit ClassSize(T v) : n(v) {}
+    __device__ __forceinline__ T divides(T x) const { return Exact<T>::div(x, n); }
+};
+template <>
+struct ClassSize<float> {
+    float n, r;
+    __device__ __forceinline__ explicit ClassSize(float v) {
+        n = v;
+        r = __frcp_rn(v);
+    }
+    __device__ __forceinline__ float divides(float x) const {
+        const float q = __fmul_rn(x, r);
+        const float f = __fmaf_rn(__fmaf_rn(-q, n, x), r, q);
+        const float ax = fabsf(x);
+        if ((ax > 1e-25f && ax < 1e30f) || __float_as_uint(x) == 0u) return f;
+        return general(x, n);
+    }
+    static __device__ __noinline__ float general(float x, float n) { return __fdiv_rn(x, n); }
+};
+
+template <class T>
+__device__ __forceinline__ T combine(int comb, T mA, T vA, const ClassSize<T>& nA, T mB, T vB,
+                                     const ClassSize<T>& nB) {
     using E = Exact<T>;
-    if (COMB == COMB_DIFF) return E::sub(mA, mB);
-    if (COMB == COMB_RATIO) return E::div(mA, mB);
-    if (COMB == COMB_LOG2) return E::log2q(E::div(mA, mB));
-    if (COMB == COMB_S2N) {
+    if (comb == COMB_DIFF) return E::sub(mA, mB);
+    if (comb == COMB_RATIO) return E::div(mA, mB);
+    if (comb == COMB_LOG2) return E::log2q(E::div(mA, mB));
+    if (comb == COMB_S2N) {
         T sA = E::sqrt(vA), sB = E::sqrt(vB);
         const T lowA = E::low(0.2, cuabs(mA));
         const T lowB = E::low(0.2, cuabs(mB));
@@ -52,7 +90,7 @@ __device__ __forceinline__ T combine(T mA, T vA, T nA, T mB, T vB, T nB) {
     const T lowB = E::low(0.04, cuabs(mB));
     wA = lowA < wA ? wA : lowA;
     wB = lowB < wB ? wB : lowB;
-    return E::div(E::sub(mA, mB), E::sqrt(E::add(E::div(wA, nA), E::div(wB, nB))));
+    return E::div(E::sub(mA, mB), E::sqrt(E::add(nA.divides(wA), nB.divides(wB))));
 }
 
 // NaN keys (0/0 in the ratio metrics, log of a negative mean, ...) are
@@ -64,493 +102,649 @@ __device__ __forceinline__ double canonical_nan(double v) {
     return v != v ? __longlong_as_double(0x7fffffffffffffffll) : v;
 }
 
-// Exact, predicated form: every class update is a conditional operation, as
-// in the reference, so it is bit-exact for any input including inf / NaN.
-// Called by one thread per gene with the block's masks in shared memory.
-template <int ACC, int COMB, class T, int PB>
-__device__ __forceinline__ void metric_exact(const T* __restrict__ X, int G, int S, const uint32_t* sm_masks,
-                                             int words, int num_perms, int p0, T nA, T nB, T* __restrict__ keys,
-                                             int g) {
+// A lane's genes as vectors: pairs of floats (paired FP32 instructions, each
+// half rounded on its own), single doubles.
+template <class T> struct Vec;
+template <> struct Vec<float> {
+    using V = unsigned long long;
+    static constexpr int kLanes = 2;
+    static __device__ __forceinline__ V zero() { return 0ull; }
+    static __device__ __forceinline__ V pack(const float* f) {
+        V r;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(f[0]), "f"(f[1]));
+        return r;
+    }
+    static __device__ __forceinline__ void unpack(V v, float* f) {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(f[0]), "=f"(f[1]) : "l"(v));
+    }
+    static __device__ __forceinline__ V add(V a, V b) {
+        V d;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+        return d;
+    }
+    static __device__ __forceinline__ V sub(V a, V b) {
+        V d;
+        asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+        return d;
+    }
+    static __device__ __forceinline__ V mul(V a, V b) {
+        V d;
+        asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+        return d;
+    }
+    // acc + prod for a product of mul(): the assembler fuses a paired multiply
+    // and add into one rounding (it does not for the scalar instructions), but
+    // not a multiply into a multiply-add by a `one` it does not know
+    static __device__ __forceinline__ V add_product(V acc, V prod, V one) {
+        V d;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(one), "l"(prod), "l"(acc));
+        return d;
+    }
+    static __device__ __forceinline__ V runtime_one() {
+        const float f[2] = {(float)blockDim.z, (float)blockDim.z};  // 1
+        return pack(f);
+    }
+};
+template <> struct Vec<double> {
+    using V = double;
+    static constexpr int kLanes = 1;
+    static __device__ __forceinline__ V zero() { return 0.0; }
+    static __device__ __forceinline__ V pack(const double* f) { return f[0]; }
+    static __device__ __forceinline__ void unpack(V v, double* f) { f[0] = v; }
+    static __device__ __forceinline__ V add(V a, V b) { return __dadd_rn(a, b); }
+    static __device__ __forceinline__ V sub(V a, V b) { return __dsub_rn(a, b); }
+    static __device__ __forceinline__ V mul(V a, V b) { return __dmul_rn(a, b); }
+    static __device__ __forceinline__ V add_product(V acc, V prod, V) { return __dadd_rn(acc, prod); }
+    static __device__ __forceinline__ V runtime_one() { return 1.0; }
+};
+
+// permutations of a warp, warps of a block (they share a tile) and samples
+// copied at a time
+template <class T>
+constexpr int metric_q() { return sizeof(T) == 4 ? 2 : 4; }
+constexpr int kMaxWarps = 8;
+// resident blocks the registers are kept for
+template <int ACC, class T>
+constexpr int metric_blocks() {
+    return sizeof(T) == 8 ? 2 : ACC == ACC_OVERKILL || ACC == ACC_KNUTH ? 3 : 4;
+}
+constexpr int kChunk = 32;
+
+template <int ACC, class T>
+constexpr int metric_vecs() { return sizeof(T) == 8 ? 1 : 2; }  // vectors per lane
+template <int ACC, class T>
+constexpr int metric_genes() { return 32 * metric_vecs<ACC, T>() * Vec<T>::kLanes; }  // genes of a tile
+template <int ACC, class T>
+constexpr size_t metric_smem(int warps, int S) {
+    return sizeof(T) * metric_genes<ACC, T>() * (2 * kChunk + (size_t)warps) + (size_t)warps * S;
+}
+
+// one copy of BYTES (4, 8, 16), both addresses aligned to it
+template <int BYTES>
+__device__ __forceinline__ void async_copy(uint32_t dst, const void* src) {
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+
+// ---- the samples of the paired fp32 statistics, as one assembly loop -------
+// Two samples at a time: an indirect branch on their four class bits (two
+// samples, two permutations) to one of sixteen cases, each updating its
+// accumulators in place.  In assembly, loop and all, because the compiler
+// copies every accumulator where the cases meet (written as a C++ switch: 55
+// instructions for what takes 24).  The branch has a long latency: two
+// vectors a lane (128 genes a warp) leave registers for 32 warps an SM, which
+// hide it better than four vectors and 20 warps (20,000 genes x 200 samples x
+// 1,000 permutations 912 against 980 us, 2,000 x 40 x 1,024 43 against 54).
+// Operand numbers: statistics of class, permutation and vector M_ 0-7, W_
+// 8-15, U_ 16-23; X_ the loaded vector of a sample.
+#define GM_0A0(OP) OP(0, 8, 16, 0) OP(1, 9, 17, 1)
+#define GM_0A1(OP) OP(2, 10, 18, 0) OP(3, 11, 19, 1)
+#define GM_0B0(OP) OP(4, 12, 20, 0) OP(5, 13, 21, 1)
+#define GM_0B1(OP) OP(6, 14, 22, 0) OP(7, 15, 23, 1)
+#define GM_1A0(OP) OP(0, 8, 16, 2) OP(1, 9, 17, 3)
+#define GM_1A1(OP) OP(2, 10, 18, 2) OP(3, 11, 19, 3)
+#define GM_1B0(OP) OP(4, 12, 20, 2) OP(5, 13, 21, 3)
+#define GM_1B1(OP) OP(6, 14, 22, 2) OP(7, 15, 23, 3)
+#define GM_CASE(N, P0, P1, P2, P3) "C" #N ":\n" P0 P1 P2 P3 "bra.uni NEXT;\n"
+#define GM_LOAD(XP, AT, A, B) "ld.shared.v2.b64 {x" #A ", x" #B "}, [%" #XP "+" #AT "];\n"
+// rows of 128 genes: 512 bytes
+// operands PP, XP, N: addresses of the class bits and of the lane's vectors, pairs of samples
+#define GM_LOOP(OP, PP, XP, N)                                                                                \
+    "{\n .reg .b64 d, e, x0, x1, x2, x3;\n .reg .u32 bits;\n .reg .pred more;\n"                    \
+    " TS: .branchtargets C0, C1, C2, C3, C4, C5, C6, C7, C8, C9, C10, C11, C12, C13, C14, C15;\n"               \
+    "LOOP: ld.shared.u8 bits, [%" #PP "];\n" GM_LOAD(XP, 0, 0, 1) GM_LOAD(XP, 512, 2, 3)                          \
+    " add.u32 %" #PP ", %" #PP ", 2;\n add.u32 %" #XP ", %" #XP ", 1024;\n sub.u32 %" #N ", %" #N ", 1;\n" \
+    " brx.idx.uni bits, TS;\n"                                                                                   \
+    GM_CASE(0, GM_0B0(OP), GM_0B1(OP), GM_1B0(OP), GM_1B1(OP)) \
+    GM_CASE(1, GM_0A0(OP), GM_0B1(OP), GM_1B0(OP), GM_1B1(OP)) \
+    GM_CASE(2, GM_0B0(OP), GM_0A1(OP), GM_1B0(OP), GM_1B1(OP)) \
+    GM_CASE(3, GM_0A0(OP), GM_0A1(OP), GM_1B0(OP), GM_1B1(OP)) \
+    GM_CASE(4, GM_0B0(OP), GM_0B1(OP), GM_1A0(OP), GM_1B1(OP)) \
+    GM_CASE(5, GM_0A0(OP), GM_0B1(OP), GM_1A0(OP), GM_1B1(OP)) \
+    GM_CASE(6, GM_0B0(OP), GM_0A1(OP), GM_1A0(OP), GM_1B1(OP)) \
+    GM_CASE(7, GM_0A0(OP), GM_0A1(OP), GM_1A0(OP), GM_1B1(OP)) \
+    GM_CASE(8, GM_0B0(OP), GM_0B1(OP), GM_1B0(OP), GM_1A1(OP)) \
+    GM_CASE(9, GM_0A0(OP), GM_0B1(OP), GM_1B0(OP), GM_1A1(OP)) \
+    GM_CASE(10, GM_0B0(OP), GM_0A1(OP), GM_1B0(OP), GM_1A1(OP)) \
+    GM_CASE(11, GM_0A0(OP), GM_0A1(OP), GM_1B0(OP), GM_1A1(OP)) \
+    GM_CASE(12, GM_0B0(OP), GM_0B1(OP), GM_1A0(OP), GM_1A1(OP)) \
+    GM_CASE(13, GM_0A0(OP), GM_0B1(OP), GM_1A0(OP), GM_1A1(OP)) \
+    GM_CASE(14, GM_0B0(OP), GM_0A1(OP), GM_1A0(OP), GM_1A1(OP)) \
+    GM_CASE(15, GM_0A0(OP), GM_0A1(OP), GM_1A0(OP), GM_1A1(OP)) \
+    "NEXT: setp.ne.u32 more, %" #N ", 0;\n @more bra.uni LOOP;\n}\n"
+// the last sample of an odd number
+#define GM_ONE(OP, PP, XP, N)                                                                                 \
+    "{\n .reg .b64 d, e, x0, x1, x2, x3;\n .reg .u32 bits;\n"                                      \
+    " TS: .branchtargets C0, C1, C2, C3;\n"                                                                      \
+    " ld.shared.u8 bits, [%" #PP "];\n and.b32 bits, bits, 3;\n" GM_LOAD(XP, 0, 0, 1) " brx.idx.uni bits, TS;\n"           \
+    GM_CASE(0, GM_0B0(OP), GM_0B1(OP), "", "") \
+    GM_CASE(1, GM_0A0(OP), GM_0B1(OP), "", "") \
+    GM_CASE(2, GM_0B0(OP), GM_0A1(OP), "", "") \
+    GM_CASE(3, GM_0A0(OP), GM_0A1(OP), "", "") \
+    "NEXT:\n}\n"
+// x added to the sum
+#define GM_SUM(M_, W_, U_, X_) "add.rn.f32x2 %" #M_ ", %" #M_ ", x" #X_ ";\n"
+// ... and x^2 to the sum of squares; one: 19
+#define GM_ONEPASS(M_, W_, U_, X_)                                                        \
+    GM_SUM(M_, W_, U_, X_) "mul.rn.f32x2 d, x" #X_ ", x" #X_ ";\n fma.rn.f32x2 %" #W_ ", %19, d, %" #W_ ";\n"
+// Kahan step: W_ the compensation
+#define GM_KAHAN(M_, W_, U_, X_)                                                                     \
+    "sub.rn.f32x2 d, x" #X_ ", %" #W_ ";\n add.rn.f32x2 e, %" #M_ ", d;\n"                          \
+    "sub.rn.f32x2 %" #W_ ", e, %" #M_ ";\n sub.rn.f32x2 %" #W_ ", %" #W_ ", d;\n mov.b64 %" #M_ ", e;\n"
+// squared deviation from the mean M_ added to W_; one: 19
+#define GM_DEV(M_, W_, U_, X_) \
+    "sub.rn.f32x2 d, x" #X_ ", %" #M_ ";\n mul.rn.f32x2 d, d, d;\n fma.rn.f32x2 %" #W_ ", %19, d, %" #W_ ";\n"
+// ... and the deviation itself to W_, the square to U_; one: 27
+#define GM_DEV2(M_, W_, U_, X_)                                                                \
+    "sub.rn.f32x2 d, x" #X_ ", %" #M_ ";\n add.rn.f32x2 %" #W_ ", %" #W_ ", d;\n"             \
+    "mul.rn.f32x2 d, d, d;\n fma.rn.f32x2 %" #U_ ", %27, d, %" #U_ ";\n"
+// a statistic's registers, class by class, permutation by permutation
+#define GM_RW(A) "+l"(A[0][0][0]), "+l"(A[0][0][1]), "+l"(A[0][1][0]), "+l"(A[0][1][1]), "+l"(A[1][0][0]),      \
+    "+l"(A[1][0][1]), "+l"(A[1][1][0]), "+l"(A[1][1][1])
+
+enum WalkMode { WALK_SUMS, WALK_STRICT, WALK_DEVIATIONS };
+
+// Running statistics of a lane's genes for the warp's permutations: class c
+// (0: A, 1: B), permutation j, vector v.
+template <int ACC, class T>
+struct Stats {
     using E = Exact<T>;
-    const T* xg = X + g;
+    using A = Vec<T>;
+    using V = typename A::V;
+    static constexpr int NV = metric_vecs<ACC, T>(), L = A::kLanes, kQ = metric_q<T>();
+    static constexpr bool TWO = ACC == ACC_TWOPASS || ACC == ACC_OVERKILL;
+    static constexpr bool VAR = ACC == ACC_ONEPASS || ACC == ACC_KNUTH || TWO;  // variances
+    static constexpr bool COMP = ACC == ACC_KAHAN || ACC == ACC_OVERKILL;       // compensated sums
+    V m[2][kQ][NV];
+    V q[2][COMP ? kQ : 1][COMP ? NV : 1];
+    V var[2][VAR ? kQ : 1][VAR ? NV : 1];
+    int it[2][ACC == ACC_KNUTH ? kQ : 1];
+    V one;
 
-    T mA[PB], mB[PB], vA[PB], vB[PB], cA[PB], cB[PB];
-    int iA[PB], iB[PB];
+    __device__ __forceinline__ void clear() {
+        one = A::runtime_one();
 #pragma unroll
-    for (int j = 0; j < PB; j++) {
-        mA[j] = mB[j] = vA[j] = vB[j] = cA[j] = cB[j] = T(0);
-        iA[j] = iB[j] = 0;
-    }
-
-    // ---------------- pass 1 ----------------
-    for (int s0 = 0, w = 0; s0 < S; s0 += 32, w++) {
-        uint32_t mw[PB];
+        for (int c = 0; c < 2; c++)
 #pragma unroll
-        for (int j = 0; j < PB; j++) mw[j] = sm_masks[j * words + w];
-        const int n = min(32, S - s0);
-        for (int t = 0; t < n; t++) {
-            const T x = __ldg(xg + (int64_t)(s0 + t) * G);
-            T xx = T(0);
-            if (ACC == ACC_ONEPASS) xx = E::mul(x, x);
+            for (int j = 0; j < kQ; j++) {
+                if constexpr (ACC == ACC_KNUTH) it[c][j] = 0;
 #pragma unroll
-            for (int j = 0; j < PB; j++) {
-                const bool l = (mw[j] >> t) & 1u;  // class A <=> permuted label 0
-                if (ACC == ACC_NAIVE) {
-                    mA[j] = E::add(mA[j], E::mul(l ? T(1) : T(0), x));
-                    mB[j] = E::add(mB[j], E::mul(l ? T(0) : T(1), x));
-                } else if (ACC == ACC_KAHAN || ACC == ACC_OVERKILL) {
-                    const T acc = l ? mA[j] : mB[j];
-                    const T alpha = E::sub(x, l ? cA[j] : cB[j]);
-                    const T beta = E::add(acc, alpha);
-                    const T kk = E::sub(E::sub(beta, acc), alpha);
-                    if (l) { cA[j] = kk; mA[j] = beta; } else { cB[j] = kk; mB[j] = beta; }
-                } else if (ACC == ACC_ONEPASS) {
-                    // one add into the selected accumulator (the same rounding
-                    // as the reference's conditional add, one FP64 / FP32 op)
-                    const T m = E::add(l ? mA[j] : mB[j], x);
-                    const T v = E::add(l ? vA[j] : vB[j], xx);
-                    mA[j] = l ? m : mA[j];
-                    mB[j] = l ? mB[j] : m;
-                    vA[j] = l ? v : vA[j];
-                    vB[j] = l ? vB[j] : v;
-                } else if (ACC == ACC_TWOPASS) {
-                    const T m = E::add(l ? mA[j] : mB[j], x);
-                    mA[j] = l ? m : mA[j];
-                    mB[j] = l ? mB[j] : m;
-                } else {  // ACC_KNUTH: the update of the selected class
-                    const int it = (l ? iA[j] : iB[j]) + 1;
-                    const T mo = l ? mA[j] : mB[j];
-                    const T d = E::sub(x, mo);
-                    const T mn = E::add(mo, E::div(d, (T)it));
-                    const T vn = E::add(l ? vA[j] : vB[j], E::mul(d, E::sub(x, mn)));
-                    iA[j] = l ? it : iA[j];
-                    iB[j] = l ? iB[j] : it;
-                    mA[j] = l ? mn : mA[j];
-                    mB[j] = l ? mB[j] : mn;
-                    vA[j] = l ? vn : vA[j];
-                    vB[j] = l ? vB[j] : vn;
+                for (int v = 0; v < NV; v++) {
+                    m[c][j][v] = A::zero();
+                    if constexpr (COMP) q[c][j][v] = A::zero();
+                    if constexpr (VAR) var[c][j][v] = A::zero();
                 }
             }
-        }
     }
-
-    if (ACC != ACC_KNUTH) {
+    // one sample with class-A bits B
+    template <int MODE, int B>
+    __device__ __forceinline__ void step(const V* x) {
 #pragma unroll
-        for (int j = 0; j < PB; j++) { mA[j] = E::div(mA[j], nA); mB[j] = E::div(mB[j], nB); }
-    }
-    if (ACC == ACC_ONEPASS) {
+        for (int j = 0; j < kQ; j++) {
+            constexpr int kBits = B;
+            const int c = ((kBits >> j) & 1) ? 0 : 1;
+            if constexpr (MODE == WALK_DEVIATIONS) {
 #pragma unroll
-        for (int j = 0; j < PB; j++) {
-            vA[j] = E::sub(E::div(vA[j], nA), E::mul(mA[j], mA[j]));
-            vB[j] = E::sub(E::div(vB[j], nB), E::mul(mB[j], mB[j]));
-        }
-    }
-
-    // ---------------- pass 2 (twopass, overkill) ----------------
-    if (ACC == ACC_TWOPASS || ACC == ACC_OVERKILL) {
-        // cA/cB hold the sums of deviations (overkill's aux) from here on
+                for (int v = 0; v < NV; v++) {
+                    const V d = A::sub(x[v], m[c][j][v]);
+                    if constexpr (ACC == ACC_OVERKILL) q[c][j][v] = A::add(q[c][j][v], d);
+                    if constexpr (TWO) var[c][j][v] = A::add_product(var[c][j][v], A::mul(d, d), one);
+                }
+            } else {
+                if constexpr (ACC == ACC_KNUTH) it[c][j]++;
 #pragma unroll
-        for (int j = 0; j < PB; j++) cA[j] = cB[j] = T(0);
-        for (int s0 = 0, w = 0; s0 < S; s0 += 32, w++) {
-            uint32_t mw[PB];
+                for (int v = 0; v < NV; v++) {
+                    if constexpr (COMP) {
+                        const V alpha = A::sub(x[v], q[c][j][v]);
+                        const V beta = A::add(m[c][j][v], alpha);
+                        q[c][j][v] = A::sub(A::sub(beta, m[c][j][v]), alpha);
+                        m[c][j][v] = beta;
+                    } else if constexpr (ACC == ACC_KNUTH) {
+                        T xs[L], ms[L], vs[L];
+                        A::unpack(x[v], xs);
+                        A::unpack(m[c][j][v], ms);
+                        A::unpack(var[c][j][v], vs);
 #pragma unroll
-            for (int j = 0; j < PB; j++) mw[j] = sm_masks[j * words + w];
-            const int n = min(32, S - s0);
-            for (int t = 0; t < n; t++) {
-                const T x = __ldg(xg + (int64_t)(s0 + t) * G);
-#pragma unroll
-                for (int j = 0; j < PB; j++) {
-                    const bool l = (mw[j] >> t) & 1u;
-                    const T d = E::sub(x, l ? mA[j] : mB[j]);
-                    const T dd = E::mul(d, d);
-                    if (ACC == ACC_OVERKILL) {
-                        const T c = E::add(l ? cA[j] : cB[j], d);
-                        cA[j] = l ? c : cA[j];
-                        cB[j] = l ? cB[j] : c;
+                        for (int l = 0; l < L; l++) {
+                            const T d = E::sub(xs[l], ms[l]);
+                            ms[l] = E::add(ms[l], E::div(d, (T)it[c][j]));
+                            vs[l] = E::add(vs[l], E::mul(d, E::sub(xs[l], ms[l])));
+                        }
+                        m[c][j][v] = A::pack(ms);
+                        var[c][j][v] = A::pack(vs);
+                    } else {
+                        m[c][j][v] = A::add(m[c][j][v], x[v]);
+                        if constexpr (ACC == ACC_ONEPASS)
+                            var[c][j][v] = A::add_product(var[c][j][v], A::mul(x[v], x[v]), one);
                     }
-                    const T v = E::add(l ? vA[j] : vB[j], dd);
-                    vA[j] = l ? v : vA[j];
-                    vB[j] = l ? vB[j] : v;
+                    if constexpr (MODE == WALK_STRICT) {
+                        T none[L];
+#pragma unroll
+                        for (int l = 0; l < L; l++) none[l] = T(0);
+                        m[1 - c][j][v] = A::add(m[1 - c][j][v], A::mul(x[v], A::pack(none)));
+                    }
                 }
             }
         }
-#pragma unroll
-        for (int j = 0; j < PB; j++) {
-            if (ACC == ACC_OVERKILL) {
-                vA[j] = E::sub(vA[j], E::div(E::mul(cA[j], cA[j]), nA));
-                vB[j] = E::sub(vB[j], E::div(E::mul(cB[j], cB[j]), nB));
+    }
+    // whether two samples are taken by one assembly block
+    template <int MODE>
+    static constexpr bool paired() { return sizeof(T) == 4 && ACC != ACC_KNUTH && MODE != WALK_STRICT; }
+    // `pairs` pairs of samples (COUNT = 2) or one sample (COUNT = 1) from the
+    // shared-memory addresses of their class bits and of the lane's vectors.
+    // The bits are the same in every lane: one branch, no divergence.
+    template <int MODE, int COUNT>
+    __device__ __forceinline__ void samples(uint32_t pp, uint32_t xp, uint32_t pairs) {
+#define GM_RUN(OP, PP, XP, N, ...)                                                                                \
+    if constexpr (COUNT == 2)                                                                                     \
+        asm volatile(GM_LOOP(OP, PP, XP, N) : __VA_ARGS__, "+r"(pp), "+r"(xp), "+r"(pairs) : "l"(one) : "memory"); \
+    else                                                                                                          \
+        asm volatile(GM_ONE(OP, PP, XP, N) : __VA_ARGS__, "+r"(pp), "+r"(xp), "+r"(pairs) : "l"(one) : "memory");
+        if constexpr (MODE == WALK_SUMS && (ACC == ACC_NAIVE || ACC == ACC_TWOPASS)) {
+            GM_RUN(GM_SUM, 8, 9, 10, GM_RW(m))
+        } else if constexpr (ACC == ACC_ONEPASS) {
+            GM_RUN(GM_ONEPASS, 16, 17, 18, GM_RW(m), GM_RW(var))
+        } else if constexpr (ACC == ACC_KAHAN || (ACC == ACC_OVERKILL && MODE == WALK_SUMS)) {
+            GM_RUN(GM_KAHAN, 16, 17, 18, GM_RW(m), GM_RW(q))
+        } else if constexpr (ACC == ACC_TWOPASS) {
+            GM_RUN(GM_DEV, 16, 17, 18, GM_RW(m), GM_RW(var))
+        } else if constexpr (ACC == ACC_OVERKILL) {
+            GM_RUN(GM_DEV2, 24, 25, 26, GM_RW(m), GM_RW(q), GM_RW(var))
+        }
+#undef GM_RUN
+    }
+    // one sample by a switch (FP64: bound by its pipe; Knuth's divisions)
+    template <int MODE>
+    __device__ __forceinline__ void sample(int bits, const V* x) {
+        if constexpr (kQ == 4) {
+            switch (bits) {
+                case 0: step<MODE, 0>(x); break;
+                case 1: step<MODE, 1>(x); break;
+                case 2: step<MODE, 2>(x); break;
+                case 3: step<MODE, 3>(x); break;
+                case 4: step<MODE, 4>(x); break;
+                case 5: step<MODE, 5>(x); break;
+                case 6: step<MODE, 6>(x); break;
+                case 7: step<MODE, 7>(x); break;
+                case 8: step<MODE, 8>(x); break;
+                case 9: step<MODE, 9>(x); break;
+                case 10: step<MODE, 10>(x); break;
+                case 11: step<MODE, 11>(x); break;
+                case 12: step<MODE, 12>(x); break;
+                case 13: step<MODE, 13>(x); break;
+                case 14: step<MODE, 14>(x); break;
+                default: step<MODE, 15>(x); break;
             }
-            vA[j] = E::div(vA[j], nA);
-            vB[j] = E::div(vB[j], nB);
+        } else {
+            switch (bits) {
+                case 0: step<MODE, 0>(x); break;
+                case 1: step<MODE, 1>(x); break;
+                case 2: step<MODE, 2>(x); break;
+                default: step<MODE, 3>(x); break;
+            }
         }
     }
-    if (ACC == ACC_KNUTH) {
-#pragma unroll
-        for (int j = 0; j < PB; j++) { vA[j] = E::div(vA[j], nA); vB[j] = E::div(vB[j], nB); }
-    }
+};
 
+// The expression tile of a block and its walks over the samples.
+template <int ACC, class T>
+struct Tile {
+    using S_ = Stats<ACC, T>;
+    using V = typename S_::V;
+    static constexpr int NV = S_::NV, L = S_::L, GW = metric_genes<ACC, T>();
+    const T* X;   // first gene of the tile
+    T* tile;      // [2][kChunk][GW]
+    const uint8_t* pat;
+    int G, S, gn;
+    bool wide;      // 16-byte copies: every row starts on a 16-byte boundary
+    bool resident;  // the whole table of the tile is in the two buffers (resident())
+
+    __device__ __forceinline__ void load(int c) const {
+        constexpr int PER = 16 / (int)sizeof(T);
+        const int s0 = c * kChunk, n = min(kChunk, S - s0);
+        T* const to = tile + (c & 1) * kChunk * GW;
+        const T* const from = X + (int64_t)s0 * G;
+        if (wide) {
+            for (int i = threadIdx.x; i < n * (GW / PER); i += blockDim.x) {
+                const int r = i / (GW / PER), q = (i % (GW / PER)) * PER;
+                async_copy<16>(smem_u32(to + r * GW + q), from + (int64_t)r * G + q);
+            }
+        } else {
+            for (int i = threadIdx.x; i < n * GW; i += blockDim.x) {
+                const int r = i / GW, q = i % GW;
+                if (q < gn) async_copy<(int)sizeof(T)>(smem_u32(to + r * GW + q), from + (int64_t)r * G + q);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    // at most two chunks: copied once, for every pass and round of the block
+    __device__ __forceinline__ void load_all() const {
+        load(0);
+        if (S > kChunk) load(1);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+    }
+    // every sample in index order; the whole block takes part in the copies
+    template <int MODE>
+    __device__ __forceinline__ void walk(S_& st, bool mine) const {
+        const int chunks = (S + kChunk - 1) / kChunk, lane = threadIdx.x & 31;
+        if (!resident) {
+            __syncthreads();  // the buffers are free
+            load(0);
+        }
+        for (int c = 0; c < chunks; c++) {
+            if (!resident) {
+                if (c + 1 < chunks) {
+                    load(c + 1);
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                } else {
+                    asm volatile("cp.async.wait_group 0;" ::: "memory");
+                }
+                __syncthreads();
+            }
+            if (mine) {
+                const int s0 = c * kChunk, n = min(kChunk, S - s0);
+                const V* const row = reinterpret_cast<const V*>(tile + (c & 1) * kChunk * GW) + lane * NV;
+                auto get = [&](int t, V* x) {
+                    if constexpr (NV == 2) {
+                        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(row + t * (GW / L));
+                        x[0] = q.x;
+                        x[1] = q.y;
+                    } else {
+                        x[0] = row[t * (GW / L)];
+                    }
+                };
+                if constexpr (S_::template paired<MODE>()) {
+                    const uint32_t pp = smem_u32(pat + s0), xp = smem_u32(row);
+                    static_assert(GW * sizeof(T) == 512, "the loop's row stride");
+                    if (n > 1) st.template samples<MODE, 2>(pp, xp, n >> 1);
+                    if (n & 1) st.template samples<MODE, 1>(pp + n - 1, xp + (n - 1) * GW * (int)sizeof(T), 0u);
+                } else {
+#pragma unroll 1
+                    for (int t = 0; t < n; t++) {
+                        V x[NV];
+                        get(t, x);
+                        st.template sample<MODE>(sizeof(T) == 4 ? pat[s0 + t] & 3 : pat[s0 + t], x);
+                    }
+                }
+            }
+            if (!resident) __syncthreads();
+        }
+    }
+};
+
+// One block: gene tile `gt`, permutations p0 .. p0 + kQ * warps * rounds - 1
+// (a warp takes `rounds` groups one after the other; with at most two chunks
+// of samples the tile is copied once for all of them).  `strict`
+// (naive accumulator, a table with values that are not finite): the
+// reference adds 0 * x to the other class, which is NaN there.
+template <int ACC, class T>
+__device__ __forceinline__ void metric_block(const T* __restrict__ X, int G, int S,
+                                             const uint32_t* __restrict__ masks, int words, int num_perms, T nA, T nB,
+                                             T* __restrict__ keys, int comb, bool strict, int gt, int p0, int rounds) {
+    using E = Exact<T>;
+    using St = Stats<ACC, T>;
+    using A = Vec<T>;
+    constexpr int NV = St::NV, L = St::L, GL = NV * L, GW = 32 * GL;  // vectors, genes of a lane
+    constexpr int kQ = St::kQ;
+    constexpr bool TWO = St::TWO, VAR = St::VAR;
+    extern __shared__ __align__(16) unsigned char smem[];
+    T* const tile = reinterpret_cast<T*>(smem);                 // [2][kChunk][GW]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    T* const out = tile + 2 * kChunk * GW + warp * GW;          // [warps][GW]
+    uint8_t* const pat = reinterpret_cast<uint8_t*>(tile + (2 * kChunk + warps) * GW) + warp * S;  // [warps][S]
+    const int g0 = gt * GW;
+    const int gn = min(GW, G - g0);  // genes of the tile
+    const bool wide = gn == GW && (G % (16 / (int)sizeof(T))) == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
+    const Tile<ACC, T> tl{X + g0, tile, pat, G, S, gn, wide, S <= 2 * kChunk};
+    if (tl.resident) tl.load_all();
+
+    for (int round = 0; round < rounds; round++) {
+        const int p = p0 + (round * warps + warp) * kQ;  // the warp's permutations
+        const bool mine = p < num_perms;
+        __syncwarp();
+        if (mine) {  // class-A bits of the permutations, a byte per sample; above them the next sample's
+            for (int w = 0; w < words; w++) {
+                uint32_t mw[kQ], b = 0u;
 #pragma unroll
-    for (int j = 0; j < PB; j++) {
-        if (p0 + j < num_perms)
-            keys[(int64_t)(p0 + j) * G + g] = canonical_nan(combine<T, COMB>(mA[j], vA[j], nA, mB[j], vB[j], nB));
+                for (int j = 0; j < kQ; j++) {
+                    mw[j] = p + j < num_perms ? __ldg(masks + (int64_t)(p + j) * words + w) : 0u;
+                    b |= ((mw[j] >> lane) & 1u) << j;
+                }
+                if (sizeof(T) == 4) b |= __shfl_down_sync(kFullMask, b, 1) << kQ;  // pairs start at even samples
+                if (w * 32 + lane < S) pat[w * 32 + lane] = (uint8_t)b;
+            }
+        }
+        __syncwarp();
+        St st;
+        st.clear();
+        // pass 1: sums (or running means and squares)
+        if constexpr (ACC == ACC_NAIVE) {
+            if (strict) tl.template walk<WALK_STRICT>(st, mine);
+            else tl.template walk<WALK_SUMS>(st, mine);
+        } else {
+            tl.template walk<WALK_SUMS>(st, mine);
+        }
+        const ClassSize<T> n[2] = {ClassSize<T>(nA), ClassSize<T>(nB)};
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+#pragma unroll
+            for (int j = 0; j < kQ; j++)
+#pragma unroll
+                for (int v = 0; v < NV; v++) {
+                    T ms[L], vs[L];
+                    A::unpack(st.m[c][j][v], ms);
+                    if constexpr (VAR) A::unpack(st.var[c][j][v], vs);
+#pragma unroll
+                    for (int l = 0; l < L; l++) {
+                        if constexpr (ACC != ACC_KNUTH) ms[l] = n[c].divides(ms[l]);
+                        if constexpr (ACC == ACC_ONEPASS) vs[l] = E::sub(n[c].divides(vs[l]), E::mul(ms[l], ms[l]));
+                        if constexpr (ACC == ACC_KNUTH) vs[l] = n[c].divides(vs[l]);
+                    }
+                    st.m[c][j][v] = A::pack(ms);
+                    if constexpr (VAR && !TWO) st.var[c][j][v] = A::pack(vs);
+                    if constexpr (ACC == ACC_OVERKILL) st.q[c][j][v] = A::zero();  // sums of deviations from here on
+                }
+        // pass 2: squared deviations from the own class mean
+        if constexpr (TWO) tl.template walk<WALK_DEVIATIONS>(st, mine);
+        if (!mine) continue;
+        // the metric, its keys stored a permutation at a time
+#pragma unroll
+        for (int j = 0; j < kQ; j++) {
+            if (p + j >= num_perms) break;
+            T key[GL];
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                T ms[2][L], vs[2][L], qs[L];
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    A::unpack(st.m[c][j][v], ms[c]);
+                    if constexpr (VAR) A::unpack(st.var[c][j][v], vs[c]);
+                    if constexpr (ACC == ACC_OVERKILL) {
+                        A::unpack(st.q[c][j][v], qs);
+#pragma unroll
+                        for (int l = 0; l < L; l++) vs[c][l] = E::sub(vs[c][l], n[c].divides(E::mul(qs[l], qs[l])));
+                    }
+#pragma unroll
+                    for (int l = 0; l < L; l++) {
+                        if constexpr (TWO) vs[c][l] = n[c].divides(vs[c][l]);
+                        if constexpr (!VAR) vs[c][l] = T(0);
+                    }
+                }
+#pragma unroll
+                for (int l = 0; l < L; l++)
+                    key[v * L + l] = canonical_nan(combine<T>(comb, ms[0][l], vs[0][l], n[0], ms[1][l], vs[1][l], n[1]));
+            }
+#pragma unroll
+            for (int i = 0; i < GL; i++) out[lane * GL + i] = key[i];
+            __syncwarp();
+            T* const kp = keys + (int64_t)(p + j) * G + g0;
+#pragma unroll
+            for (int i = 0; i < GL; i++)
+                if (lane + 32 * i < gn) kp[lane + 32 * i] = out[lane + 32 * i];
+            __syncwarp();
+        }
     }
 }
 
-// one CTA of the exact form: genes bx*128.., permutations by*PB..
-template <int ACC, int COMB, class T, int PB>
-__device__ __forceinline__ void metric_exact_block(const T* __restrict__ X, int G, int S,
-                                                   const uint32_t* __restrict__ masks, int words, int num_perms,
-                                                   T nA, T nB, T* __restrict__ keys, int bx, int by) {
-    extern __shared__ uint32_t sm_masks[];  // [PB][words]
-    const int p0 = by * PB;
-    for (int i = threadIdx.x; i < PB * words; i += blockDim.x) {
-        const int j = i / words, w = i - j * words;
-        sm_masks[i] = (p0 + j < num_perms) ? masks[(int64_t)(p0 + j) * words + w] : 0u;
-    }
-    __syncthreads();
-    const int g = bx * blockDim.x + threadIdx.x;
-    if (g >= G) return;
-    metric_exact<ACC, COMB, T, PB>(X, G, S, sm_masks, words, num_perms, p0, nA, nB, keys, g);
-}
-
-template <int ACC, int COMB, class T, int PB>
-__global__ void __launch_bounds__(128)
-metric_kernel(const T* __restrict__ X, int G, int S, const uint32_t* __restrict__ masks, int words,
-              int num_perms, T nA, T nB, T* __restrict__ keys) {
-    metric_exact_block<ACC, COMB, T, PB>(X, G, S, masks, words, num_perms, nA, nB, keys, blockIdx.x, blockIdx.y);
+template <int ACC, class T>
+__global__ void __launch_bounds__(32 * kMaxWarps, metric_blocks<ACC, T>())
+metric_kernel(const T* __restrict__ X, int G, int S, const uint32_t* __restrict__ masks, int words, int num_perms,
+              T nA, T nB, T* __restrict__ keys, int comb, const int* __restrict__ finite, int rounds) {
+    const bool strict = ACC == ACC_NAIVE && finite && *finite == 0;
+    metric_block<ACC, T>(X, G, S, masks, words, num_perms, nA, nB, keys, comb, strict, blockIdx.x,
+                         blockIdx.y * (blockDim.x >> 5) * metric_q<T>() * rounds, rounds);
 }
 
 // every instance of a batch group in one launch (blockIdx.z = instance; the
-// grid covers the largest instance, CTAs beyond an instance's extent leave)
-template <int ACC, int COMB, class T, int PB>
-__global__ void __launch_bounds__(128) metric_multi(const MetricTask<T>* __restrict__ tasks) {
+// grid covers the largest instance, blocks beyond an instance's extent leave)
+template <int ACC, class T>
+__global__ void __launch_bounds__(32 * kMaxWarps, metric_blocks<ACC, T>())
+metric_multi(const MetricTask<T>* __restrict__ tasks, int comb, int rounds) {
     const MetricTask<T> t = tasks[blockIdx.z];
-    if ((int)blockIdx.x * 128 >= t.G || (int)blockIdx.y * PB >= t.num_perms) return;
-    metric_exact_block<ACC, COMB, T, PB>(t.X, t.G, t.S, t.masks, t.words, t.num_perms, t.nA, t.nB, t.keys,
-                                         blockIdx.x, blockIdx.y);
+    const int p0 = blockIdx.y * (blockDim.x >> 5) * metric_q<T>() * rounds;
+    if ((int)blockIdx.x * metric_genes<ACC, T>() >= t.G || p0 >= t.num_perms) return;
+    const bool strict = ACC == ACC_NAIVE && t.fast_ok && *t.fast_ok == 0;
+    metric_block<ACC, T>(t.X, t.G, t.S, t.masks, t.words, t.num_perms, t.nA, t.nB, t.keys, comb, strict, blockIdx.x,
+                         p0, rounds);
 }
 
-// ---------------------------------------------------------------------------
-// Packed fast form (fp32, naive / onepass / twopass accumulators).
-//
-// With a class weight l in {0, 1}, fma(l, v, acc) rounds exactly like the
-// reference's conditional `acc + v` when v is finite (l = 1: one rounding of
-// acc + v; l = 0: acc unchanged), and the naive accumulator's literal
-// `acc + l*v` for any v.  Blackwell's paired-FP32 instructions (fma / add /
-// mul .rn.f32x2) then update two permutations per instruction with no
-// predication: pass 1 is one packed FMA per class and permutation pair, pass 2
-// selects the class mean as lA*mA + lB*mB (exact: one product is zero) and
-// adds the squared deviation with the class weights.  The expression table is
-// checked once per upload (gsea::launch_finite_check): any value that is not
-// finite or has |x| >= 2^60 (whose square could overflow) sends the kernel to
-// the exact predicated form instead.
-__device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2_unpack(unsigned long long v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
+inline int metric_sms() {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 1;
 }
 
-// one CTA of the packed form: genes bx*128.., permutations by*PB..
-template <int ACC, int COMB, int PB>
-__device__ __forceinline__ void metric_fast_block(const float* __restrict__ X, int G, int S,
-                                                  const uint32_t* __restrict__ masks, int words, int num_perms,
-                                                  float nA, float nB, float* __restrict__ keys,
-                                                  const int* __restrict__ fast_ok, int bx, int by) {
-    static_assert(PB % 2 == 0, "permutations are processed in pairs");
-    constexpr int PAIRS = PB / 2;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ulonglong2* lab = reinterpret_cast<ulonglong2*>(smem_raw);                       // [S][PAIRS]
-    uint32_t* sm_masks = reinterpret_cast<uint32_t*>(lab + (size_t)S * PAIRS);        // [PB][words]
-    const int p0 = by * PB;
-    for (int i = threadIdx.x; i < PB * words; i += blockDim.x) {
-        const int j = i / words, w = i - j * words;
-        sm_masks[i] = (p0 + j < num_perms) ? masks[(int64_t)(p0 + j) * words + w] : 0u;
-    }
-    __syncthreads();
-    const bool fast = ACC == ACC_NAIVE || *fast_ok != 0;
-    if (fast) {
-        for (int i = threadIdx.x; i < S * PAIRS; i += blockDim.x) {
-            const int sidx = i / PAIRS, q = i - sidx * PAIRS;
-            const int w = sidx >> 5, t = sidx & 31;
-            const float a0 = (float)((sm_masks[(2 * q) * words + w] >> t) & 1u);
-            const float a1 = (float)((sm_masks[(2 * q + 1) * words + w] >> t) & 1u);
-            lab[i] = make_ulonglong2(f2_pack(a0, a1), f2_pack(1.f - a0, 1.f - a1));
-        }
-    }
-    __syncthreads();
-    const int g = bx * blockDim.x + threadIdx.x;
-    if (g >= G) return;
-    if (!fast) {
-        metric_exact<ACC, COMB, float, PB>(X, G, S, sm_masks, words, num_perms, p0, nA, nB, keys, g);
-        return;
-    }
-    const float* xg = X + g;
-    unsigned long long mA[PAIRS], mB[PAIRS], vA[PAIRS], vB[PAIRS];
-#pragma unroll
-    for (int q = 0; q < PAIRS; q++) mA[q] = mB[q] = vA[q] = vB[q] = 0ull;
-    // samples per unrolled step: eight loads of the table in flight (two
-    // for onepass, whose extra accumulators leave no registers for more)
-    constexpr int kUnroll = ACC == ACC_ONEPASS ? 2 : 8;
-    // pass 1: class sums (and sums of squares for onepass)
-#pragma unroll kUnroll
-    for (int sidx = 0; sidx < S; sidx++) {
-        const float x = __ldg(xg + (int64_t)sidx * G);
-        const unsigned long long xx = f2_pack(x, x);
-        unsigned long long sq = 0ull;
-        if (ACC == ACC_ONEPASS) {
-            const float x2 = __fmul_rn(x, x);
-            sq = f2_pack(x2, x2);
-        }
-        const ulonglong2* ls = lab + (size_t)sidx * PAIRS;
-#pragma unroll
-        for (int q = 0; q < PAIRS; q++) {
-            const ulonglong2 l = ls[q];
-            mA[q] = f2_fma(l.x, xx, mA[q]);
-            mB[q] = f2_fma(l.y, xx, mB[q]);
-            if (ACC == ACC_ONEPASS) {
-                vA[q] = f2_fma(l.x, sq, vA[q]);
-                vB[q] = f2_fma(l.y, sq, vB[q]);
-            }
-        }
-    }
-    float fmA[PB], fmB[PB];
-#pragma unroll
-    for (int q = 0; q < PAIRS; q++) {
-        f2_unpack(mA[q], fmA[2 * q], fmA[2 * q + 1]);
-        f2_unpack(mB[q], fmB[2 * q], fmB[2 * q + 1]);
-    }
-#pragma unroll
-    for (int j = 0; j < PB; j++) {
-        fmA[j] = __fdiv_rn(fmA[j], nA);
-        fmB[j] = __fdiv_rn(fmB[j], nB);
-    }
-    float fvA[PB], fvB[PB];
-#pragma unroll
-    for (int j = 0; j < PB; j++) fvA[j] = fvB[j] = 0.f;
-    if (ACC == ACC_ONEPASS) {
-#pragma unroll
-        for (int q = 0; q < PAIRS; q++) {
-            f2_unpack(vA[q], fvA[2 * q], fvA[2 * q + 1]);
-            f2_unpack(vB[q], fvB[2 * q], fvB[2 * q + 1]);
-        }
-#pragma unroll
-        for (int j = 0; j < PB; j++) {
-            fvA[j] = __fsub_rn(__fdiv_rn(fvA[j], nA), __fmul_rn(fmA[j], fmA[j]));
-            fvB[j] = __fsub_rn(__fdiv_rn(fvB[j], nB), __fmul_rn(fmB[j], fmB[j]));
-        }
-    }
-    if (ACC == ACC_TWOPASS) {
-        // pass 2: squared deviations from the own class mean
-#pragma unroll
-        for (int q = 0; q < PAIRS; q++) {
-            mA[q] = f2_pack(fmA[2 * q], fmA[2 * q + 1]);
-            mB[q] = f2_pack(fmB[2 * q], fmB[2 * q + 1]);
-        }
-#pragma unroll kUnroll
-        for (int sidx = 0; sidx < S; sidx++) {
-            const float x = __ldg(xg + (int64_t)sidx * G);
-            const unsigned long long xx = f2_pack(x, x);
-            const ulonglong2* ls = lab + (size_t)sidx * PAIRS;
-#pragma unroll
-            for (int q = 0; q < PAIRS; q++) {
-                const ulonglong2 l = ls[q];
-                const unsigned long long m = f2_fma(l.x, mA[q], f2_mul(l.y, mB[q]));  // own class mean
-                const unsigned long long dv = f2_sub(xx, m);
-                const unsigned long long dd = f2_mul(dv, dv);
-                vA[q] = f2_fma(l.x, dd, vA[q]);
-                vB[q] = f2_fma(l.y, dd, vB[q]);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < PAIRS; q++) {
-            f2_unpack(vA[q], fvA[2 * q], fvA[2 * q + 1]);
-            f2_unpack(vB[q], fvB[2 * q], fvB[2 * q + 1]);
-        }
-#pragma unroll
-        for (int j = 0; j < PB; j++) {
-            fvA[j] = __fdiv_rn(fvA[j], nA);
-            fvB[j] = __fdiv_rn(fvB[j], nB);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < PB; j++) {
-        if (p0 + j < num_perms)
-            keys[(int64_t)(p0 + j) * G + g] =
-                canonical_nan(combine<float, COMB>(fmA[j], fvA[j], nA, fmB[j], fvB[j], nB));
-    }
+// Warps of a block: eight share a tile; fewer where that leaves SMs without
+// two blocks (few permutations of few genes; `units`: gene tiles times groups
+// of a warp), or where the class bits of very many samples need the shared
+// memory.  The grid's second dimension (at most 65,535 blocks) is a batch's
+// groups by the warps of a block.
+constexpr int kMetricMaxPerms = 4 * 65535;
+template <int ACC, class T>
+int metric_warps(int64_t units, int64_t groups, int S) {
+    const int64_t want = 2 * (int64_t)metric_sms();
+    int w = kMaxWarps;
+    while (w > 1 && (units / w < want || metric_smem<ACC, T>(w, S) > 110 * 1024) &&
+           (groups + w / 2 - 1) / (w / 2) <= 65535)
+        w >>= 1;
+    return w;
 }
 
-template <int ACC, int COMB, int PB>
-__global__ void __launch_bounds__(128, 8)
-metric_fast_kernel(const float* __restrict__ X, int G, int S, const uint32_t* __restrict__ masks, int words,
-                   int num_perms, float nA, float nB, float* __restrict__ keys, const int* __restrict__ fast_ok) {
-    metric_fast_block<ACC, COMB, PB>(X, G, S, masks, words, num_perms, nA, nB, keys, fast_ok, blockIdx.x,
-                                     blockIdx.y);
+// Rounds of a warp: as tuned, but where the tile stays in shared memory as
+// many as leave four waves of blocks (2,000 genes x 40 samples x 1,024
+// permutations: the copies and their latency once per block, not per round).
+template <int ACC, class T>
+int metric_rounds(int64_t tiles, int64_t num_perms, int S, int tuned) {
+    if (S > 2 * kChunk) return tuned;
+    const int64_t blocks = tiles * num_perms / (metric_q<T>() * kMaxWarps);
+    const int64_t r = blocks / (16 * (int64_t)metric_sms());
+    return r < tuned ? tuned : r > 16 ? 16 : (int)r;
 }
 
-template <int ACC, int COMB, int PB>
-__global__ void __launch_bounds__(128, 8) metric_fast_multi(const MetricTask<float>* __restrict__ tasks) {
-    const MetricTask<float> t = tasks[blockIdx.z];
-    if ((int)blockIdx.x * 128 >= t.G || (int)blockIdx.y * PB >= t.num_perms) return;
-    metric_fast_block<ACC, COMB, PB>(t.X, t.G, t.S, t.masks, t.words, t.num_perms, t.nA, t.nB, t.keys, t.fast_ok,
-                                     blockIdx.x, blockIdx.y);
-}
-
-template <int ACC, int COMB, int PB>
-cudaError_t launch_metric_fast_pb(const float* X, int G, int S, const uint32_t* masks, int words, int num_perms,
-                                  int64_t nA, int64_t nB, float* keys, const int* fast_ok, cudaStream_t st) {
-    const int threads = 128;
-    dim3 grid((G + threads - 1) / threads, (num_perms + PB - 1) / PB);
-    const size_t smem = sizeof(ulonglong2) * (size_t)S * (PB / 2) + sizeof(uint32_t) * PB * words;
-    auto kern = metric_fast_kernel<ACC, COMB, PB>;
+template <int ACC, class T>
+cudaError_t launch_metric_acc(int comb, const T* X, int G, int S, const uint32_t* masks, int words, int num_perms,
+                              int64_t nA, int64_t nB, T* keys, const int* finite, int tuned, cudaStream_t st) {
+    const int tiles = (G + metric_genes<ACC, T>() - 1) / metric_genes<ACC, T>();
+    const int rounds = metric_rounds<ACC, T>(tiles, num_perms, S, tuned);
+    const int per = metric_q<T>() * rounds, groups = (num_perms + per - 1) / per;
+    const int w = metric_warps<ACC, T>((int64_t)tiles * groups, groups, S);
+    const size_t smem = metric_smem<ACC, T>(w, S);
+    auto kern = metric_kernel<ACC, T>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    kern<<<grid, threads, smem, st>>>(X, G, S, masks, words, num_perms, (float)nA, (float)nB, keys, fast_ok);
+    kern<<<dim3((unsigned)tiles, (unsigned)((groups + w - 1) / w)), 32 * w, smem, st>>>(
+        X, G, S, masks, words, num_perms, (T)nA, (T)nB, keys, comb, finite, rounds);
     launches_add(1);
     return cudaGetLastError();
 }
 
-// pb: permutations per thread (4 or 8; 0 = 8), identical keys either way
-template <int ACC, int COMB>
-cudaError_t launch_metric_fast(const float* X, int G, int S, const uint32_t* masks, int words, int num_perms,
-                               int64_t nA, int64_t nB, float* keys, const int* fast_ok, int pb, cudaStream_t st) {
-    if (pb == 4)
-        return launch_metric_fast_pb<ACC, COMB, 4>(X, G, S, masks, words, num_perms, nA, nB, keys, fast_ok, st);
-    return launch_metric_fast_pb<ACC, COMB, 8>(X, G, S, masks, words, num_perms, nA, nB, keys, fast_ok, st);
+// accumulator and combiner of a metric id
+inline bool metric_parts(int metric, int& acc, int& comb) {
+    static const int accs[14] = {ACC_NAIVE, ACC_NAIVE, ACC_NAIVE, ACC_KAHAN, ACC_KAHAN, ACC_KAHAN, ACC_ONEPASS,
+                                 ACC_ONEPASS, ACC_TWOPASS, ACC_TWOPASS, ACC_KNUTH, ACC_KNUTH, ACC_OVERKILL,
+                                 ACC_OVERKILL};
+    static const int combs[14] = {COMB_DIFF, COMB_RATIO, COMB_LOG2, COMB_DIFF, COMB_RATIO, COMB_LOG2, COMB_S2N,
+                                  COMB_TTEST, COMB_S2N, COMB_TTEST, COMB_S2N, COMB_TTEST, COMB_S2N, COMB_TTEST};
+    if (metric < 0 || metric >= 14) return false;
+    acc = accs[metric];
+    comb = combs[metric];
+    return true;
 }
 
-template <int ACC, int COMB, class T>
-cudaError_t launch_metric_t(const T* X, int G, int S, const uint32_t* masks, int words,
-                            int num_perms, int64_t nA, int64_t nB, T* keys, cudaStream_t st) {
-    constexpr int PB = 8;
-    const int threads = 128;
-    dim3 grid((G + threads - 1) / threads, (num_perms + PB - 1) / PB);
-    const size_t smem = sizeof(uint32_t) * PB * words;
-    metric_kernel<ACC, COMB, T, PB><<<grid, threads, smem, st>>>(X, G, S, masks, words, num_perms,
-                                                                 (T)nA, (T)nB, keys);
-    launches_add(1);
-    return cudaGetLastError();
-}
+#define GSEA_BY_ACC(CALL)                      \
+    switch (acc) {                             \
+        case ACC_NAIVE: CALL(ACC_NAIVE);       \
+        case ACC_KAHAN: CALL(ACC_KAHAN);       \
+        case ACC_ONEPASS: CALL(ACC_ONEPASS);   \
+        case ACC_TWOPASS: CALL(ACC_TWOPASS);   \
+        case ACC_KNUTH: CALL(ACC_KNUTH);       \
+        default: CALL(ACC_OVERKILL);           \
+    }
 
+// pb: rounds of a warp, 4 (0): one, 8: two; identical keys
 template <class T>
-cudaError_t launch_metric_impl(int metric, const T* X, int G, int S, const uint32_t* masks,
-                               int words, int num_perms, int64_t nA, int64_t nB, T* keys,
-                               const int* fast_ok, cudaStream_t st, int pb) {
-    if (pb != 0 && pb != 4 && pb != 8) return cudaErrorInvalidValue;
+cudaError_t launch_metric_impl(int metric, const T* X, int G, int S, const uint32_t* masks, int words, int num_perms,
+                               int64_t nA, int64_t nB, T* keys, const int* finite, cudaStream_t st, int pb) {
+    int acc, comb;
+    if ((pb != 0 && pb != 4 && pb != 8) || !metric_parts(metric, acc, comb)) return cudaErrorInvalidValue;
     if (num_perms <= 0) return cudaSuccess;
-    if constexpr (std::is_same<T, float>::value) {
-      if (fast_ok && (size_t)S * 4 * 16 + 32 * (size_t)words <= 100 * 1024) {
-        const float* Xf = X;
-        float* kf = keys;
-        switch (metric) {
-            case 0: return launch_metric_fast<ACC_NAIVE, COMB_DIFF>(Xf, G, S, masks, words, num_perms, nA, nB, kf, fast_ok, pb, st);
-            case 1: return launch_metric_fast<ACC_NAIVE, COMB_RATIO>(Xf, G, S, masks, words, num_perms, nA, nB, kf, fast_ok, pb, st);
-            case 2: return launch_metric_fast<ACC_NAIVE, COMB_LOG2>(Xf, G, S, masks, words, num_perms, nA, nB, kf, fast_ok, pb, st);
-            case 6: return launch_metric_fast<ACC_ONEPASS, COMB_S2N>(Xf, G, S, masks, words, num_perms, nA, nB, kf, fast_ok, pb, st);
-            case 7: return launch_metric_fast<ACC_ONEPASS, COMB_TTEST>(Xf, G, S, masks, words, num_perms, nA, nB, kf, fast_ok, pb, st);
-            case 8: return launch_metric_fast<ACC_TWOPASS, COMB_S2N>(Xf, G, S, masks, words, num_perms, nA, nB, kf, fast_ok, pb, st);
-            case 9: return launch_metric_fast<ACC_TWOPASS, COMB_TTEST>(Xf, G, S, masks, words, num_perms, nA, nB, kf, fast_ok, pb, st);
-            default: break;
-        }
-      }
-    }
-#define GSEA_M(ID, A, C)                                                                        \
-    case ID:                                                                                   \
-        return launch_metric_t<A, C, T>(X, G, S, masks, words, num_perms, nA, nB, keys, st);
-    switch (metric) {
-        GSEA_M(0, ACC_NAIVE, COMB_DIFF)
-        GSEA_M(1, ACC_NAIVE, COMB_RATIO)
-        GSEA_M(2, ACC_NAIVE, COMB_LOG2)
-        GSEA_M(3, ACC_KAHAN, COMB_DIFF)
-        GSEA_M(4, ACC_KAHAN, COMB_RATIO)
-        GSEA_M(5, ACC_KAHAN, COMB_LOG2)
-        GSEA_M(6, ACC_ONEPASS, COMB_S2N)
-        GSEA_M(7, ACC_ONEPASS, COMB_TTEST)
-        GSEA_M(8, ACC_TWOPASS, COMB_S2N)
-        GSEA_M(9, ACC_TWOPASS, COMB_TTEST)
-        GSEA_M(10, ACC_KNUTH, COMB_S2N)
-        GSEA_M(11, ACC_KNUTH, COMB_TTEST)
-        GSEA_M(12, ACC_OVERKILL, COMB_S2N)
-        GSEA_M(13, ACC_OVERKILL, COMB_TTEST)
-        default:
-            return cudaErrorInvalidValue;
-    }
-#undef GSEA_M
+    if (num_perms > kMetricMaxPerms) return cudaErrorInvalidValue;
+#define GSEA_CALL(A) \
+    return launch_metric_acc<A, T>(comb, X, G, S, masks, words, num_perms, nA, nB, keys, finite, pb == 8 ? 2 : 1, st)
+    GSEA_BY_ACC(GSEA_CALL)
+#undef GSEA_CALL
 }
 
 // Batched instances: the group key of an instance (instances with equal keys
-// share one launch) -- the metric and the path launch_metric_impl takes for
-// it (exact, or packed with 4 or 8 permutations per thread).
-template <class T>
-int metric_multi_key_impl(int metric, int S, int words, bool fast_ok, int pb) {
-    bool fast = false;
-    if constexpr (std::is_same<T, float>::value)
-        fast = fast_ok && (size_t)S * 4 * 16 + 32 * (size_t)words <= 100 * 1024 &&
-               (metric <= 2 || (metric >= 6 && metric <= 9));
-    return metric * 4 + (fast ? (pb == 4 ? 1 : 2) : 0);
-}
+// share one launch): the metric and the rounds of a warp.
+inline int metric_multi_key_impl(int metric, int pb) { return metric * 2 + (pb == 8 ? 1 : 0); }
 
-// grid over the largest instance of a group; PB permutations per thread,
-// `lab` bytes of packed class weights per sample (0 for the exact form)
-template <class T>
-void multi_extent(const MetricTask<T>* h, int n, int PB, size_t lab, dim3& grid, size_t& smem) {
-    unsigned gx = 1, gy = 1;
-    smem = 0;
+template <int ACC, class T>
+cudaError_t launch_metric_multi_acc(int comb, int rounds, const MetricTask<T>* d, const MetricTask<T>* h, int n,
+                                    cudaStream_t st) {
+    int64_t tiles = 1, groups = 1, work = 0;
+    int smax = 0;
     for (int i = 0; i < n; i++) {
-        gx = std::max(gx, (unsigned)((h[i].G + 127) / 128));
-        gy = std::max(gy, (unsigned)((h[i].num_perms + PB - 1) / PB));
-        smem = std::max(smem, lab * (size_t)h[i].S + sizeof(uint32_t) * PB * (size_t)h[i].words);
+        const int64_t t = (h[i].G + metric_genes<ACC, T>() - 1) / metric_genes<ACC, T>();
+        const int per = metric_q<T>() * rounds;
+        const int64_t g = (h[i].num_perms + per - 1) / per;
+        tiles = std::max(tiles, t);
+        groups = std::max(groups, g);
+        work += t * g;
+        smax = std::max(smax, h[i].S);
     }
-    grid = dim3(gx, gy, (unsigned)n);
-}
-
-template <int ACC, int COMB, int PB>
-cudaError_t launch_fast_multi_pb(const MetricTask<float>* d, const MetricTask<float>* h, int n, cudaStream_t st) {
-    dim3 grid;
-    size_t smem;
-    multi_extent<float>(h, n, PB, sizeof(ulonglong2) * (PB / 2), grid, smem);
-    auto kern = metric_fast_multi<ACC, COMB, PB>;
+    const int w = metric_warps<ACC, T>(work, groups, smax);
+    const size_t smem = metric_smem<ACC, T>(w, smax);
+    auto kern = metric_multi<ACC, T>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    kern<<<grid, 128, smem, st>>>(d);
-    launches_add(1);
-    return cudaGetLastError();
-}
-
-template <int ACC, int COMB, class T>
-cudaError_t launch_exact_multi(const MetricTask<T>* d, const MetricTask<T>* h, int n, cudaStream_t st) {
-    constexpr int PB = 8;
-    dim3 grid;
-    size_t smem;
-    multi_extent<T>(h, n, PB, 0, grid, smem);
-    auto kern = metric_multi<ACC, COMB, T, PB>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    kern<<<grid, 128, smem, st>>>(d);
+    kern<<<dim3((unsigned)tiles, (unsigned)((groups + w - 1) / w), (unsigned)n), 32 * w, smem, st>>>(d, comb, rounds);
     launches_add(1);
     return cudaGetLastError();
 }
@@ -561,50 +755,13 @@ cudaError_t launch_metric_multi_impl(int key, const MetricTask<T>* d, const Metr
     if (n <= 0) return cudaSuccess;
     if (n > 65535) return cudaErrorInvalidValue;
     for (int i = 0; i < n; i++)
-        if ((h[i].num_perms + 7) / 8 > 65535) return cudaErrorInvalidValue;
-    const int metric = key / 4, path = key % 4;
-    if constexpr (std::is_same<T, float>::value) {
-        if (path != 0) {
-#define GSEA_F(ID, A, C)                                                                   \
-    case ID:                                                                              \
-        return path == 1 ? launch_fast_multi_pb<A, C, 4>(d, h, n, st) : launch_fast_multi_pb<A, C, 8>(d, h, n, st);
-            switch (metric) {
-                GSEA_F(0, ACC_NAIVE, COMB_DIFF)
-                GSEA_F(1, ACC_NAIVE, COMB_RATIO)
-                GSEA_F(2, ACC_NAIVE, COMB_LOG2)
-                GSEA_F(6, ACC_ONEPASS, COMB_S2N)
-                GSEA_F(7, ACC_ONEPASS, COMB_TTEST)
-                GSEA_F(8, ACC_TWOPASS, COMB_S2N)
-                GSEA_F(9, ACC_TWOPASS, COMB_TTEST)
-                default:
-                    return cudaErrorInvalidValue;
-            }
-#undef GSEA_F
-        }
-    }
-    if (path != 0) return cudaErrorInvalidValue;
-#define GSEA_X(ID, A, C) \
-    case ID:             \
-        return launch_exact_multi<A, C, T>(d, h, n, st);
-    switch (metric) {
-        GSEA_X(0, ACC_NAIVE, COMB_DIFF)
-        GSEA_X(1, ACC_NAIVE, COMB_RATIO)
-        GSEA_X(2, ACC_NAIVE, COMB_LOG2)
-        GSEA_X(3, ACC_KAHAN, COMB_DIFF)
-        GSEA_X(4, ACC_KAHAN, COMB_RATIO)
-        GSEA_X(5, ACC_KAHAN, COMB_LOG2)
-        GSEA_X(6, ACC_ONEPASS, COMB_S2N)
-        GSEA_X(7, ACC_ONEPASS, COMB_TTEST)
-        GSEA_X(8, ACC_TWOPASS, COMB_S2N)
-        GSEA_X(9, ACC_TWOPASS, COMB_TTEST)
-        GSEA_X(10, ACC_KNUTH, COMB_S2N)
-        GSEA_X(11, ACC_KNUTH, COMB_TTEST)
-        GSEA_X(12, ACC_OVERKILL, COMB_S2N)
-        GSEA_X(13, ACC_OVERKILL, COMB_TTEST)
-        default:
-            return cudaErrorInvalidValue;
-    }
-#undef GSEA_X
+        if (h[i].num_perms > kMetricMaxPerms) return cudaErrorInvalidValue;
+    int acc, comb;
+    if (!metric_parts(key / 2, acc, comb)) return cudaErrorInvalidValue;
+#define GSEA_CALL(A) return launch_metric_multi_acc<A, T>(comb, key % 2 + 1, d, h, n, st)
+    GSEA_BY_ACC(GSEA_CALL)
+#undef GSEA_CALL
 }
+#undef GSEA_BY_ACC
 
 }  // namespace gsea

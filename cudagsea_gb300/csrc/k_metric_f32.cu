@@ -8,8 +8,8 @@ cudaError_t launch_metric<float>(int metric, const float* X, int G, int S, const
     return launch_metric_impl<float>(metric, X, G, S, masks, words, num_perms, nA, nB, keys, fast_ok, st, pb);
 }
 template <>
-int metric_multi_key<float>(int metric, int S, int words, bool fast_ok, int pb) {
-    return metric_multi_key_impl<float>(metric, S, words, fast_ok, pb);
+int metric_multi_key<float>(int metric, int pb) {
+    return metric_multi_key_impl(metric, pb);
 }
 template <>
 cudaError_t launch_metric_multi<float>(int key, const MetricTask<float>* d, const MetricTask<float>* h, int n,

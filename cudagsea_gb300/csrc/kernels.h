@@ -12,20 +12,19 @@ cudaError_t launch_permute(const uint8_t* labels, int S, int64_t num_perms, int6
                            uint32_t seed, uint32_t* masks, int words, cudaStream_t st);
 
 // Plain-form class statistics + metric: keys[p][g] for p < num_perms.
-// fast_ok (device int, may be null): set by launch_finite_check; non-zero lets
-// the fp32 kernels use the packed form (bit-identical for finite inputs).
+// fast_ok (device int, may be null): set by launch_finite_check; zero makes the
+// naive accumulators add 0 * x to the other class, as the reference does
+// (nothing for finite values).
 template <class T>
 cudaError_t launch_metric(int metric, const T* exprs, int G, int S, const uint32_t* masks,
                           int words, int num_perms, int64_t nA, int64_t nB, T* keys,
                           const int* fast_ok, cudaStream_t st, int pb = 0);
-// (pb: permutations per thread of the packed fp32 form, 4 or 8; 0 = 8)
+// (pb: permutations a warp takes, 4 or 8 in two rounds; 0 = 4)
 
 // Batched instances: one launch of the metric over every instance of a group
 // (blockIdx.z = instance), keys bit-identical to launch_metric's.  Instances
-// share a group when metric_multi_key agrees (metric, and the path -- exact or
-// packed with pb permutations per thread -- that launch_metric takes; fast_ok:
-// the instance has a finite-check flag).  At most 65,535 instances and
-// 524,280 permutations per instance.
+// share a group when metric_multi_key agrees (metric and pb).  At most 65,535
+// instances and 262,140 permutations per instance.
 template <class T>
 struct MetricTask {
     const T* X;
@@ -36,7 +35,7 @@ struct MetricTask {
     T nA, nB;
 };
 template <class T>
-int metric_multi_key(int metric, int S, int words, bool fast_ok, int pb);
+int metric_multi_key(int metric, int pb);
 template <class T>
 cudaError_t launch_metric_multi(int key, const MetricTask<T>* d_tasks, const MetricTask<T>* h_tasks, int n,
                                 cudaStream_t st);

@@ -57,7 +57,7 @@ struct gsea_plan_s {
     std::vector<int32_t> h_set_order;  // host staging of set_order
     std::vector<int64_t> h_set_size;   // members of each set (after mapping)
     uint32_t* masks = nullptr;
-    int* fast_ok = nullptr;            // expression values allow the packed metric form
+    int* fast_ok = nullptr;            // the expression values are finite (and below 2^60)
     void* decay = nullptr;             // [G+1] T: miss step per hit count
     // chosen form (tensor-core class statistics)
     float* gene_mu = nullptr;

@@ -275,7 +275,7 @@ int gsea_stats_device_noalloc(const void* es, int64_t num_sets, int64_t num_perm
  *      Every setting computes identical results; only the speed differs.
  *      0 / -1 leave a choice automatic.                                    */
 typedef struct gsea_tuning {
-    int32_t metric_pb;    /* plain fp32 metric: permutations per thread, 4 or 8 */
+    int32_t metric_pb;    /* plain metric: permutations a warp takes, 4 or 8 (in two rounds) */
     int32_t chosen_tile;  /* tensor-core form: permutations per tile, 128 (the automatic choice: one
                              persistent CTA per SM walking the tiles, the copies, MMAs and
                              epilogue on separate warps) or 256 (one tile per CTA) */
