@@ -432,29 +432,31 @@ int autotune_b(gsea_batch_s* b, int64_t n) {
         const int64_t items = std::min<int64_t>(b->classes[ci].nitems, std::max<int64_t>(n, 1) * 4);
         float best = 1e30f;
         gsea::EsTuning pick;
-        for (int w : {32, 24, 16, 8}) {
-            for (int stage : {1, 3, 2, 0}) {
-                gsea::EsTuning t;
-                t.warps = w;
-                t.stage = stage;
-                if (launch_class<T>(b, ci, items, t, b->main) != cudaSuccess) {  // warm-up, or does not fit
-                    cudaGetLastError();
-                    continue;
-                }
-                float ms_best = 1e30f;
-                for (int r = 0; r < 3; r++) {
-                    cudaEventRecord(t0, b->main);
-                    launch_class<T>(b, ci, items, t, b->main);
-                    cudaEventRecord(t1, b->main);
-                    cudaEventSynchronize(t1);
-                    float ms = 0.f;
-                    cudaEventElapsedTime(&ms, t0, t1);
-                    ms_best = std::min(ms_best, ms);
-                }
-                if (ms_best < best) {
-                    best = ms_best;
-                    pick = t;
-                }
+        std::vector<std::pair<int, int>> cands;
+        if (sizeof(T) == 8) cands.emplace_back(0, -1);  // the automatic choice stages more than may be asked for
+        for (int w : {32, 24, 16, 8})
+            for (int stage : {1, 3, 2, 0}) cands.emplace_back(w, stage);
+        for (const auto& cand : cands) {
+            gsea::EsTuning t;
+            t.warps = cand.first;
+            t.stage = cand.second;
+            if (launch_class<T>(b, ci, items, t, b->main) != cudaSuccess) {  // warm-up, or does not fit
+                cudaGetLastError();
+                continue;
+            }
+            float ms_best = 1e30f;
+            for (int r = 0; r < 3; r++) {
+                cudaEventRecord(t0, b->main);
+                launch_class<T>(b, ci, items, t, b->main);
+                cudaEventRecord(t1, b->main);
+                cudaEventSynchronize(t1);
+                float ms = 0.f;
+                cudaEventElapsedTime(&ms, t0, t1);
+                ms_best = std::min(ms_best, ms);
+            }
+            if (ms_best < best) {
+                best = ms_best;
+                pick = t;
             }
         }
         b->es_tuning[b->classes[ci].wpl] = pick;

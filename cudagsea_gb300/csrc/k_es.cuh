@@ -404,6 +404,88 @@ __device__ __forceinline__ float set_score_direct(const uint32_t* bmw, int w0, c
     return set_score_positions_f32<WPL>(bmw, w0, wt, decay, G, lane, Wt);
 }
 
+// fp64 where fp32 cannot decide: the set's weight from its marked ranks, then
+// the procedure with positions in double.  Out of line: seldom taken.
+template <int WPL>
+__device__ __noinline__ double set_score_positions_f64(const uint32_t* bmw, int w0, const double* wt,
+                                                       const double* __restrict__ decay, int G, int lane) {
+    const LaneWords<WPL> words(bmw);
+    Acc<double> Wt;
+    HitWalk<WPL> hit(bmw, w0, words);
+    for (int t = 0; t < words.cnt; t++) Wt.add(weight_at(wt, hit.next()));
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) Wt.merge(Wt.shfl_xor(o));
+    return set_score_positions<double, WPL>(bmw, w0, wt, decay, G, lane, Wt);
+}
+
+// fp64, direct procedure: the walk in fp32, to find the hit the score is
+// taken at.  The fp32 candidates are off by less than 1e-6 (weights, their
+// sum, its reciprocal, the decay and the candidate itself, each rounded to
+// fp32, values at most 1 and the prefix compensated), so an extremum ahead of
+// every other candidate by kMargin is the extremum.  Returns the rank of the
+// hit (the largest value: after it, the smallest: before it), or -1 where the
+// lead is smaller, the end of the list would win, or the weights are outside
+// fp32's range.  `wf(r4)`: the weight at rank r4 / 4 as a float.
+constexpr float kMargin = 4e-6f;
+template <int WPL, class Weight>
+__device__ __forceinline__ int find_extremum(const uint32_t* bmw, int w0, Weight&& wf,
+                                             const double* __restrict__ decay, int G, int lane,
+                                             const Acc<float>& Wt, int& n, bool& largest) {
+    const LaneWords<WPL> words(bmw);
+    const int excl = hits_before(words.cnt, lane, n);
+    const float inv = n > 0 ? 1.f / Wt.value() : 0.f;
+    largest = false;
+    if (!__all_sync(kFullMask, isfinite(Wt.value()) && isfinite(inv) && Wt.value() > 1e-30f)) return -1;
+    const float d = (float)decay[n], d4 = 0.25f * d;
+    constexpr uint32_t kMagic = 0x4b000000u;
+    uint32_t e4 = 4u * (uint32_t)excl - kMagic;
+    const uint32_t end4 = e4 + 4u * (uint32_t)words.cnt;
+    Acc<float> Wl;
+    // the extrema, the next best of each, and the hits (times four) they are at
+    float mx = -CUDART_INF_F, mx2 = -CUDART_INF_F, mn = CUDART_INF_F, mn2 = CUDART_INF_F;
+    uint32_t pmx = ~0u, pmn = ~0u;
+    HitWalk<WPL> hit(bmw, w0, words);
+#pragma unroll 2
+    while (e4 != end4) {
+        const uint32_t r4 = hit.next();
+        const float m4 = __fadd_rn(__uint_as_float(r4 - e4), -8388608.f);
+        const float md = __fmul_rn(-m4, d4);
+        const float before = Wl.scaled_plus(inv, md);
+        mn2 = fminf(mn2, fmaxf(mn, before));
+        pmn = before < mn ? r4 : pmn;
+        mn = fminf(mn, before);
+        Wl.add(wf(r4));
+        const float after = Wl.scaled_plus(inv, md);
+        mx2 = fmaxf(mx2, fminf(mx, after));
+        pmx = after > mx ? r4 : pmx;
+        mx = fmaxf(mx, after);
+        e4 += 4u;
+    }
+    const float shift = weight_before<float>(Wl, excl, inv, lane);
+    mx += shift;
+    mx2 += shift;
+    mn += shift;
+    mn2 += shift;
+    if (lane == 31) {  // end of the list: no hit to evaluate at
+        const float end = Wt.scaled_plus(inv, -(float)(G - n) * d);
+        mn2 = fminf(mn2, fmaxf(mn, end));
+        if (end < mn) {
+            mn = end;
+            pmn = ~0u;
+        }
+    }
+    const float up = __uint_as_float(warp_top(mx)), down = __uint_as_float(warp_top(-mn));
+    largest = up > down;
+    if (fabsf(up - down) <= kMargin) return -1;
+    const float lead = largest ? up : -down;
+    const float first = largest ? mx : -mn, second = largest ? mx2 : -mn2;
+    const uint32_t near = __ballot_sync(kFullMask, first >= fabsf(lead) - kMargin);
+    const bool tied = __any_sync(kFullMask, second >= fabsf(lead) - kMargin);
+    if (tied || (near & (near - 1u)) != 0u || near == 0u) return -1;
+    const uint32_t at = __shfl_sync(kFullMask, largest ? pmx : pmn, __ffs((int)near) - 1);
+    return at == ~0u ? -1 : (int)(at >> 2);
+}
+
 // General procedure (any G, any set size): each lane walks its own word range
 // twice -- weights first, then candidates with the exact prefix from a scan.
 template <class T>
@@ -499,14 +581,32 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
     const int w0 = min(lane * wpl, words), w1 = min(w0 + wpl, words);
     __syncthreads();  // previous permutation finished with the staging and the counter
     if (tid == 0) *next_set = 0;
+    constexpr bool F64 = std::is_same<T, double>::value && WPL > 0;  // walk in fp32, score from double sums
+    float* const s_wf = reinterpret_cast<float*>(s_w);
     if (STAGE) {
         for (int i = tid; i < G; i += WARPS * 32) {
-            if (STAGE == 1 || STAGE == 3) s_w[i] = wt[i];
+            if (STAGE == 1 || STAGE == 3) {
+                if constexpr (F64) s_wf[i] = (float)wt[i];
+                else s_w[i] = wt[i];
+            }
             if (STAGE == 1 || STAGE == 2) s_rank[i] = rk[i];
         }
         if (STAGE == 1 || STAGE == 2) rk = s_rank;
-        if (STAGE == 1 || STAGE == 3) wt = s_w;
+        if ((STAGE == 1 || STAGE == 3) && !F64) wt = s_w;
     }
+    // fp64: the scores of up to 32 sets wait in the lanes for their division
+    double up_to = 0.0, beyond = 0.0;  // weight up to the extremum, weight after it
+    int misses = 0, hits = 0, waiting = -1, held = 0;
+    auto flush = [&]() {
+        if constexpr (F64) {
+            if (waiting >= 0) {
+                const double inv = 1.0 / (up_to + beyond);
+                es_col[(int64_t)waiting * es_stride] = fma(up_to, inv, -(double)misses * decay[hits]);
+            }
+            waiting = -1;
+            held = 0;
+        }
+    };
     __syncthreads();
     while (true) {
         int slot = 0;
@@ -520,17 +620,21 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
         const int k = set_order ? set_order[slot] : slot;
         T score;
         if constexpr (WPL > 0) {
-            Acc<T> Wm;
+            auto weight = [&](uint32_t r) -> float {
+                if constexpr (F64) return STAGE == 1 || STAGE == 3 ? s_wf[r] : (float)wt[r];
+                else return wt[r];
+            };
+            Acc<float> Wm;
             const int2 rec = __ldg(sets.rec + k);  // first group of the set's list, members
+            const uint2* __restrict__ const list = sets.list + (int64_t)rec.x * 32 + lane;
+            const int full = rec.y >> 7, rem = rec.y & 127;
             if (rec.y >= 0) {
-                const uint2* __restrict__ list = sets.list + (int64_t)rec.x * 32 + lane;
-                const int full = rec.y >> 7, rem = rec.y & 127;
 #pragma unroll 1
-                for (int i = 0; i < full; i++, list += 32) {
-                    const uint2 q = __ldg(list);
+                for (int i = 0; i < full; i++) {
+                    const uint2 q = __ldg(list + 32 * i);
                     const uint32_t r0 = rk[q.x & 0xffffu], r1 = rk[q.x >> 16];
                     const uint32_t r2 = rk[q.y & 0xffffu], r3 = rk[q.y >> 16];
-                    const T a0 = wt[r0], a1 = wt[r1], a2 = wt[r2], a3 = wt[r3];
+                    const float a0 = weight(r0), a1 = weight(r1), a2 = weight(r2), a3 = weight(r3);
                     mark<WPL>(bm, r0);
                     mark<WPL>(bm, r1);
                     mark<WPL>(bm, r2);
@@ -541,14 +645,14 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
                     Wm.add(a3);
                 }
                 if (rem) {
-                    const uint2 q = __ldg(list);
+                    const uint2 q = __ldg(list + 32 * full);
                     const uint32_t g[4] = {q.x & 0xffffu, q.x >> 16, q.y & 0xffffu, q.y >> 16};
                     uint32_t r[4];
-                    T a[4];
+                    float a[4];
 #pragma unroll
                     for (int i = 0; i < 4; i++) {  // the unused entries of a list are gene 0
                         r[i] = rk[g[i]];
-                        a[i] = wt[r[i]];
+                        a[i] = weight(r[i]);
                     }
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
@@ -567,7 +671,7 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
                     if (g >= 0 && g < G) {
                         const uint32_t r = rk[g];
                         const uint32_t bit = __funnelshift_r(0x80000000u, 0u, r);
-                        if (!(atomicOr(rank_word<WPL>(bm, r), bit) & bit)) Wm.add(wt[r]);
+                        if (!(atomicOr(rank_word<WPL>(bm, r), bit) & bit)) Wm.add(weight(r));
                     }
                 }
             }
@@ -575,12 +679,78 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
 #pragma unroll
             for (int o = 16; o >= 1; o >>= 1) Wm.merge(Wm.shfl_xor(o));  // the set's weight, every lane
             uint32_t* const bmw = bm + lane * lane_stride<WPL>();
-            if constexpr (std::is_same<T, float>::value) {
+            if constexpr (!F64) {
                 score = set_score_direct<WPL>(bmw, lane * WPL, wt, decay, G, lane, Wm);
+                clear_words<WPL>(bmw);
             } else {
-                score = set_score_positions<T, WPL>(bmw, lane * WPL, wt, decay, G, lane, Wm);
+                int n;
+                bool largest;
+                const int at = rec.y < 0 ? -1
+                                         : find_extremum<WPL>(
+                                               bmw, lane * WPL,
+                                               [&](uint32_t r4) -> float {
+                                                   if constexpr (STAGE == 1 || STAGE == 3) return weight_at(s_wf, r4);
+                                                   else return (float)weight_at(wt, r4);
+                                               },
+                                               decay, G, lane, Wm, n, largest);
+                if (at < 0) {  // warp-uniform
+                    score = set_score_positions_f64<WPL>(bmw, lane * WPL, wt, decay, G, lane);
+                    clear_words<WPL>(bmw);
+                } else {
+                    clear_words<WPL>(bmw);
+                    // the members' weights once more, in double, on either side
+                    // of the extremum: one addition a member
+                    const uint32_t limit = (uint32_t)at + (largest ? 1u : 0u);
+                    double lo = 0.0, hi = 0.0;
+                    int before = 0;
+                    auto add = [&](uint32_t r, double w) {
+                        const bool in = r < limit;
+                        const double sum = (in ? lo : hi) + w;
+                        lo = in ? sum : lo;
+                        hi = in ? hi : sum;
+                        before += r < (uint32_t)at ? 1 : 0;
+                    };
+#pragma unroll 1
+                    for (int i = 0; i < full; i++) {
+                        const uint2 q = __ldg(list + 32 * i);
+                        const uint32_t r0 = rk[q.x & 0xffffu], r1 = rk[q.x >> 16];
+                        const uint32_t r2 = rk[q.y & 0xffffu], r3 = rk[q.y >> 16];
+                        const double a0 = wt[r0], a1 = wt[r1], a2 = wt[r2], a3 = wt[r3];
+                        add(r0, a0);
+                        add(r1, a1);
+                        add(r2, a2);
+                        add(r3, a3);
+                    }
+                    if (rem) {
+                        const uint2 q = __ldg(list + 32 * full);
+                        const uint32_t g[4] = {q.x & 0xffffu, q.x >> 16, q.y & 0xffffu, q.y >> 16};
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            if (lane + 32 * i < rem) {
+                                const uint32_t r = rk[g[i]];
+                                add(r, wt[r]);
+                            }
+                        }
+                    }
+                    before = __reduce_add_sync(kFullMask, before);
+                    // both sums in five steps: after the first, lanes 0-15 hold
+                    // one and lanes 16-31 the other
+                    double mine = (lane < 16 ? lo : hi) + __shfl_xor_sync(kFullMask, lane < 16 ? hi : lo, 16);
+#pragma unroll
+                    for (int o = 8; o >= 1; o >>= 1) mine += __shfl_xor_sync(kFullMask, mine, o);
+                    const double s_lo = __shfl_sync(kFullMask, mine, 0), s_hi = __shfl_sync(kFullMask, mine, 16);
+                    if (lane == held) {
+                        up_to = s_lo;
+                        beyond = s_hi;
+                        misses = at - before;
+                        hits = n;
+                        waiting = k;
+                    }
+                    if (++held == 32) flush();
+                    __syncwarp();
+                    continue;
+                }
             }
-            clear_words<WPL>(bmw);
         } else {
             // mark the members' ranks (duplicates and unknown ids fall away)
             const int64_t a = sets.off[k];
@@ -598,14 +768,18 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
         if (lane == 0) es_col[(int64_t)k * es_stride] = score;
         __syncwarp();
     }
+    flush();
 }
 
-// bytes of a CTA's staging: weights + ranks (1), ranks (2), weights (3), none (0)
+// bytes of a CTA's staging: weights + ranks (1), ranks (2), weights (3), none
+// (0); the direct procedures stage fp64 weights as floats (the walk's)
+template <class T, class RankT>
+__host__ __device__ constexpr size_t es_weight_bytes() { return sizeof(RankT) == 2 ? 4 : sizeof(T); }
 template <class T, class RankT, int STAGE>
 __host__ __device__ __forceinline__ size_t es_stage_bytes(int G) {
-    return STAGE == 1   ? (sizeof(T) + sizeof(RankT)) * (size_t)G
+    return STAGE == 1   ? (es_weight_bytes<T, RankT>() + sizeof(RankT)) * (size_t)G
            : STAGE == 2 ? sizeof(RankT) * (size_t)G
-           : STAGE == 3 ? sizeof(T) * (size_t)G
+           : STAGE == 3 ? es_weight_bytes<T, RankT>() * (size_t)G
                         : 0;
 }
 
@@ -615,7 +789,7 @@ __device__ __forceinline__ void es_smem_layout(unsigned char* smem, int G, int r
                                                uint32_t*& bm) {
     const int warp = threadIdx.x >> 5;
     s_w = reinterpret_cast<T*>(smem);
-    s_rank = reinterpret_cast<RankT*>(smem + (STAGE == 1 ? sizeof(T) * (size_t)G : 0));
+    s_rank = reinterpret_cast<RankT*>(smem + (STAGE == 1 ? es_weight_bytes<T, RankT>() * (size_t)G : 0));
     size_t bm_off = es_stage_bytes<T, RankT, STAGE>(G);
     bm_off = (bm_off + 15) & ~(size_t)15;
     bm = reinterpret_cast<uint32_t*>(smem + bm_off) + (size_t)warp * region;
@@ -737,9 +911,12 @@ size_t es_smem_bytes(int G) {
 // with 28 KB of L1 772 us, 16 warps with 92 KB 477; 45,000: 32 warps 731, 24
 // warps 380), so more warps are only worth it while the bitmaps stay below
 // 164 KB.
-inline bool es_fits(int warps, int stage, size_t smem, int wpl, size_t cap, bool leave_l1, const EsTuning& tune) {
+// `asked`: what an explicit request of staged weights must leave room for
+// (fp64: the weights themselves, though the kernel stages them as floats).
+inline bool es_fits(int warps, int stage, size_t smem, size_t asked, int wpl, size_t cap, bool leave_l1,
+                    const EsTuning& tune) {
     constexpr size_t kLeavesL1 = 163 * 1024;
-    if (smem > cap) return false;
+    if (smem + (tune.stage == 1 || tune.stage == 3 ? asked : 0) > cap) return false;
     if ((stage >= 2 || warps == 24) && wpl < 24) return false;
     if (stage == 1 && wpl >= 40) return false;
     if (tune.warps && tune.warps != warps) return false;
@@ -821,25 +998,29 @@ cudaError_t launch_es_t(const RankT* ranks, const T* sorted_abs, int G, int P, c
     const size_t cap = (size_t)max_smem - 64;  // static shared counter
     const int grid = sms;  // times the resident CTAs per SM; the last round's permutations are split by sets
     // candidates in the automatic order (es_fits): staging the weights first,
-    // 32 warps, then 24; then nothing staged.  The partial stagings are for
-    // the large-G classes (24-64 bitmap words per lane)
+    // 32 warps, then 24; then the ranks at 24 warps (36,161 genes, 116 x 4,105
+    // scores: 1,049 us, against 1,102 for 32 warps and nothing staged); then
+    // nothing.  The partial stagings are for the large-G classes (24-64 bitmap
+    // words per lane)
     struct Cand { int warps; int stage; size_t smem; };
     const Cand cands[] = {{32, 1, es_smem_bytes<T, RankT, 32, 1>(G)},
                           {32, 3, es_smem_bytes<T, RankT, 32, 3>(G)},
                           {24, 3, es_smem_bytes<T, RankT, 24, 3>(G)},
+                          {24, 2, es_smem_bytes<T, RankT, 24, 2>(G)},
                           {32, 0, es_smem_bytes<T, RankT, 32, 0>(G)},
                           {24, 0, es_smem_bytes<T, RankT, 24, 0>(G)},
                           {16, 0, es_smem_bytes<T, RankT, 16, 0>(G)},
                           {32, 2, es_smem_bytes<T, RankT, 32, 2>(G)},
                           {16, 1, es_smem_bytes<T, RankT, 16, 1>(G)},
-                          {24, 2, es_smem_bytes<T, RankT, 24, 2>(G)},
                           {16, 2, es_smem_bytes<T, RankT, 16, 2>(G)},
                           {8, 1, es_smem_bytes<T, RankT, 8, 1>(G)},
                           {8, 0, es_smem_bytes<T, RankT, 8, 0>(G)}};
     const int wpl = es_wpl(G, sizeof(RankT) == 2);
     for (int pass = 0; pass < 2; pass++)
     for (const Cand& c : cands) {
-        if (!es_fits(c.warps, c.stage, c.smem, wpl, cap, pass == 0, tune)) continue;
+        if (!es_fits(c.warps, c.stage, c.smem, (sizeof(T) - es_weight_bytes<T, RankT>()) * (size_t)G, wpl, cap,
+                     pass == 0, tune))
+            continue;
 #define GSEA_ES(W, S) \
     return launch_es_w<T, RankT, W, S>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, \
                                        K_dev)
@@ -933,18 +1114,20 @@ cudaError_t launch_es_batch(const EsTask<T>* tasks, const int64_t* item_end, int
     const Cand cands[] = {{32, 1, es_smem_bytes<T, uint16_t, 32, 1>(Gmax)},
                           {32, 3, es_smem_bytes<T, uint16_t, 32, 3>(Gmax)},
                           {24, 3, es_smem_bytes<T, uint16_t, 24, 3>(Gmax)},
+                          {24, 2, es_smem_bytes<T, uint16_t, 24, 2>(Gmax)},
                           {32, 0, es_smem_bytes<T, uint16_t, 32, 0>(Gmax)},
                           {24, 0, es_smem_bytes<T, uint16_t, 24, 0>(Gmax)},
                           {16, 0, es_smem_bytes<T, uint16_t, 16, 0>(Gmax)},
                           {32, 2, es_smem_bytes<T, uint16_t, 32, 2>(Gmax)},
                           {16, 1, es_smem_bytes<T, uint16_t, 16, 1>(Gmax)},
-                          {24, 2, es_smem_bytes<T, uint16_t, 24, 2>(Gmax)},
                           {16, 2, es_smem_bytes<T, uint16_t, 16, 2>(Gmax)},
                           {8, 1, es_smem_bytes<T, uint16_t, 8, 1>(Gmax)},
                           {8, 0, es_smem_bytes<T, uint16_t, 8, 0>(Gmax)}};
     for (int pass = 0; pass < 2; pass++)
     for (const Cand& c : cands) {
-        if (!es_fits(c.warps, c.stage, c.smem, wpl, cap, pass == 0, tune)) continue;
+        if (!es_fits(c.warps, c.stage, c.smem, (sizeof(T) - es_weight_bytes<T, uint16_t>()) * (size_t)Gmax, wpl, cap,
+                     pass == 0, tune))
+            continue;
 #define GSEA_ESB(W, S) return launch_es_batch_w<T, W, S>(tasks, item_end, ntasks, nitems, counter, Gmax, wpl, st)
         if (c.warps == 32 && c.stage == 1) GSEA_ESB(32, 1);
         if (c.warps == 16 && c.stage == 1) GSEA_ESB(16, 1);

@@ -123,24 +123,27 @@ int autotune_t(gsea_plan_s* p, int64_t n64, unsigned stages, gsea_tuning* best_o
     }
     // enrichment (on the last sort's output: identical for every variant)
     float ebest = 1e30f;
-    for (int w : {32, 24, 16, 8}) {
-        for (int stage : {1, 3, 2, 0}) {
-            if (!(stages & kEs)) break;
-            gsea::EsTuning et;
-            et.warps = w;
-            et.stage = stage;
-            const float ms = time_best(
-                [&]() {
-                    return gsea::launch_es<T>(p->ranks, p->ranks16, static_cast<const T*>(p->sorted), G, n,
-                                              gsea::plan_sets(p), p->set_order, static_cast<const T*>(p->decay), K,
-                                              static_cast<T*>(p->es), c.num_perms, 0, st, et);
-                },
-                st, t);
-            if (ms >= 0.f && ms < ebest) {
-                ebest = ms;
-                best.es_warps = w;
-                best.es_stage = stage;
-            }
+    std::vector<std::pair<int, int>> ec;
+    if (c.precision == 64) ec.emplace_back(0, -1);  // the automatic choice stages more than may be asked for
+    for (int w : {32, 24, 16, 8})
+        for (int stage : {1, 3, 2, 0}) ec.emplace_back(w, stage);
+    for (const auto& cand : ec) {
+        if (!(stages & kEs)) break;
+        const int w = cand.first, stage = cand.second;
+        gsea::EsTuning et;
+        et.warps = w;
+        et.stage = stage;
+        const float ms = time_best(
+            [&]() {
+                return gsea::launch_es<T>(p->ranks, p->ranks16, static_cast<const T*>(p->sorted), G, n,
+                                          gsea::plan_sets(p), p->set_order, static_cast<const T*>(p->decay), K,
+                                          static_cast<T*>(p->es), c.num_perms, 0, st, et);
+            },
+            st, t);
+        if (ms >= 0.f && ms < ebest) {
+            ebest = ms;
+            best.es_warps = w;
+            best.es_stage = stage;
         }
     }
     GSEA_CUDA(cudaStreamSynchronize(st), "stream sync");
