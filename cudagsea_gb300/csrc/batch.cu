@@ -18,7 +18,7 @@
 //      lane of the register procedure, fixed by G): its CTAs pull
 //      (instance, permutation) items from a global counter, heaviest
 //      instances first, so uneven instances keep every SM busy to the end;
-//   5. the statistics of every instance: one launch per step (nine), the
+//   5. the statistics of every instance: one launch per step (four), the
 //      instances whose FDR histogram does not fit shared memory on their own.
 // Every instance's results are those of its solo plan bit for bit.  The
 // first execute captures the stages into one CUDA graph; later executes

@@ -70,11 +70,15 @@ __device__ __forceinline__ void stats_set_kernel_body(int bx, const T* __restric
             if (b >= P) break;  // warp-uniform
             const T av = fabs(cur[j]);
             if (b + lane < P && av >= aes0) np++;
-            const int n = (int)(P - b < 32 ? P - b : 32);
-            // sequential sum in index order, as the reference's host loop
-            for (int i = 0; i < n; i++) {
-                const T x = __shfl_sync(kFullMask, av, i);
-                sum = Exact<T>::add(sum, x);
+            // sequential sum in index order, as the reference's host loop;
+            // unrolled, the shuffles run ahead of the chain of additions
+            // (50 sets x 1,024 columns 16.5 -> 8.5 us)
+            if (P - b >= 32) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) sum = Exact<T>::add(sum, __shfl_sync(kFullMask, av, i));
+            } else {
+                const int n = (int)(P - b);
+                for (int i = 0; i < n; i++) sum = Exact<T>::add(sum, __shfl_sync(kFullMask, av, i));
             }
         }
 #pragma unroll
@@ -292,20 +296,18 @@ stats_fdr_hist_kernel(const T* __restrict__ es, int K, int64_t ld, const int64_t
 // Dense form (every set has all ld columns, unit weights): block b bins an
 // equal contiguous share of the K x (ld - 1) null scores (row-major, column
 // 0 excluded) into shared-memory integer histograms of both sides, against
-// the sorted observed keys staged beside them, and writes them as row b of
-// `partial` (width 2(K+2) + 2: H_pos | H_neg | #null >= 0 | #null <= 0).
-// stats_fdr_hist_sum_kernel adds the rows up column by column: exact integer
-// counts, no global atomics, the same result in any order.
-constexpr int kDenseHistThreads = 512;
-constexpr size_t kDenseHistPartialBytes = size_t(1) << 20;
+// the sorted observed keys staged beside them, and adds its bins that are not
+// empty to the global ones: exact integer counts, the same in any order.
+constexpr int kDenseHistThreads = 1024;
 constexpr size_t kDenseHistSmemMax = 96 * 1024;
+constexpr int kDenseHistShare = 4096;  // scores of a block, at least
 template <class T>
 __device__ __forceinline__ void
-stats_fdr_hist_dense_kernel_body(int bx, int gx, const T* __restrict__ es, int K, int64_t ld, const T* __restrict__ fac,
-                            const T* __restrict__ sorted_pos, const T* __restrict__ sorted_neg,
-                            const unsigned long long* __restrict__ totals, unsigned* __restrict__ partial) {
+stats_fdr_hist_dense_body(int bx, int gx, const T* __restrict__ es, int K, int64_t ld, const T* __restrict__ fac,
+                          const T* __restrict__ sorted_pos, const T* __restrict__ sorted_neg,
+                          const unsigned long long* __restrict__ totals, unsigned long long* __restrict__ bins) {
     extern __shared__ __align__(16) unsigned char dense_smem[];
-    const int W = 2 * (K + 2) + 2;
+    const int W = 2 * (K + 2);
     unsigned* h = reinterpret_cast<unsigned*>(dense_smem);  // W counters
     T* s_pos = reinterpret_cast<T*>(dense_smem + (((size_t)W * 4 + 15) & ~(size_t)15));
     const unsigned npos = (unsigned)totals[2], nneg = (unsigned)totals[3];
@@ -317,7 +319,6 @@ stats_fdr_hist_dense_kernel_body(int bx, int gx, const T* __restrict__ es, int K
     const int64_t cols = ld - 1;
     const int64_t total = (int64_t)K * cols;
     const int64_t lo = total * bx / gx, hi = total * (bx + 1) / gx;
-    unsigned cpos = 0, cneg = 0;
     int64_t k = lo / cols;
     int64_t c = lo - k * cols;  // column - 1 within row k
     for (int64_t i = lo; i < hi;) {
@@ -326,44 +327,16 @@ stats_fdr_hist_dense_kernel_body(int bx, int gx, const T* __restrict__ es, int K
         const T* row = es + k * ld + 1 + c;
         for (int64_t j = threadIdx.x; j < run; j += kDenseHistThreads) {
             const T v = Exact<T>::mul(row[j], f);
-            if (v >= T(0)) {
-                cpos++;
-                atomicAdd(&h[upper_bound_t(s_pos, npos, v)], 1u);
-            }
-            if (v <= T(0)) {
-                cneg++;
-                atomicAdd(&h[(K + 2) + upper_bound_t(s_neg, nneg, -v)], 1u);
-            }
+            if (v >= T(0)) atomicAdd(&h[upper_bound_t(s_pos, npos, v)], 1u);
+            if (v <= T(0)) atomicAdd(&h[(K + 2) + upper_bound_t(s_neg, nneg, -v)], 1u);
         }
         i += run;
         k++;
         c = 0;
     }
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        cpos += __shfl_xor_sync(kFullMask, cpos, o);
-        cneg += __shfl_xor_sync(kFullMask, cneg, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (cpos) atomicAdd(&h[W - 2], cpos);
-        if (cneg) atomicAdd(&h[W - 1], cneg);
-    }
     __syncthreads();
-    unsigned* out = partial + (size_t)bx * W;
-    for (int i = threadIdx.x; i < W; i += kDenseHistThreads) out[i] = h[i];
-}
-
-// column sums of the partial histograms: H_pos, H_neg (contiguous, 2(K+2)
-// doubles) and the null counts per side (totals[4], [5] as doubles)
-__device__ __forceinline__ void stats_fdr_hist_sum_kernel_body(int bx, const unsigned* __restrict__ partial, int rows, int K,
-                                          double* __restrict__ hist, unsigned long long* __restrict__ totals) {
-    const int W = 2 * (K + 2) + 2;
-    const int j = bx * blockDim.x + threadIdx.x;
-    if (j >= W) return;
-    unsigned long long s = 0;
-    for (int r = 0; r < rows; r++) s += partial[(size_t)r * W + j];
-    if (j < W - 2) hist[j] = (double)s;
-    else reinterpret_cast<double*>(totals + 4)[j - (W - 2)] = (double)s;
+    for (int i = threadIdx.x; i < W; i += kDenseHistThreads)
+        if (h[i]) atomicAdd(&bins[i], (unsigned long long)h[i]);
 }
 
 template <class T>
@@ -371,14 +344,14 @@ size_t dense_hist_smem(int K) {
     const size_t W = 2 * ((size_t)K + 2) + 2;
     return ((W * 4 + 15) & ~(size_t)15) + 2 * sizeof(T) * (size_t)K;
 }
-// rows of the partial histograms (0: the dense form does not apply)
+// blocks of the dense histogram (0: the dense form does not apply): two to
+// an SM, fewer where a share would not pay for staging the observed keys
 template <class T>
-int dense_hist_rows(int K, int sms) {
+int dense_hist_blocks(int K, int64_t ld, int sms) {
     if (dense_hist_smem<T>(K) > kDenseHistSmemMax) return 0;
-    const size_t W = 2 * ((size_t)K + 2) + 2;
-    const size_t cap = kDenseHistPartialBytes / (4 * W);
-    const size_t want = 2 * (size_t)(sms > 0 ? sms : 1);
-    return (int)(cap < want ? cap : want);
+    const int64_t shares = ((int64_t)K * (ld - 1) + kDenseHistShare - 1) / kDenseHistShare;
+    const int64_t want = 2 * (int64_t)(sms > 0 ? sms : 1);
+    return (int)(shares < 1 ? 1 : shares < want ? shares : want);
 }
 
 // in-place suffix sums of the two histograms (one block each)
@@ -455,7 +428,7 @@ struct RaggedLayout {
     double* hpos;
     double* hneg;
     unsigned long long* totals;
-    unsigned* partial;
+    unsigned long long* bins;  // dense form: null scores per bin, 2(K+2)
     __host__ __device__ RaggedLayout(void* scratch, int K, int64_t p_fwer) {
         unsigned char* s = static_cast<unsigned char*>(scratch);
         auto align16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
@@ -472,7 +445,7 @@ struct RaggedLayout {
         hpos = reinterpret_cast<double*>(s + off);
         hneg = hpos + (K + 2);
         totals = reinterpret_cast<unsigned long long*>(hneg + (K + 2));
-        partial = reinterpret_cast<unsigned*>(s + align16(off + sizeof(double) * (2 * ((size_t)K + 2) + 8)));
+        bins = reinterpret_cast<unsigned long long*>(s + align16(off + sizeof(double) * (2 * ((size_t)K + 2) + 8)));
     }
 };
 
@@ -498,17 +471,6 @@ __global__ void stats_fdr_obs_kernel(int K, const T* __restrict__ out, unsigned 
                                      T* __restrict__ sorted_neg, unsigned long long* __restrict__ totals) {
     stats_fdr_obs_kernel_body<T>(blockIdx.x, K, out, cnt_obs, lcount, sorted_pos, sorted_neg, totals);
 }
-template <class T>
-__global__ void __launch_bounds__(kDenseHistThreads)
-stats_fdr_hist_dense_kernel(const T* __restrict__ es, int K, int64_t ld, const T* __restrict__ fac,
-                            const T* __restrict__ sorted_pos, const T* __restrict__ sorted_neg,
-                            const unsigned long long* __restrict__ totals, unsigned* __restrict__ partial) {
-    stats_fdr_hist_dense_kernel_body<T>(blockIdx.x, gridDim.x, es, K, ld, fac, sorted_pos, sorted_neg, totals, partial);
-}
-__global__ void stats_fdr_hist_sum_kernel(const unsigned* __restrict__ partial, int rows, int K,
-                                          double* __restrict__ hist, unsigned long long* __restrict__ totals) {
-    stats_fdr_hist_sum_kernel_body(blockIdx.x, partial, rows, K, hist, totals);
-}
 __global__ void stats_fdr_suffix_kernel(double* __restrict__ hpos, double* __restrict__ hneg,
                                         const unsigned long long* __restrict__ totals) {
     stats_fdr_suffix_kernel_body(blockIdx.x, hpos, hneg, totals);
@@ -521,72 +483,168 @@ __global__ void stats_fdr_final_kernel(int K, const unsigned long long* __restri
     stats_fdr_final_kernel_body<T>(blockIdx.x, K, cnt_obs, lcount, spos, sneg, totals, out);
 }
 
-// ---- the same kernels over many instances at once ----------------------------
-// blockIdx.z = the instance; every instance has all its columns (the dense
-// form); grids are sized for the largest instance and the blocks beyond an
-// instance's own extent return at once.  Each instance's results are those
-// of its solo run bit for bit: the same bodies, the same block decomposition.
+// ---- the dense form in four steps --------------------------------------------
+// Every set has all its columns.  Independent kernels of the list above share
+// a launch (blocks of different kinds), the buffers are cleared by the first:
+//   1. factors, NES, NP; histogram, totals and extrema cleared
+//   2. extrema per column; counts and order of the observed scores
+//   3. null histogram; FWER
+//   4. suffix sums and q
+// (Eight launches and three memsets before: 70 us at 50 sets x 1,024
+// permutations, most of it launches, one thread adding up 300 partial rows
+// and FP64 prefix sums; the counts are integers here.)
+struct DenseDims {
+    int K, rows;        // sets; blocks of the histogram
+    int64_t ld, p_fwer;
+    __host__ __device__ int set_blocks() const { return (K + 7) / 8; }
+    __host__ __device__ int64_t init() const { return p_fwer > 2 * (K + 2) + 8 ? p_fwer : 2 * (K + 2) + 8; }
+    __host__ __device__ int extrema_x() const { return (int)((p_fwer + 127) / 128); }
+    __host__ __device__ int64_t extrema_blocks() const {
+        return (int64_t)extrema_x() * ((K + kExtremaSets - 1) / kExtremaSets);
+    }
+    __host__ __device__ int64_t step2_blocks() const { return extrema_blocks() + (K + 3) / 4; }
+    __host__ __device__ int step3_blocks() const { return rows + (K + kDenseHistThreads / 32 - 1) / (kDenseHistThreads / 32); }
+};
+
 template <class T>
-__global__ void stats_init_multi(const StatsTask<T>* __restrict__ tasks) {
+__device__ __forceinline__ void dense_step1(int64_t bx, int64_t gx, const DenseDims& d, const T* es, T* out,
+                                            const RaggedLayout<T>& L) {
     using U = typename RadixKey<T>::U;
-    const StatsTask<T> t = tasks[blockIdx.z];
-    const RaggedLayout<T> L(t.scratch, t.K, t.P);
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 2 * ((int64_t)t.K + 2) + 8) L.hpos[i] = 0.0;  // H_pos | H_neg | totals
-    if (i < t.P) {
-        L.mx[i] = U(0);
-        L.mn[i] = ~U(0);
+    for (int64_t i = bx * blockDim.x + threadIdx.x; i < d.init(); i += gx * blockDim.x) {
+        if (i < 2 * (d.K + 2)) L.bins[i] = 0ull;
+        else if (i < 2 * (d.K + 2) + 8) L.totals[i - 2 * (d.K + 2)] = 0ull;
+        if (i < d.p_fwer) {
+            L.mx[i] = U(0);
+            L.mn[i] = ~U(0);
+        }
+    }
+    if (bx < d.set_blocks()) stats_set_kernel_body<T>((int)bx, es, d.K, d.ld, nullptr, out, L.fac);
+}
+template <class T>
+__device__ __forceinline__ void dense_step2(int64_t bx, const DenseDims& d, const T* es, const T* out,
+                                            const RaggedLayout<T>& L) {
+    const int64_t ext = d.extrema_blocks();
+    if (bx < ext) {
+        const int gx = d.extrema_x();
+        stats_extrema_kernel_body<T>((int)(bx % gx), (int)(bx / gx), es, d.K, d.ld, d.p_fwer, L.fac, L.mx, L.mn);
+    } else {
+        stats_fdr_obs_kernel_body<T>((int)(bx - ext), d.K, out, L.cnt_obs, L.lcount, L.sorted_pos, L.sorted_neg,
+                                     L.totals);
     }
 }
 template <class T>
-__global__ void stats_set_multi(const StatsTask<T>* __restrict__ tasks) {
-    const StatsTask<T> t = tasks[blockIdx.z];
-    const RaggedLayout<T> L(t.scratch, t.K, t.P);
-    stats_set_kernel_body<T>(blockIdx.x, t.es, t.K, t.P, nullptr, t.stats, L.fac);
+__device__ __forceinline__ void dense_step3(int bx, const DenseDims& d, const T* es, T* out,
+                                            const RaggedLayout<T>& L) {
+    if (bx < d.rows)
+        stats_fdr_hist_dense_body<T>(bx, d.rows, es, d.K, d.ld, L.fac, L.sorted_pos, L.sorted_neg, L.totals, L.bins);
+    else
+        stats_fwer_kernel_body<T>(bx - d.rows, d.K, d.p_fwer, L.mx, L.mn, out);
+}
+// q of kQSets sets on one side (0: positive, 1: negative).  Every block sums
+// the side's bins for itself, in shared memory: the quotients are what takes
+// time (four FP64 divisions a set; one block for 1,000 sets: 18 us), and a
+// warp to each quarter of the SM is as many as they keep busy.
+constexpr int kQSets = 128;
+template <class T>
+__device__ __forceinline__ void dense_step4(int bx, int side, const DenseDims& d, T* out, const RaggedLayout<T>& L) {
+    extern __shared__ __align__(16) unsigned long long above_bin[];  // [K + 2] scores in bin i or above
+    __shared__ unsigned long long carry, wsum[32];
+    const unsigned long long* const h = L.bins + side * (d.K + 2);
+    const int m = (int)L.totals[2 + side], n = m + 1;  // bins 0..m
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) carry = 0ull;
+    __syncthreads();
+    for (int top = n - 1; top >= 0; top -= (int)blockDim.x) {  // from the top bin down
+        const int i = top - (int)threadIdx.x;
+        unsigned long long v = i >= 0 ? h[i] : 0ull;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFullMask, v, o);
+            if (lane >= o) v += y;
+        }
+        if (lane == 31) wsum[warp] = v;
+        __syncthreads();
+        unsigned long long w = wsum[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFullMask, w, o);
+            if (lane >= o) w += y;
+        }
+        const unsigned long long before = warp > 0 ? __shfl_sync(kFullMask, w, (warp + 31) & 31) : 0ull;
+        const unsigned long long all = __shfl_sync(kFullMask, w, 31), c = carry;
+        if (i >= 0) above_bin[i] = v + before + c;
+        __syncthreads();
+        if (threadIdx.x == 0) carry = c + all;
+        __syncthreads();
+    }
+    const double null_side = (double)carry;
+    const int k = bx * kQSets + (int)threadIdx.x;
+    if (threadIdx.x >= kQSets || k >= d.K) return;
+    const T s = out[d.K + k];
+    const bool up = s > T(0);
+    if (!(s == s)) {
+        if (side == 0) out[4 * d.K + k] = s;
+    } else if (up == (side == 0)) {
+        const unsigned long long above = L.lcount[k] + 1;
+        const double c_null = above <= (unsigned long long)m ? (double)above_bin[above] : 0.0;
+        const double fn = null_side > 0 ? c_null / null_side : 0.0;
+        const double fo = (double)L.cnt_obs[k] / (double)m;
+        const double r = fn / fo;
+        out[4 * d.K + k] = (T)(r < 1.0 ? r : 1.0);
+    }
+}
+inline size_t dense_q_smem(int K) { return sizeof(unsigned long long) * ((size_t)K + 2); }
+
+template <class T>
+__global__ void __launch_bounds__(256) stats_dense1_kernel(DenseDims d, const T* es, T* out, RaggedLayout<T> L) {
+    dense_step1<T>(blockIdx.x, gridDim.x, d, es, out, L);
 }
 template <class T>
-__global__ void stats_extrema_multi(const StatsTask<T>* __restrict__ tasks) {
-    const StatsTask<T> t = tasks[blockIdx.z];
-    const RaggedLayout<T> L(t.scratch, t.K, t.P);
-    stats_extrema_kernel_body<T>(blockIdx.x, blockIdx.y, t.es, t.K, t.P, t.P, L.fac, L.mx, L.mn);
+__global__ void __launch_bounds__(128) stats_dense2_kernel(DenseDims d, const T* es, T* out, RaggedLayout<T> L) {
+    dense_step2<T>(blockIdx.x, d, es, out, L);
 }
 template <class T>
-__global__ void stats_fwer_multi(const StatsTask<T>* __restrict__ tasks) {
-    const StatsTask<T> t = tasks[blockIdx.z];
-    const RaggedLayout<T> L(t.scratch, t.K, t.P);
-    stats_fwer_kernel_body<T>(blockIdx.x, t.K, t.P, L.mx, L.mn, t.stats);
+__global__ void __launch_bounds__(kDenseHistThreads)
+stats_dense3_kernel(DenseDims d, const T* es, T* out, RaggedLayout<T> L) {
+    dense_step3<T>(blockIdx.x, d, es, out, L);
 }
 template <class T>
-__global__ void stats_fdr_obs_multi(const StatsTask<T>* __restrict__ tasks) {
+__global__ void __launch_bounds__(1024) stats_dense4_kernel(DenseDims d, T* out, RaggedLayout<T> L) {
+    dense_step4<T>(blockIdx.x, blockIdx.y, d, out, L);
+}
+
+// many instances at once: blockIdx.z = the instance; grids are sized for the
+// largest and the blocks beyond an instance's own extent return at once
+template <class T>
+__device__ __forceinline__ DenseDims dims_of(const StatsTask<T>& t) { return DenseDims{t.K, t.rows, t.P, t.P}; }
+template <class T>
+__global__ void __launch_bounds__(256) stats_dense1_multi(const StatsTask<T>* __restrict__ tasks) {
     const StatsTask<T> t = tasks[blockIdx.z];
     const RaggedLayout<T> L(t.scratch, t.K, t.P);
-    stats_fdr_obs_kernel_body<T>(blockIdx.x, t.K, t.stats, L.cnt_obs, L.lcount, L.sorted_pos, L.sorted_neg, L.totals);
+    dense_step1<T>(blockIdx.x, gridDim.x, dims_of(t), t.es, t.stats, L);
 }
 template <class T>
-__global__ void __launch_bounds__(kDenseHistThreads) stats_fdr_hist_dense_multi(const StatsTask<T>* __restrict__ tasks) {
+__global__ void __launch_bounds__(128) stats_dense2_multi(const StatsTask<T>* __restrict__ tasks) {
     const StatsTask<T> t = tasks[blockIdx.z];
-    if ((int)blockIdx.x >= t.rows) return;  // the whole block: before any barrier
+    const DenseDims d = dims_of(t);
+    if ((int64_t)blockIdx.x >= d.step2_blocks()) return;
     const RaggedLayout<T> L(t.scratch, t.K, t.P);
-    stats_fdr_hist_dense_kernel_body<T>(blockIdx.x, t.rows, t.es, t.K, t.P, L.fac, L.sorted_pos, L.sorted_neg,
-                                        L.totals, L.partial);
+    dense_step2<T>(blockIdx.x, d, t.es, t.stats, L);
 }
 template <class T>
-__global__ void stats_fdr_hist_sum_multi(const StatsTask<T>* __restrict__ tasks) {
+__global__ void __launch_bounds__(kDenseHistThreads) stats_dense3_multi(const StatsTask<T>* __restrict__ tasks) {
     const StatsTask<T> t = tasks[blockIdx.z];
+    const DenseDims d = dims_of(t);
+    if ((int)blockIdx.x >= d.step3_blocks()) return;  // the whole block: before any barrier
     const RaggedLayout<T> L(t.scratch, t.K, t.P);
-    stats_fdr_hist_sum_kernel_body(blockIdx.x, L.partial, t.rows, t.K, L.hpos, L.totals);
+    dense_step3<T>(blockIdx.x, d, t.es, t.stats, L);
 }
 template <class T>
-__global__ void stats_fdr_suffix_multi(const StatsTask<T>* __restrict__ tasks) {
+__global__ void __launch_bounds__(1024) stats_dense4_multi(const StatsTask<T>* __restrict__ tasks) {
     const StatsTask<T> t = tasks[blockIdx.z];
+    if ((int)blockIdx.x * kQSets >= t.K) return;  // the whole block: before any barrier
     const RaggedLayout<T> L(t.scratch, t.K, t.P);
-    stats_fdr_suffix_kernel_body(blockIdx.x, L.hpos, L.hneg, L.totals);
-}
-template <class T>
-__global__ void stats_fdr_final_multi(const StatsTask<T>* __restrict__ tasks) {
-    const StatsTask<T> t = tasks[blockIdx.z];
-    const RaggedLayout<T> L(t.scratch, t.K, t.P);
-    stats_fdr_final_kernel_body<T>(blockIdx.x, t.K, L.cnt_obs, L.lcount, L.hpos, L.hneg, L.totals, t.stats);
+    dense_step4<T>(blockIdx.x, blockIdx.y, dims_of(t), t.stats, L);
 }
 
 // Lower bound of every set's FDR q after the statistics (adaptive stopping):
@@ -673,10 +731,11 @@ template cudaError_t launch_fdr_bound<double>(int, int64_t, const double*, const
 
 template <class T>
 size_t stats_scratch_bytes(int K, int64_t P) {
-    // + the dense histograms' partial rows (at most kDenseHistPartialBytes)
+    // + room for the dense histogram (2(K+2) 64-bit bins; what its rows of
+    // partial counts once took, which callers of the C entry have allowed for)
     const size_t W = 2 * ((size_t)K + 2) + 2;
     const size_t dense = dense_hist_smem<T>(K) <= kDenseHistSmemMax
-                             ? (kDenseHistPartialBytes / (4 * W)) * 4 * W + 16 : 0;
+                             ? ((size_t(1) << 20) / (4 * W)) * 4 * W + 16 : 0;
     return StatsScratch::bytes(K, P, sizeof(T)) + 256 + dense;
 }
 template size_t stats_scratch_bytes<float>(int, int64_t);
@@ -689,6 +748,30 @@ cudaError_t launch_stats_ragged(const T* es, int K, int64_t ld, const int64_t* c
     if (K <= 0 || ld <= 0 || p_fwer <= 0 || p_fwer > ld) return K <= 0 ? cudaSuccess : cudaErrorInvalidValue;
     using U = typename RadixKey<T>::U;
     const RaggedLayout<T> L(scratch, K, p_fwer);
+    int dev = 0, max_smem = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (!counts && ld > 1 && hist_cols == ld) {
+        const DenseDims d{K, dense_hist_blocks<T>(K, ld, sms), ld, p_fwer};
+        if (d.rows > 0 && d.step2_blocks() <= INT32_MAX) {
+            const size_t smem = dense_hist_smem<T>(K);
+            cudaError_t e = cudaFuncSetAttribute(stats_dense3_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)smem);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(stats_dense4_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)dense_q_smem(K));
+            if (e != cudaSuccess) return e;
+            const int64_t clear = (d.init() + 255) / 256;  // blocks that clear, at most one to an SM more
+            const int b1 = d.set_blocks() > sms ? d.set_blocks() : (int)(clear < sms ? std::max<int64_t>(clear, d.set_blocks()) : sms);
+            stats_dense1_kernel<T><<<b1, 256, 0, st>>>(d, es, stats, L);
+            stats_dense2_kernel<T><<<(unsigned)d.step2_blocks(), 128, 0, st>>>(d, es, stats, L);
+            stats_dense3_kernel<T><<<d.step3_blocks(), kDenseHistThreads, smem, st>>>(d, es, stats, L);
+            stats_dense4_kernel<T><<<dim3((K + kQSets - 1) / kQSets, 2), 1024, dense_q_smem(K), st>>>(d, stats, L);
+            launches_add(4);
+            return cudaGetLastError();
+        }
+    }
     T* fac = L.fac;
     U* mx = L.mx;
     U* mn = L.mn;
@@ -699,7 +782,6 @@ cudaError_t launch_stats_ragged(const T* es, int K, int64_t ld, const int64_t* c
     double* hpos = L.hpos;
     double* hneg = L.hneg;
     unsigned long long* totals = L.totals;
-    unsigned* partial = L.partial;
     cudaError_t e = cudaMemsetAsync(hpos, 0, sizeof(double) * (2 * ((size_t)K + 2) + 8), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(mx, 0x00, sizeof(U) * (size_t)p_fwer, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(mn, 0xff, sizeof(U) * (size_t)p_fwer, st);
@@ -711,31 +793,11 @@ cudaError_t launch_stats_ragged(const T* es, int K, int64_t ld, const int64_t* c
     stats_fwer_kernel<T><<<(K + wpb - 1) / wpb, wpb * 32, 0, st>>>(K, p_fwer, mx, mn, stats);
     stats_fdr_obs_kernel<T><<<(K + wpb - 1) / wpb, wpb * 32, 0, st>>>(K, stats, cnt_obs, lcount, sorted_pos,
                                                                        sorted_neg, totals);
-    int rows = 0;
-    if (!counts && ld > 1 && hist_cols == ld) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        rows = dense_hist_rows<T>(K, sms);
-    }
-    if (rows > 0) {
-        const size_t smem = dense_hist_smem<T>(K);
-        e = cudaFuncSetAttribute(stats_fdr_hist_dense_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
-        if (e != cudaSuccess) return e;
-        stats_fdr_hist_dense_kernel<T><<<rows, kDenseHistThreads, smem, st>>>(es, K, ld, fac, sorted_pos, sorted_neg,
-                                                                            totals, partial);
-        const int W = 2 * (K + 2) + 2;
-        stats_fdr_hist_sum_kernel<<<(W + 255) / 256, 256, 0, st>>>(partial, rows, K, hpos, totals);
-    } else if (ld > 1) {
+    if (ld > 1) {
         // the sorted observed keys (at most 2K values) in shared memory: per
         // block (set x column chunk) when they fit the default 48 KB, else
         // once per resident 1,024-thread block looping over the sets
         const size_t obs_bytes = 2 * sizeof(T) * (size_t)K;
-        int dev = 0, max_smem = 0, sms = 1;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (obs_bytes > 48 * 1024 && obs_bytes + 1024 <= (size_t)max_smem) {
             auto kern = stats_fdr_hist_kernel<T, 1024>;
             e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)obs_bytes);
@@ -753,7 +815,7 @@ cudaError_t launch_stats_ragged(const T* es, int K, int64_t ld, const int64_t* c
     }
     stats_fdr_suffix_kernel<<<2, 1024, 0, st>>>(hpos, hneg, totals);
     stats_fdr_final_kernel<T><<<(K + 255) / 256, 256, 0, st>>>(K, cnt_obs, lcount, hpos, hneg, totals, stats);
-    launches_add(rows > 0 ? 8 : (ld > 1 ? 7 : 6));
+    launches_add(ld > 1 ? 7 : 6);
     return cudaGetLastError();
 }
 template cudaError_t launch_stats_ragged<float>(const float*, int, int64_t, const int64_t*, int64_t, float*, void*,
@@ -767,7 +829,7 @@ int stats_multi_rows(int K, int64_t P) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return dense_hist_rows<T>(K, sms);
+    return dense_hist_blocks<T>(K, P, sms);
 }
 template int stats_multi_rows<float>(int, int64_t);
 template int stats_multi_rows<double>(int, int64_t);
@@ -776,36 +838,32 @@ template <class T>
 cudaError_t launch_stats_multi(const StatsTask<T>* d_tasks, const StatsTask<T>* h_tasks, int n, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     if (n > 65535) return cudaErrorInvalidValue;
-    int Kmax = 0, rows = 0;
-    int64_t Pmax = 0, init = 0;
+    int b1 = 1, b3 = 1, Kmax = 1;
+    int64_t b2 = 1;
     size_t smem = 0;
     for (int i = 0; i < n; i++) {
         const StatsTask<T>& t = h_tasks[i];
         if (t.rows <= 0 || t.P < 2) return cudaErrorInvalidValue;  // the dense form only
-        Kmax = std::max(Kmax, t.K);
-        Pmax = std::max(Pmax, t.P);
-        rows = std::max(rows, t.rows);
-        init = std::max(init, std::max(2 * ((int64_t)t.K + 2) + 8, t.P));
+        const DenseDims d{t.K, t.rows, t.P, t.P};
+        b1 = std::max(b1, d.set_blocks());
+        b2 = std::max(b2, d.step2_blocks());
+        b3 = std::max(b3, d.step3_blocks());
         smem = std::max(smem, dense_hist_smem<T>(t.K));
+        Kmax = std::max(Kmax, t.K);
     }
+    if (b2 > INT32_MAX) return cudaErrorInvalidValue;
     const unsigned z = (unsigned)n;
-    const int wpb = 8;
-    const unsigned set_blocks = (unsigned)((Kmax + wpb - 1) / wpb);
-    stats_init_multi<T><<<dim3((unsigned)((init + 255) / 256), 1, z), 256, 0, st>>>(d_tasks);
-    stats_set_multi<T><<<dim3(set_blocks, 1, z), wpb * 32, 0, st>>>(d_tasks);
-    stats_extrema_multi<T><<<dim3((unsigned)((Pmax + 127) / 128), (unsigned)((Kmax + kExtremaSets - 1) / kExtremaSets), z),
-                             128, 0, st>>>(d_tasks);
-    stats_fwer_multi<T><<<dim3(set_blocks, 1, z), wpb * 32, 0, st>>>(d_tasks);
-    stats_fdr_obs_multi<T><<<dim3(set_blocks, 1, z), wpb * 32, 0, st>>>(d_tasks);
-    cudaError_t e = cudaFuncSetAttribute(stats_fdr_hist_dense_multi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(stats_dense3_multi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(stats_dense4_multi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)dense_q_smem(Kmax));
     if (e != cudaSuccess) return e;
-    stats_fdr_hist_dense_multi<T><<<dim3((unsigned)rows, 1, z), kDenseHistThreads, smem, st>>>(d_tasks);
-    const int Wmax = 2 * (Kmax + 2) + 2;
-    stats_fdr_hist_sum_multi<T><<<dim3((unsigned)((Wmax + 255) / 256), 1, z), 256, 0, st>>>(d_tasks);
-    stats_fdr_suffix_multi<T><<<dim3(2, 1, z), 1024, 0, st>>>(d_tasks);
-    stats_fdr_final_multi<T><<<dim3((unsigned)((Kmax + 255) / 256), 1, z), 256, 0, st>>>(d_tasks);
-    launches_add(9);
+    stats_dense1_multi<T><<<dim3((unsigned)b1, 1, z), 256, 0, st>>>(d_tasks);
+    stats_dense2_multi<T><<<dim3((unsigned)b2, 1, z), 128, 0, st>>>(d_tasks);
+    stats_dense3_multi<T><<<dim3((unsigned)b3, 1, z), kDenseHistThreads, smem, st>>>(d_tasks);
+    stats_dense4_multi<T><<<dim3((Kmax + kQSets - 1) / kQSets, 2, z), 1024, dense_q_smem(Kmax), st>>>(d_tasks);
+    launches_add(4);
     return cudaGetLastError();
 }
 template cudaError_t launch_stats_multi<float>(const StatsTask<float>*, const StatsTask<float>*, int, cudaStream_t);

@@ -191,8 +191,8 @@ cudaError_t launch_permute_multi(const PermTask* d_tasks, const PermTask* h_task
 // Statistics of many instances at once (batched form): one launch per step
 // over all instances (blockIdx.z = instance), each instance's results those
 // of its solo launch_stats bit for bit.  Dense form only: every instance has
-// P >= 2 columns and rows = stats_multi_rows<T>(K, P) > 0 (its FDR
-// histogram fits shared memory).
+// P >= 2 columns and rows = stats_multi_rows<T>(K, P) > 0 (blocks of its FDR
+// histogram, which fits shared memory).
 template <class T>
 struct StatsTask {
     const T* es;    // [K][P]
