@@ -57,6 +57,7 @@
 // the same magnitude: such a set, and one whose weights are not finite, takes
 // the procedure with positions (set_score_positions).
 #pragma once
+#include <algorithm>
 #include <climits>
 #include <type_traits>
 
@@ -795,10 +796,16 @@ __device__ __forceinline__ void es_smem_layout(unsigned char* smem, int G, int r
     bm = reinterpret_cast<uint32_t*>(smem + bm_off) + (size_t)warp * region;
 }
 
+// 16 warps with everything staged come as two CTAs to an SM (launch_es_t)
+template <class T, int WARPS, int STAGE>
+constexpr bool pairs_up() {
+    return sizeof(T) == 4 && WARPS == 16 && STAGE == 1;
+}
+
 // WPL > 0: bitmap words per lane held in registers by the list procedure
 // (G <= 1024*WPL, ranks < 65536); WPL == 0: general procedure only.
 template <class T, class RankT, int WARPS, int STAGE, int WPL>
-__global__ void __launch_bounds__(WARPS * 32)
+__global__ void __launch_bounds__(WARPS * 32, pairs_up<T, WARPS, STAGE>() ? 2 : 1)
 es_kernel(const RankT* __restrict__ ranks, const T* __restrict__ sorted_abs, int G, int num_perms,
           const EsSets sets, const int32_t* __restrict__ set_order, const T* __restrict__ decay, int K,
           T* __restrict__ es, int64_t es_stride, int64_t col0, const int* __restrict__ K_dev) {
@@ -924,17 +931,34 @@ inline bool es_fits(int warps, int stage, size_t smem, size_t asked, int wpl, si
     return !(leave_l1 && stage == 0 && smem > kLeavesL1);
 }
 
-// Shared memory for the CTA and as much L1 as that leaves: what is not staged
-// is gathered through L1.  Without the request an SM keeps the split of the
-// kernel that ran on it before, the sort's with hardly any L1, whenever passes
-// on several streams leave it no idle moment (passes of several plans in turn:
-// 60,000 genes 1,183 -> 948 us, 36,161 genes 1,554 -> 1,145; a single plan's
-// the same, all staged the same; all of it as shared memory 1,219 and 1,636).
-template <class K>
-cudaError_t es_shared_memory(K kern, size_t smem) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+// Launch with the shared memory of the resident CTAs and all the L1 that
+// leaves: what is not staged is gathered through L1.  Without the request an
+// SM keeps the split of the kernel that ran on it before, the sort's with
+// hardly any L1, whenever passes on several streams leave it no idle moment
+// (passes of several plans in turn: 60,000 genes 1,183 -> 948 us, 36,161 genes
+// 1,554 -> 1,145; a single plan's the same, all staged the same; all of it as
+// shared memory 1,219 and 1,636).
+template <class... P, class... A>
+cudaError_t launch_es_kernel(void (*kern)(P...), int grid, int warps, size_t smem, int per_sm, cudaStream_t st,
+                             A... args) {
+    int dev = 0, all = 0, reserved = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&all, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+    cudaLaunchAttribute l1;
+    l1.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    // per cent, rounded down: the split in use is the next larger one
+    l1.val.sharedMemCarveout =
+        (unsigned)std::min<size_t>(100, (size_t)per_sm * (smem + (size_t)reserved) * 100 / (size_t)std::max(all, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)warps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &l1;
+    cfg.numAttrs = 1;
+    launches_add(1);
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 template <class T, class RankT, int WARPS, int STAGE, int WPL>
@@ -943,17 +967,14 @@ cudaError_t launch_es_v(const RankT* ranks, const T* sorted_abs, int G, int P, c
                         int64_t col0, int grid, cudaStream_t st, const int* K_dev) {
     const size_t smem = es_smem_bytes<T, RankT, WARPS, STAGE>(G);
     auto kern = es_kernel<T, RankT, WARPS, STAGE, WPL>;
-    cudaError_t e = es_shared_memory(kern, smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;  // resident CTAs per SM: the grid fills the device once
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidValue;
-    grid *= per_sm;
-    kern<<<grid, WARPS * 32, smem, st>>>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0,
-                                         K_dev);
-    launches_add(1);
-    return cudaGetLastError();
+    return launch_es_kernel(kern, grid * per_sm, WARPS, smem, per_sm, st, ranks, sorted_abs, G, P, sets, order, decay,
+                            K, es, stride, col0, K_dev);
 }
 
 template <class T, class RankT, int WARPS, int STAGE>
@@ -1029,14 +1050,26 @@ cudaError_t launch_es_t(const RankT* ranks, const T* sorted_abs, int G, int P, c
                           {8, 1, es_smem_bytes<T, RankT, 8, 1>(G)},
                           {8, 0, es_smem_bytes<T, RankT, 8, 0>(G)}};
     const int wpl = es_wpl(G, sizeof(RankT) == 2);
+#define GSEA_ES(W, S) \
+    return launch_es_w<T, RankT, W, S>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, \
+                                       K_dev)
+    // Few sets to a permutation: two CTAs of 16 warps, of which one scores while
+    // the other stages its permutation or waits for its last sets.  50 sets x
+    // 1,024 permutations, 2,000 genes: 86 -> 82 us (passes in turn 128 -> 119),
+    // 12,000 genes 88 -> 82; 250 sets 287 -> 281, 300 sets 373 -> 373, 600 sets
+    // 367 -> 379.
+    if constexpr (pairs_up<T, 16, 1>()) {
+        int all = 0, reserved = 0;
+        cudaDeviceGetAttribute(&all, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+        const size_t pair = 2 * (es_smem_bytes<T, RankT, 16, 1>(G) + 64 + (size_t)reserved);
+        if (K <= 256 && !tune.warps && tune.stage < 0 && wpl < 40 && pair <= (size_t)all) GSEA_ES(16, 1);
+    }
     for (int pass = 0; pass < 2; pass++)
     for (const Cand& c : cands) {
         if (!es_fits(c.warps, c.stage, c.smem, (sizeof(T) - es_weight_bytes<T, RankT>()) * (size_t)G, wpl, cap,
                      pass == 0, tune))
             continue;
-#define GSEA_ES(W, S) \
-    return launch_es_w<T, RankT, W, S>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, \
-                                       K_dev)
         if (c.warps == 32 && c.stage == 1) GSEA_ES(32, 1);
         if (c.warps == 16 && c.stage == 1) GSEA_ES(16, 1);
         if (c.warps == 8 && c.stage == 1) GSEA_ES(8, 1);
@@ -1059,7 +1092,7 @@ cudaError_t launch_es_batch_v(const EsTask<T>* tasks, const int64_t* item_end, i
                               unsigned long long* counter, int Gmax, cudaStream_t st) {
     const size_t smem = es_smem_bytes<T, uint16_t, WARPS, STAGE>(Gmax);
     auto kern = es_batch_kernel<T, uint16_t, WARPS, STAGE, WPL>;
-    cudaError_t e = es_shared_memory(kern, smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 1, per_sm = 0;
     cudaGetDevice(&dev);
@@ -1071,9 +1104,7 @@ cudaError_t launch_es_batch_v(const EsTask<T>* tasks, const int64_t* item_end, i
     const int grid = (int)(nitems < want ? nitems : want);
     e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    kern<<<grid, WARPS * 32, smem, st>>>(tasks, item_end, ntasks, nitems, counter, Gmax);
-    launches_add(1);
-    return cudaGetLastError();
+    return launch_es_kernel(kern, grid, WARPS, smem, per_sm, st, tasks, item_end, ntasks, nitems, counter, Gmax);
 }
 
 template <class T, int WARPS, int STAGE>
