@@ -46,7 +46,10 @@ struct gsea_plan_s {
     int64_t nA = 0, nB = 0;
     int64_t nnz = 0, nnz_cap = 0;
     int64_t last_launches = 0;
-    // device buffers
+    // device buffers; those of plan creation are parts of one allocation, the
+    // others (sets beyond it, debug, adaptive test) have their own
+    void* arena = nullptr;
+    bool own_sets = false;             // set_genes and set_list are not parts of the arena
     void* exprs = nullptr;
     uint8_t* labels = nullptr;
     int64_t* set_off = nullptr;
