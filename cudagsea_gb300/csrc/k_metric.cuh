@@ -169,6 +169,10 @@ constexpr int metric_blocks() {
     return sizeof(T) == 8 ? 2 : ACC == ACC_OVERKILL || ACC == ACC_KNUTH ? 3 : 4;
 }
 constexpr int kChunk = 32;
+// class bits of a warp: a byte per sample, the chunks kPatStep bytes apart;
+// behind a chunk's last pair kEnd (an odd last sample's bits follow it)
+constexpr int kPatStep = kChunk + 2, kEnd = 16;
+constexpr int pat_bytes(int S) { return (S + kChunk - 1) / kChunk * kPatStep; }
 
 template <int ACC, class T>
 constexpr int metric_vecs() { return sizeof(T) == 8 ? 1 : 2; }  // vectors per lane
@@ -176,7 +180,7 @@ template <int ACC, class T>
 constexpr int metric_genes() { return 32 * metric_vecs<ACC, T>() * Vec<T>::kLanes; }  // genes of a tile
 template <int ACC, class T>
 constexpr size_t metric_smem(int warps, int S) {
-    return sizeof(T) * metric_genes<ACC, T>() * (2 * kChunk + (size_t)warps) + (size_t)warps * S;
+    return sizeof(T) * metric_genes<ACC, T>() * (2 * kChunk + (size_t)warps) + (size_t)warps * pat_bytes(S);
 }
 
 // one copy of BYTES (4, 8, 16), both addresses aligned to it
@@ -191,10 +195,13 @@ __device__ __forceinline__ void async_copy(uint32_t dst, const void* src) {
 // samples, two permutations) to one of sixteen cases, each updating its
 // accumulators in place.  In assembly, loop and all, because the compiler
 // copies every accumulator where the cases meet (written as a C++ switch: 55
-// instructions for what takes 24).  The branch has a long latency: two
-// vectors a lane (128 genes a warp) leave registers for 32 warps an SM, which
-// hide it better than four vectors and 20 warps (20,000 genes x 200 samples x
-// 1,000 permutations 912 against 980 us, 2,000 x 40 x 1,024 43 against 54).
+// instructions for what takes 24).  The cases never meet: each loads the next
+// bits and branches on them itself, so that a pair costs 8 instructions besides
+// its statistics and not 12 (20,000 genes x 200 samples x 1,000 permutations
+// 944 -> 832 us).  The branch has a long latency: two vectors a lane (128 genes
+// a warp) leave registers for 32 warps an SM, which hide it better than four
+// vectors and 20 warps (2,000 genes x 40 samples x 1,024 43 against 54 us when
+// the cases still met).
 // Operand numbers: statistics of class, permutation and vector M_ 0-7, W_
 // 8-15, U_ 16-23; X_ the loaded vector of a sample.
 #define GM_0A0(OP) OP(0, 8, 16, 0) OP(1, 9, 17, 1)
@@ -205,59 +212,59 @@ __device__ __forceinline__ void async_copy(uint32_t dst, const void* src) {
 #define GM_1A1(OP) OP(2, 10, 18, 2) OP(3, 11, 19, 3)
 #define GM_1B0(OP) OP(4, 12, 20, 2) OP(5, 13, 21, 3)
 #define GM_1B1(OP) OP(6, 14, 22, 2) OP(7, 15, 23, 3)
-#define GM_CASE(N, P0, P1, P2, P3) "C" #N ":\n" P0 P1 P2 P3 "bra.uni NEXT;\n"
+#define GM_AHEAD(PP, XP)                                                                                          \
+    GM_LOAD(XP, 0, 0, 1) GM_LOAD(XP, 512, 2, 3) "ld.shared.u8 bits, [%" #PP "+2];\n"                              \
+    "add.u32 %" #PP ", %" #PP ", 2;\n add.u32 %" #XP ", %" #XP ", 1024;\n"
+#define GM_CASE(PP, XP, N, P0, P1, P2, P3) "C" #N ":\n" GM_AHEAD(PP, XP) P0 P1 P2 P3 "brx.idx.uni bits, TS;\n"
+#define GM_CASE1(N, P0, P1) "C" #N ":\n" P0 P1 "bra.uni NEXT;\n"
 #define GM_LOAD(XP, AT, A, B) "ld.shared.v2.b64 {x" #A ", x" #B "}, [%" #XP "+" #AT "];\n"
 // rows of 128 genes: 512 bytes
-// operands PP, XP, N: addresses of the class bits and of the lane's vectors, pairs of samples
-#define GM_LOOP(OP, PP, XP, N)                                                                                \
-    "{\n .reg .b64 d, e, x0, x1, x2, x3;\n .reg .u32 bits;\n .reg .pred more;\n"                    \
-    " TS: .branchtargets C0, C1, C2, C3, C4, C5, C6, C7, C8, C9, C10, C11, C12, C13, C14, C15;\n"               \
-    "LOOP: ld.shared.u8 bits, [%" #PP "];\n" GM_LOAD(XP, 0, 0, 1) GM_LOAD(XP, 512, 2, 3)                          \
-    " add.u32 %" #PP ", %" #PP ", 2;\n add.u32 %" #XP ", %" #XP ", 1024;\n sub.u32 %" #N ", %" #N ", 1;\n" \
-    " brx.idx.uni bits, TS;\n"                                                                                   \
-    GM_CASE(0, GM_0B0(OP), GM_0B1(OP), GM_1B0(OP), GM_1B1(OP)) \
-    GM_CASE(1, GM_0A0(OP), GM_0B1(OP), GM_1B0(OP), GM_1B1(OP)) \
-    GM_CASE(2, GM_0B0(OP), GM_0A1(OP), GM_1B0(OP), GM_1B1(OP)) \
-    GM_CASE(3, GM_0A0(OP), GM_0A1(OP), GM_1B0(OP), GM_1B1(OP)) \
-    GM_CASE(4, GM_0B0(OP), GM_0B1(OP), GM_1A0(OP), GM_1B1(OP)) \
-    GM_CASE(5, GM_0A0(OP), GM_0B1(OP), GM_1A0(OP), GM_1B1(OP)) \
-    GM_CASE(6, GM_0B0(OP), GM_0A1(OP), GM_1A0(OP), GM_1B1(OP)) \
-    GM_CASE(7, GM_0A0(OP), GM_0A1(OP), GM_1A0(OP), GM_1B1(OP)) \
-    GM_CASE(8, GM_0B0(OP), GM_0B1(OP), GM_1B0(OP), GM_1A1(OP)) \
-    GM_CASE(9, GM_0A0(OP), GM_0B1(OP), GM_1B0(OP), GM_1A1(OP)) \
-    GM_CASE(10, GM_0B0(OP), GM_0A1(OP), GM_1B0(OP), GM_1A1(OP)) \
-    GM_CASE(11, GM_0A0(OP), GM_0A1(OP), GM_1B0(OP), GM_1A1(OP)) \
-    GM_CASE(12, GM_0B0(OP), GM_0B1(OP), GM_1A0(OP), GM_1A1(OP)) \
-    GM_CASE(13, GM_0A0(OP), GM_0B1(OP), GM_1A0(OP), GM_1A1(OP)) \
-    GM_CASE(14, GM_0B0(OP), GM_0A1(OP), GM_1A0(OP), GM_1A1(OP)) \
-    GM_CASE(15, GM_0A0(OP), GM_0A1(OP), GM_1A0(OP), GM_1A1(OP)) \
-    "NEXT: setp.ne.u32 more, %" #N ", 0;\n @more bra.uni LOOP;\n}\n"
+// operands PP, XP: addresses of the class bits and of the lane's vectors; every
+// case loads its samples and the next pair's bits, and branches on those; the
+// bits end with kEnd
+#define GM_LOOP(OP, PP, XP)                                                                                       \
+    "{\n .reg .b64 d, e, x0, x1, x2, x3;\n .reg .u32 bits;\n"                                                    \
+    " TS: .branchtargets C0, C1, C2, C3, C4, C5, C6, C7, C8, C9, C10, C11, C12, C13, C14, C15, OUT;\n"           \
+    " ld.shared.u8 bits, [%" #PP "];\n brx.idx.uni bits, TS;\n"                                                  \
+    GM_CASE(PP, XP, 0, GM_0B0(OP), GM_0B1(OP), GM_1B0(OP), GM_1B1(OP)) \
+    GM_CASE(PP, XP, 1, GM_0A0(OP), GM_0B1(OP), GM_1B0(OP), GM_1B1(OP)) \
+    GM_CASE(PP, XP, 2, GM_0B0(OP), GM_0A1(OP), GM_1B0(OP), GM_1B1(OP)) \
+    GM_CASE(PP, XP, 3, GM_0A0(OP), GM_0A1(OP), GM_1B0(OP), GM_1B1(OP)) \
+    GM_CASE(PP, XP, 4, GM_0B0(OP), GM_0B1(OP), GM_1A0(OP), GM_1B1(OP)) \
+    GM_CASE(PP, XP, 5, GM_0A0(OP), GM_0B1(OP), GM_1A0(OP), GM_1B1(OP)) \
+    GM_CASE(PP, XP, 6, GM_0B0(OP), GM_0A1(OP), GM_1A0(OP), GM_1B1(OP)) \
+    GM_CASE(PP, XP, 7, GM_0A0(OP), GM_0A1(OP), GM_1A0(OP), GM_1B1(OP)) \
+    GM_CASE(PP, XP, 8, GM_0B0(OP), GM_0B1(OP), GM_1B0(OP), GM_1A1(OP)) \
+    GM_CASE(PP, XP, 9, GM_0A0(OP), GM_0B1(OP), GM_1B0(OP), GM_1A1(OP)) \
+    GM_CASE(PP, XP, 10, GM_0B0(OP), GM_0A1(OP), GM_1B0(OP), GM_1A1(OP)) \
+    GM_CASE(PP, XP, 11, GM_0A0(OP), GM_0A1(OP), GM_1B0(OP), GM_1A1(OP)) \
+    GM_CASE(PP, XP, 12, GM_0B0(OP), GM_0B1(OP), GM_1A0(OP), GM_1A1(OP)) \
+    GM_CASE(PP, XP, 13, GM_0A0(OP), GM_0B1(OP), GM_1A0(OP), GM_1A1(OP)) \
+    GM_CASE(PP, XP, 14, GM_0B0(OP), GM_0A1(OP), GM_1A0(OP), GM_1A1(OP)) \
+    GM_CASE(PP, XP, 15, GM_0A0(OP), GM_0A1(OP), GM_1A0(OP), GM_1A1(OP)) \
+    "OUT:\n}\n"
 // the last sample of an odd number
-#define GM_ONE(OP, PP, XP, N)                                                                                 \
-    "{\n .reg .b64 d, e, x0, x1, x2, x3;\n .reg .u32 bits;\n"                                      \
-    " TS: .branchtargets C0, C1, C2, C3;\n"                                                                      \
-    " ld.shared.u8 bits, [%" #PP "];\n and.b32 bits, bits, 3;\n" GM_LOAD(XP, 0, 0, 1) " brx.idx.uni bits, TS;\n"           \
-    GM_CASE(0, GM_0B0(OP), GM_0B1(OP), "", "") \
-    GM_CASE(1, GM_0A0(OP), GM_0B1(OP), "", "") \
-    GM_CASE(2, GM_0B0(OP), GM_0A1(OP), "", "") \
-    GM_CASE(3, GM_0A0(OP), GM_0A1(OP), "", "") \
-    "NEXT:\n}\n"
+#define GM_ONE(OP, PP, XP)                                                                                        \
+    "{\n .reg .b64 d, e, x0, x1;\n .reg .u32 bits;\n TS: .branchtargets C0, C1, C2, C3;\n"                        \
+    " ld.shared.u8 bits, [%" #PP "];\n and.b32 bits, bits, 3;\n" GM_LOAD(XP, 0, 0, 1) " brx.idx.uni bits, TS;\n"  \
+    GM_CASE1(0, GM_0B0(OP), GM_0B1(OP)) GM_CASE1(1, GM_0A0(OP), GM_0B1(OP))                                        \
+    GM_CASE1(2, GM_0B0(OP), GM_0A1(OP)) GM_CASE1(3, GM_0A0(OP), GM_0A1(OP)) "NEXT:\n}\n"
 // x added to the sum
 #define GM_SUM(M_, W_, U_, X_) "add.rn.f32x2 %" #M_ ", %" #M_ ", x" #X_ ";\n"
-// ... and x^2 to the sum of squares; one: 19
+// ... and x^2 to the sum of squares; one: 18
 #define GM_ONEPASS(M_, W_, U_, X_)                                                        \
-    GM_SUM(M_, W_, U_, X_) "mul.rn.f32x2 d, x" #X_ ", x" #X_ ";\n fma.rn.f32x2 %" #W_ ", %19, d, %" #W_ ";\n"
+    GM_SUM(M_, W_, U_, X_) "mul.rn.f32x2 d, x" #X_ ", x" #X_ ";\n fma.rn.f32x2 %" #W_ ", %18, d, %" #W_ ";\n"
 // Kahan step: W_ the compensation
 #define GM_KAHAN(M_, W_, U_, X_)                                                                     \
     "sub.rn.f32x2 d, x" #X_ ", %" #W_ ";\n add.rn.f32x2 e, %" #M_ ", d;\n"                          \
     "sub.rn.f32x2 %" #W_ ", e, %" #M_ ";\n sub.rn.f32x2 %" #W_ ", %" #W_ ", d;\n mov.b64 %" #M_ ", e;\n"
-// squared deviation from the mean M_ added to W_; one: 19
+// squared deviation from the mean M_ added to W_; one: 18
 #define GM_DEV(M_, W_, U_, X_) \
-    "sub.rn.f32x2 d, x" #X_ ", %" #M_ ";\n mul.rn.f32x2 d, d, d;\n fma.rn.f32x2 %" #W_ ", %19, d, %" #W_ ";\n"
-// ... and the deviation itself to W_, the square to U_; one: 27
+    "sub.rn.f32x2 d, x" #X_ ", %" #M_ ";\n mul.rn.f32x2 d, d, d;\n fma.rn.f32x2 %" #W_ ", %18, d, %" #W_ ";\n"
+// ... and the deviation itself to W_, the square to U_; one: 26
 #define GM_DEV2(M_, W_, U_, X_)                                                                \
     "sub.rn.f32x2 d, x" #X_ ", %" #M_ ";\n add.rn.f32x2 %" #W_ ", %" #W_ ", d;\n"             \
-    "mul.rn.f32x2 d, d, d;\n fma.rn.f32x2 %" #U_ ", %27, d, %" #U_ ";\n"
+    "mul.rn.f32x2 d, d, d;\n fma.rn.f32x2 %" #U_ ", %26, d, %" #U_ ";\n"
 // a statistic's registers, class by class, permutation by permutation
 #define GM_RW(A) "+l"(A[0][0][0]), "+l"(A[0][0][1]), "+l"(A[0][1][0]), "+l"(A[0][1][1]), "+l"(A[1][0][0]),      \
     "+l"(A[1][0][1]), "+l"(A[1][1][0]), "+l"(A[1][1][1])
@@ -350,26 +357,26 @@ struct Stats {
     // whether two samples are taken by one assembly block
     template <int MODE>
     static constexpr bool paired() { return sizeof(T) == 4 && ACC != ACC_KNUTH && MODE != WALK_STRICT; }
-    // `pairs` pairs of samples (COUNT = 2) or one sample (COUNT = 1) from the
-    // shared-memory addresses of their class bits and of the lane's vectors.
+    // the pairs of samples of a chunk (COUNT = 2) or one sample (COUNT = 1) from
+    // the shared-memory addresses of their class bits and of the lane's vectors.
     // The bits are the same in every lane: one branch, no divergence.
     template <int MODE, int COUNT>
-    __device__ __forceinline__ void samples(uint32_t pp, uint32_t xp, uint32_t pairs) {
-#define GM_RUN(OP, PP, XP, N, ...)                                                                                \
+    __device__ __forceinline__ void samples(uint32_t pp, uint32_t xp) {
+#define GM_RUN(OP, PP, XP, ...)                                                                                   \
     if constexpr (COUNT == 2)                                                                                     \
-        asm volatile(GM_LOOP(OP, PP, XP, N) : __VA_ARGS__, "+r"(pp), "+r"(xp), "+r"(pairs) : "l"(one) : "memory"); \
+        asm volatile(GM_LOOP(OP, PP, XP) : __VA_ARGS__, "+r"(pp), "+r"(xp) : "l"(one) : "memory");                \
     else                                                                                                          \
-        asm volatile(GM_ONE(OP, PP, XP, N) : __VA_ARGS__, "+r"(pp), "+r"(xp), "+r"(pairs) : "l"(one) : "memory");
+        asm volatile(GM_ONE(OP, PP, XP) : __VA_ARGS__, "+r"(pp), "+r"(xp) : "l"(one) : "memory");
         if constexpr (MODE == WALK_SUMS && (ACC == ACC_NAIVE || ACC == ACC_TWOPASS)) {
-            GM_RUN(GM_SUM, 8, 9, 10, GM_RW(m))
+            GM_RUN(GM_SUM, 8, 9, GM_RW(m))
         } else if constexpr (ACC == ACC_ONEPASS) {
-            GM_RUN(GM_ONEPASS, 16, 17, 18, GM_RW(m), GM_RW(var))
+            GM_RUN(GM_ONEPASS, 16, 17, GM_RW(m), GM_RW(var))
         } else if constexpr (ACC == ACC_KAHAN || (ACC == ACC_OVERKILL && MODE == WALK_SUMS)) {
-            GM_RUN(GM_KAHAN, 16, 17, 18, GM_RW(m), GM_RW(q))
+            GM_RUN(GM_KAHAN, 16, 17, GM_RW(m), GM_RW(q))
         } else if constexpr (ACC == ACC_TWOPASS) {
-            GM_RUN(GM_DEV, 16, 17, 18, GM_RW(m), GM_RW(var))
+            GM_RUN(GM_DEV, 16, 17, GM_RW(m), GM_RW(var))
         } else if constexpr (ACC == ACC_OVERKILL) {
-            GM_RUN(GM_DEV2, 24, 25, 26, GM_RW(m), GM_RW(q), GM_RW(var))
+            GM_RUN(GM_DEV2, 24, 25, GM_RW(m), GM_RW(q), GM_RW(var))
         }
 #undef GM_RUN
     }
@@ -424,15 +431,29 @@ struct Tile {
         const int s0 = c * kChunk, n = min(kChunk, S - s0);
         T* const to = tile + (c & 1) * kChunk * GW;
         const T* const from = X + (int64_t)s0 * G;
+        // rows by warps, so that a step is one addition to either address (15,013
+        // genes, copied four bytes at a time: 435 -> 377 us for the whole kernel,
+        // 20,000 genes 832 -> 815)
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
         if (wide) {
-            for (int i = threadIdx.x; i < n * (GW / PER); i += blockDim.x) {
-                const int r = i / (GW / PER), q = (i % (GW / PER)) * PER;
-                async_copy<16>(smem_u32(to + r * GW + q), from + (int64_t)r * G + q);
+            constexpr int PIECES = GW / PER, ROWS = 32 / PIECES;  // 16-byte pieces of a row, rows of a warp's copy
+            const int r0 = warp * ROWS + lane / PIECES, q = lane % PIECES * PER;
+            const T* src = from + (int64_t)r0 * G + q;
+            uint32_t dst = smem_u32(to + r0 * GW + q);
+            for (int r = r0; r < n; r += warps * ROWS) {
+                async_copy<16>(dst, src);
+                src += (int64_t)warps * ROWS * G;
+                dst += (uint32_t)(warps * ROWS * GW * (int)sizeof(T));
             }
         } else {
-            for (int i = threadIdx.x; i < n * GW; i += blockDim.x) {
-                const int r = i / GW, q = i % GW;
-                if (q < gn) async_copy<(int)sizeof(T)>(smem_u32(to + r * GW + q), from + (int64_t)r * G + q);
+            const T* src = from + (int64_t)warp * G + lane;
+            uint32_t dst = smem_u32(to + warp * GW + lane);
+            for (int r = warp; r < n; r += warps) {
+#pragma unroll
+                for (int i = 0; i < GW / 32; i++)
+                    if (lane + 32 * i < gn) async_copy<(int)sizeof(T)>(dst + 32u * i * (uint32_t)sizeof(T), src + 32 * i);
+                src += (int64_t)warps * G;
+                dst += (uint32_t)(warps * GW * (int)sizeof(T));
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -465,6 +486,7 @@ struct Tile {
             if (mine) {
                 const int s0 = c * kChunk, n = min(kChunk, S - s0);
                 const V* const row = reinterpret_cast<const V*>(tile + (c & 1) * kChunk * GW) + lane * NV;
+                const uint8_t* const bits = pat + c * kPatStep;
                 auto get = [&](int t, V* x) {
                     if constexpr (NV == 2) {
                         const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(row + t * (GW / L));
@@ -475,16 +497,17 @@ struct Tile {
                     }
                 };
                 if constexpr (S_::template paired<MODE>()) {
-                    const uint32_t pp = smem_u32(pat + s0), xp = smem_u32(row);
+                    const uint32_t pp = smem_u32(bits), xp = smem_u32(row);
                     static_assert(GW * sizeof(T) == 512, "the loop's row stride");
-                    if (n > 1) st.template samples<MODE, 2>(pp, xp, n >> 1);
-                    if (n & 1) st.template samples<MODE, 1>(pp + n - 1, xp + (n - 1) * GW * (int)sizeof(T), 0u);
+                    st.template samples<MODE, 2>(pp, xp);
+                    if (n & 1) st.template samples<MODE, 1>(pp + n, xp + (n - 1) * GW * (int)sizeof(T));
                 } else {
 #pragma unroll 1
                     for (int t = 0; t < n; t++) {
                         V x[NV];
                         get(t, x);
-                        st.template sample<MODE>(sizeof(T) == 4 ? pat[s0 + t] & 3 : pat[s0 + t], x);
+                        const int b = bits[sizeof(T) == 4 && t == n - 1 ? t + (n & 1) : t];
+                        st.template sample<MODE>(sizeof(T) == 4 ? b & 3 : b, x);
                     }
                 }
             }
@@ -512,7 +535,7 @@ __device__ __forceinline__ void metric_block(const T* __restrict__ X, int G, int
     T* const tile = reinterpret_cast<T*>(smem);                 // [2][kChunk][GW]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     T* const out = tile + 2 * kChunk * GW + warp * GW;          // [warps][GW]
-    uint8_t* const pat = reinterpret_cast<uint8_t*>(tile + (2 * kChunk + warps) * GW) + warp * S;  // [warps][S]
+    uint8_t* const pat = reinterpret_cast<uint8_t*>(tile + (2 * kChunk + warps) * GW) + warp * pat_bytes(S);  // [warps]
     const int g0 = gt * GW;
     const int gn = min(GW, G - g0);  // genes of the tile
     const bool wide = gn == GW && (G % (16 / (int)sizeof(T))) == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
@@ -532,7 +555,10 @@ __device__ __forceinline__ void metric_block(const T* __restrict__ X, int G, int
                     b |= ((mw[j] >> lane) & 1u) << j;
                 }
                 if (sizeof(T) == 4) b |= __shfl_down_sync(kFullMask, b, 1) << kQ;  // pairs start at even samples
-                if (w * 32 + lane < S) pat[w * 32 + lane] = (uint8_t)b;
+                const int n = min(kChunk, S - w * 32);
+                uint8_t* const to = pat + w * kPatStep;
+                if (sizeof(T) == 4 && lane == 0) to[n & ~1] = kEnd;
+                if (lane < n) to[sizeof(T) == 4 && lane == n - 1 ? lane + (n & 1) : lane] = (uint8_t)b;
             }
         }
         __syncwarp();
