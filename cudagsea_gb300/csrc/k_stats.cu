@@ -272,10 +272,13 @@ struct ObservedKeys {
     }
     static __device__ __forceinline__ float fill(unsigned short* t, const T* a, unsigned n) {
         const float scale = n ? (float)kSlots / (float)a[n - 1] : 0.f;
-        for (unsigned i = threadIdx.x; i <= n; i += blockDim.x) {  // key i fills the slots from its predecessor's on
-            const unsigned from = i > 0 ? slot(a[i - 1], scale) + 1 : 0u;
-            const unsigned to = i < n ? slot(a[i], scale) : kSlots;
-            for (unsigned q = from; q <= to; q++) t[q] = (unsigned short)i;
+        for (unsigned q = threadIdx.x; q <= kSlots; q += blockDim.x) {  // keys whose slot is lower
+            unsigned lo = 0, hi = n;
+            while (lo < hi) {
+                const unsigned mid = (lo + hi) >> 1;
+                if (slot(a[mid], scale) < q) lo = mid + 1; else hi = mid;
+            }
+            t[q] = (unsigned short)lo;
         }
         return scale;
     }
@@ -393,7 +396,7 @@ stats_fdr_hist_kernel(const T* __restrict__ es, int K, int64_t ld, const int64_t
 // empty to the global ones: exact integer counts, the same in any order.
 constexpr int kDenseHistThreads = 1024;
 constexpr size_t kDenseHistSmemMax = 96 * 1024;
-constexpr int kDenseHistShare = 4096;  // scores of a block, at least
+constexpr int kDenseHistShare = 1024;  // scores of a block, at least: one a thread
 template <class T>
 __device__ __forceinline__ void
 stats_fdr_hist_dense_body(int bx, int gx, const T* __restrict__ es, int K, int64_t ld, const T* __restrict__ fac,

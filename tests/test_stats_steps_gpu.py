@@ -1,6 +1,6 @@
 """The statistics in four steps (k_stats.cu, dense form) at the edges of their
 blocks: a set to a warp (8 and 4 to a block), 128 columns and 16 sets to an
-extrema block, the histogram's shares of 4,096 scores, 1,024 bins to a suffix
+extrema block, the histogram's shares of 1,024 scores, 1,024 bins to a suffix
 round, and the last collection that the dense form takes with the next one.
 Bit for bit the oracle's, with ties, zeros, a set of zeros and NaN."""
 import ctypes
