@@ -263,10 +263,10 @@ def peaks():
 
 # the stage's kernel profile and what bounds it (read off that profile)
 STAGE_PROFILES = {"es": ("es_kernel_full_20000x200_K1000_152perms.md", "instruction issue"),
-                  "sort": ("sort_regs_kernel_full_20000x200_152perms.md", "latency (barriers, ballots)"),
+                  "sort": ("sort_bucket_kernel_full_20000x200_152perms.md", "instruction issue, barriers"),
                   ("metric", "chosen"): ("class_stats_persistent_full_20000x200_152perms.md",
                                          "latency (epilogue)"),
-                  ("metric", "plain"): ("metric_fast_kernel_full_20000x200_152perms.md", "latency (L2 loads)")}
+                  ("metric", "plain"): ("metric_kernel_full_20000x200_152perms.md", "FP32 issue (paired instructions)")}
 
 
 def issue_limiter(stage, form):

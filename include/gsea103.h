@@ -275,7 +275,8 @@ int gsea_stats_device_noalloc(const void* es, int64_t num_sets, int64_t num_perm
  *      Every setting computes identical results; only the speed differs.
  *      0 / -1 leave a choice automatic.                                    */
 typedef struct gsea_tuning {
-    int32_t metric_pb;    /* plain metric: permutations a warp takes, 4 or 8 (in two rounds) */
+    int32_t metric_pb;    /* plain metric: 4: a warp takes one group of permutations (two in fp32, four in
+                             fp64), 8: two groups in turn */
     int32_t chosen_tile;  /* tensor-core form: permutations per tile, 128 (the automatic choice: one
                              persistent CTA per SM walking the tiles, the copies, MMAs and
                              epilogue on separate warps) or 256 (one tile per CTA) */
@@ -311,16 +312,16 @@ int gsea_plan_autotune(gsea_plan plan, int64_t sample_perms, gsea_tuning* best, 
  *      over every instance (one device batch: num_perms x num_genes buffers
  *      per instance): the permutations; the metric (tensor-core form: one
  *      launch set per metric family; plain form: one launch per metric and
- *      kernel path); the sort (one launch per
- *      register-resident class; instances beyond the register forms sort on
- *      their own); one persistent enrichment launch per size class (bitmap
+ *      rounds of a warp); the sort (one launch per shape of the bucket sort
+ *      and per class of the radix sorts behind it; instances beyond those
+ *      sort on their own); one persistent enrichment launch per size class (bitmap
  *      words per lane) whose CTAs pull (instance, permutation) items,
- *      largest instances first; the statistics (nine launches).  Every
+ *      largest instances first; the statistics (four launches).  Every
  *      instance's results are its solo plan's bit for bit.  The first
  *      execute captures all of it into one CUDA graph; later executes
  *      replay that graph (gsea_batch_set_inputs or gsea_batch_autotune make
  *      the next execute capture again).  gsea_batch_autotune tunes every
- *      instance's plain metric (permutations per thread, which picks its
+ *      instance's plain metric (rounds of a warp, which pick its
  *      launch group) and the enrichment launch per size class.            */
 typedef struct gsea_batch_s* gsea_batch;
 /* streams: size of the stream pool (0 = 16) over which an execute spreads
