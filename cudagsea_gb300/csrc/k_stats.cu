@@ -297,9 +297,9 @@ constexpr int kKeysMax = 65535;              // the table counts keys in 16 bits
 // b, b + gridDim.x, ... in the chunks c, c + gridDim.y, ... of kHistCols
 // columns of each set's columns 1..m_k-1, m_k = min(n_k, hist_cols) (the
 // adaptive test's intermediate rounds bin only the pilot columns: the same
-// pooled null, each set's nulls weighted to equal total weight).  With
-// `staged` the sorted observed keys are in shared memory, and so are counters
-// of the bins: the block takes the sets of one length, which have one weight,
+// pooled null, each set's nulls weighted to equal total weight).  staged: 1 the
+// sorted observed keys are in shared memory, 2 and counters of the bins: the
+// block takes the sets of one length, which have one weight,
 // and adds count times weight to the bins, in place of an FP64 atomic a score
 // (the six rounds of an adaptive test of 5,000 sets x up to 20,000 columns 3,566
 // -> 760 us).
@@ -308,8 +308,8 @@ __global__ void __launch_bounds__(kHistThreads)
 stats_fdr_hist_kernel(const T* __restrict__ es, int K, int64_t ld, const int64_t* __restrict__ counts,
                       int64_t hist_cols, const T* __restrict__ fac, const T* sorted_pos, const T* sorted_neg,
                       double* __restrict__ hpos, double* __restrict__ hneg, unsigned long long* __restrict__ totals,
-                      bool staged) {
-    extern __shared__ __align__(16) unsigned char hist_smem[];  // when staged: ObservedKeys, counters
+                      int staged) {
+    extern __shared__ __align__(16) unsigned char hist_smem[];  // ObservedKeys, counters
     const unsigned npos = (unsigned)totals[2], nneg = (unsigned)totals[3];
     double* wtot = reinterpret_cast<double*>(totals + 4);
     double cpos = 0.0, cneg = 0.0;
@@ -331,7 +331,19 @@ stats_fdr_hist_kernel(const T* __restrict__ es, int K, int64_t ld, const int64_t
         return n < hist_cols ? n : hist_cols;
     };
     auto weight = [&](int64_t n) { return counts ? (double)(ld - 1) / (double)(n - 1) : 1.0; };
-    if (staged) {
+    // a score at a time
+    auto one_by_one = [&](auto&& upto) {
+        for (int64_t k = blockIdx.x; k < K; k += gridDim.x) {
+            const int64_t n = columns(k);
+            if (n < 2) continue;
+            const double w = weight(n);
+            row_scores(k, n, [&](bool pos, T v) {
+                (pos ? cpos : cneg) += w;
+                atomicAdd((pos ? hpos : hneg) + upto(pos, v), w);
+            });
+        }
+    };
+    if (staged == 2) {
         const ObservedKeys<T> keys(hist_smem, K, sorted_pos, sorted_neg, npos, nneg);
         unsigned* const h = reinterpret_cast<unsigned*>(hist_smem + ObservedKeys<T>::bytes(K));  // 2 (K + 2)
         const int W = 2 * (K + 2);
@@ -367,17 +379,13 @@ stats_fdr_hist_kernel(const T* __restrict__ es, int K, int64_t ld, const int64_t
                 }
             }
         }
+    } else if (staged == 1) {
+        const ObservedKeys<T> keys(hist_smem, K, sorted_pos, sorted_neg, npos, nneg);
+        one_by_one([&](bool pos, T v) { return keys.upto(pos, v); });
     } else {
-        for (int64_t k = blockIdx.x; k < K; k += gridDim.x) {
-            const int64_t n = columns(k);
-            if (n < 2) continue;
-            const double w = weight(n);
-            row_scores(k, n, [&](bool pos, T v) {
-                (pos ? cpos : cneg) += w;
-                atomicAdd(pos ? &hpos[upper_bound_t(sorted_pos, 0u, npos, v)]
-                              : &hneg[upper_bound_t(sorted_neg, 0u, nneg, v)], w);
-            });
-        }
+        one_by_one([&](bool pos, T v) {
+            return upper_bound_t(pos ? sorted_pos : sorted_neg, 0u, pos ? npos : nneg, v);
+        });
     }
     for (int o = 16; o >= 1; o >>= 1) {
         cpos += __shfl_xor_sync(kFullMask, cpos, o);
@@ -892,14 +900,16 @@ cudaError_t launch_stats_ragged(const T* es, int K, int64_t ld, const int64_t* c
     if (ld > 1) {
         // Two blocks to an SM where the keys leave room for it, each over many
         // sets, so that staging the keys pays; few sets are split by columns.
-        const size_t smem = ObservedKeys<T>::bytes(K) + 2 * ((size_t)K + 2) * sizeof(unsigned);
-        const bool staged = smem + 1024 <= (size_t)max_smem && 2 * (int64_t)K <= kKeysMax;
+        const size_t room = max_smem > 1024 ? (size_t)max_smem - 1024 : 0, keys = ObservedKeys<T>::bytes(K);
+        const size_t counters = 2 * ((size_t)K + 2) * sizeof(unsigned);
+        const int staged = 2 * (int64_t)K > kKeysMax || keys > room ? 0 : keys + counters > room ? 1 : 2;
+        const size_t smem = staged == 0 ? 0 : staged == 1 ? keys : keys + counters;
         const int64_t want = 2 * (int64_t)sms, chunks = (hist_cols - 1 + kHistCols - 1) / kHistCols;
         const int64_t x = K < want ? K : want, y = std::min<int64_t>(std::max<int64_t>(1, 2 * want / x), chunks);
         auto kern = stats_fdr_hist_kernel<T>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, staged ? (int)smem : 0);
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kern<<<dim3((unsigned)x, (unsigned)(y > 0 ? y : 1)), kHistThreads, staged ? smem : 0, st>>>(
+        kern<<<dim3((unsigned)x, (unsigned)(y > 0 ? y : 1)), kHistThreads, smem, st>>>(
             es, K, ld, counts, hist_cols, fac, sorted_pos, sorted_neg, hpos, hneg, totals, staged);
     }
     stats_fdr_suffix_kernel<<<2, 1024, 0, st>>>(hpos, hneg, totals);

@@ -62,11 +62,11 @@ def test_statistics_at_block_edges(gpu, K, P, dtype):
 
 
 @pytest.mark.parametrize("K,P", [(1, 2), (2, 9000), (5, 8193), (303, 40), (305, 33), (1023, 9), (6150, 12),
-                                 (15000, 3), (30000, 3)])
+                                 (15000, 3), (20000, 4), (30000, 3)])
 @pytest.mark.parametrize("dtype", [np.float32, np.float64], ids=["f32", "f64"])
 def test_ragged_form_with_every_column(gpu, K, P, dtype):
-    """The weighted histogram with weights of 1: keys in shared memory or (the
-    largest collections) not, sets over blocks, columns over blocks."""
+    """The weighted histogram with weights of 1: keys and counters in shared
+    memory, keys only or (the largest collections) neither; sets over blocks, columns over blocks."""
     import torch
     es = scores(K, P, dtype)
     x = torch.from_numpy(es).cuda()
