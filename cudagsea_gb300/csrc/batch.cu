@@ -542,10 +542,9 @@ int gsea_batch_set_inputs(gsea_batch b, int64_t i, const void* exprs, const uint
     GSEA_CUDA(cudaSetDevice(b->device), "cudaSetDevice");
     if (b->main) GSEA_CUDA(cudaStreamSynchronize(b->main), "stream sync");
     const int rc = gsea_plan_set_inputs(b->plans[i], exprs, labels, set_offsets, set_genes);
-    if (rc) return rc;
-    b->ready[i] = 1;
     drop_graph(b);  // buffers of the sets may have moved
-    return GSEA_OK;
+    b->ready[i] = b->plans[i]->inputs_set ? 1 : 0;  // a failed upload may have left the instance without sets
+    return rc;
 }
 
 int gsea_batch_autotune(gsea_batch b, int64_t sample_perms) {

@@ -180,6 +180,7 @@ int upload_sets(gsea_plan_s* p, const int64_t* off, const int32_t* genes, cudaSt
     const int64_t nnz = off[K];
     if (nnz > p->nnz_cap || (p->ranks16 && !p->set_list)) {
         drop_graph(p);  // the captured launches point at the old buffer
+        p->inputs_set = false;  // until the upload is complete: there are no sets if an allocation fails
         if (p->own_sets && p->set_genes) cudaFree(p->set_genes);
         p->set_genes = nullptr;
         if (p->own_sets && p->set_list) cudaFree(p->set_list);
