@@ -579,6 +579,9 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
                                             T* __restrict__ es_col, int64_t es_stride, T* s_w, RankT* s_rank,
                                             uint32_t* bm, int* next_set, int part_lo = 0, int part_hi = 1,
                                             int parts = 1) {
+    // the general procedure reads weights of type T; 16-bit ranks have room
+    // for floats only (es_weight_bytes)
+    static_assert(WPL > 0 || sizeof(RankT) == 4, "16-bit ranks take the direct procedures");
     const int tid = threadIdx.x, lane = tid & 31;
     const int words = (G + 31) >> 5;
     const int wpl = WPL > 0 ? WPL : (words + 31) >> 5;  // bitmap words per lane
@@ -806,7 +809,7 @@ constexpr bool pairs_up() {
 }
 
 // WPL > 0: bitmap words per lane held in registers by the list procedure
-// (G <= 1024*WPL, ranks < 65536); WPL == 0: general procedure only.
+// (G <= 1024*WPL, 16-bit ranks); WPL == 0: general procedure (32-bit ranks).
 template <class T, class RankT, int WARPS, int STAGE, int WPL>
 __global__ void __launch_bounds__(WARPS * 32, pairs_up<T, WARPS, STAGE>() ? 2 : 1)
 es_kernel(const RankT* __restrict__ ranks, const T* __restrict__ sorted_abs, int G, int num_perms,
@@ -861,8 +864,7 @@ es_kernel(const RankT* __restrict__ ranks, const T* __restrict__ sorted_abs, int
 // items from a global counter until all are done; items run in task order
 // (tasks sorted by decreasing cost by the caller) and a task's permutations
 // in order.  item_end[t] = items of tasks 0..t; Gmax sizes the staging and
-// the bitmap regions of the size class (every task: G <= Gmax, and
-// G <= 1024*WPL for WPL > 0).
+// the bitmap regions of the size class (every task: G <= Gmax <= 1024*WPL).
 template <class T, class RankT, int WARPS, int STAGE, int WPL>
 __global__ void __launch_bounds__(WARPS * 32)
 es_batch_kernel(const EsTask<T>* __restrict__ tasks, const int64_t* __restrict__ item_end, int ntasks,
@@ -870,7 +872,7 @@ es_batch_kernel(const EsTask<T>* __restrict__ tasks, const int64_t* __restrict__
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int next_set;
     __shared__ long long s_item;
-    const int region = WPL > 0 ? lane_stride<WPL>() * 32 : (Gmax + 31) >> 5;
+    const int region = lane_stride<WPL>() * 32;
     T* s_w;
     RankT* s_rank;
     uint32_t* bm;
@@ -1017,10 +1019,8 @@ cudaError_t launch_es_w(const RankT* ranks, const T* sorted_abs, int G, int P, c
             case 64:
                 if constexpr (STAGE == 0) return launch_es_v<T, RankT, WARPS, 0, 64>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride, col0, grid, st, K_dev);
                 return cudaErrorInvalidValue;
-            default: break;
+            default: return cudaErrorInvalidValue;  // none: es_wpl covers every G of 16-bit ranks
         }
-        return launch_es_v<T, RankT, WARPS, STAGE, 0>(ranks, sorted_abs, G, P, sets, order, decay, K, es, stride,
-                                                      col0, grid, st, K_dev);
     }
 }
 
@@ -1140,7 +1140,6 @@ cudaError_t launch_es_batch_w(const EsTask<T>* tasks, const int64_t* item_end, i
         case 64:
             if constexpr (STAGE == 0) return launch_es_batch_v<T, WARPS, 0, 64>(tasks, item_end, ntasks, nitems, counter, Gmax, st);
             return cudaErrorInvalidValue;
-        case 0: return launch_es_batch_v<T, WARPS, STAGE, 0>(tasks, item_end, ntasks, nitems, counter, Gmax, st);
         default: return cudaErrorInvalidValue;
     }
     }
