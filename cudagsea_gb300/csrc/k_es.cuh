@@ -217,13 +217,19 @@ struct HitWalk {
     uint32_t word4 = 0u, lane4;  // four times the rank of the word's top bit / of the lane's first
     __device__ __forceinline__ HitWalk(const uint32_t* words, int w0, const LaneWords<WPL>& w)
         : bmw((uint32_t)__cvta_generic_to_shared(words)), nz(w.nz), nz2(w.nz2), lane4((uint32_t)w0 << 7) {}
+    // next()'s reads are unknown to the compiler, which could move the clearing
+    // of the words before them: every store after the walk's scope stays behind
+    // this, and its inputs are what the last read gave
+    __device__ __forceinline__ ~HitWalk() { asm volatile("" ::"r"(cur), "r"(nz) : "memory"); }
     __device__ __forceinline__ uint32_t next() {
         if (WPL > 32 && (cur | nz) == 0u) {
             nz = nz2;
             bmw += 32u * 4u;
             lane4 += 32u << 7;
         }
-        // reads words no one changes during the walk: no memory clobber
+        // No memory clobber, which would order the walk's other loads too: the
+        // words were marked before nz was read from them, and are cleared after
+        // the walk's scope (the destructor).
         asm(
             "{\n"
             " .reg .pred p;\n"
