@@ -978,7 +978,7 @@ cudaError_t launch_es_v(const RankT* ranks, const T* sorted_abs, int G, int P, c
                         int64_t col0, int grid, cudaStream_t st, const int* K_dev) {
     const size_t smem = es_smem_bytes<T, RankT, WARPS, STAGE>(G);
     auto kern = es_kernel<T, RankT, WARPS, STAGE, WPL>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;  // resident CTAs per SM: the grid fills the device once
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WARPS * 32, smem);
@@ -1101,7 +1101,7 @@ cudaError_t launch_es_batch_v(const EsTask<T>* tasks, const int64_t* item_end, i
                               unsigned long long* counter, int Gmax, cudaStream_t st) {
     const size_t smem = es_smem_bytes<T, uint16_t, WARPS, STAGE>(Gmax);
     auto kern = es_batch_kernel<T, uint16_t, WARPS, STAGE, WPL>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 1, per_sm = 0;
     cudaGetDevice(&dev);

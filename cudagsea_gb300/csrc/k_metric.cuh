@@ -699,7 +699,7 @@ cudaError_t launch_metric_acc(int comb, const T* X, int G, int S, const uint32_t
     const size_t smem = metric_smem<ACC, T>(w, S);
     auto kern = metric_kernel<ACC, T>;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(kern, smem);
         if (e != cudaSuccess) return e;
     }
     kern<<<dim3((unsigned)tiles, (unsigned)((groups + w - 1) / w)), 32 * w, smem, st>>>(
@@ -767,7 +767,7 @@ cudaError_t launch_metric_multi_acc(int comb, int rounds, const MetricTask<T>* d
     const size_t smem = metric_smem<ACC, T>(w, smax);
     auto kern = metric_multi<ACC, T>;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(kern, smem);
         if (e != cudaSuccess) return e;
     }
     kern<<<dim3((unsigned)tiles, (unsigned)((groups + w - 1) / w), (unsigned)n), 32 * w, smem, st>>>(d, comb, rounds);

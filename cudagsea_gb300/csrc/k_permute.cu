@@ -134,8 +134,10 @@ cudaError_t launch_permute(const uint8_t* labels, int S, int64_t num_perms, int6
     if (num_perms <= 0) return cudaSuccess;
     const size_t smem = (size_t)S * kPermThreads;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(permute_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) {
+        const cudaError_t e = allow_smem(permute_kernel, smem);
+        if (e != cudaSuccess) return e;
+    }
     const int64_t blocks = (num_perms + kPermThreads - 1) / kPermThreads;
     permute_kernel<<<(unsigned)blocks, kPermThreads, smem, st>>>(labels, S, num_perms, perm_offset,
                                                                seed, masks, words);
@@ -154,7 +156,7 @@ cudaError_t launch_permute_multi(const PermTask* d_tasks, const PermTask* h_task
     }
     const size_t smem = (size_t)smax * kPermThreads;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(permute_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(permute_multi, smem);
     if (e != cudaSuccess) return e;
     const int64_t blocks = (pmax + kPermThreads - 1) / kPermThreads;
     permute_multi<<<dim3((unsigned)blocks, 1, (unsigned)n), kPermThreads, smem, st>>>(d_tasks);

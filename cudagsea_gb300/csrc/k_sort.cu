@@ -751,7 +751,7 @@ cudaError_t launch_regs(const T* keys, int G, int P, bool desc, const SortBuffer
                         cudaStream_t st) {
     const size_t smem = regs_smem_bytes<T, ITEMS>();
     auto kern = sort_regs_kernel<T, RankT, ITEMS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     const int fill = (only ? 1 : 4) * num_sms();  // after the bucket sort there is seldom anything left
     kern<<<P < fill ? P : fill, kThreads, smem, st>>>(keys, G, P, desc, static_cast<RankT*>(o.ranks),
@@ -765,7 +765,7 @@ cudaError_t launch_cluster(const T* keys, int G, int P, bool desc, const SortBuf
                            cudaStream_t st) {
     const size_t smem = cluster_smem_bytes<T, ITEMS>();
     auto kern = sort_cluster_kernel<T, RankT, ITEMS, CL>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 1;  // a one-CTA "cluster" may share its SM with another CTA
     if (CL == 1) {
@@ -824,7 +824,7 @@ cudaError_t launch_radix(const T* keys, int G, int P, bool desc, const SortBuffe
     const size_t dyn = stage && rbytes > tiled_stage_bytes<U>() ? rbytes : tiled_stage_bytes<U>();
     auto kern = sort_tiled_kernel<T, RankT>;
     // opt in every time: static + dynamic pass the 48 KB default
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    cudaError_t e = allow_smem(kern, dyn);
     if (e != cudaSuccess) return e;
     kern<<<grid, kThreads, dyn, st>>>(keys, G, P, desc, static_cast<RankT*>(o.ranks), static_cast<T*>(o.sorted_abs),
                                       o.order, static_cast<unsigned char*>(o.scratch), stage, o.error_flag, only);
@@ -853,7 +853,7 @@ template <class T, class RankT, int ITEMS>
 cudaError_t launch_regs_multi(const SortTask* d, int n, cudaStream_t st) {
     const size_t smem = regs_smem_bytes<T, ITEMS>();
     auto kern = sort_regs_multi<T, RankT, ITEMS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     const int per = (num_sms() + n - 1) / n;  // CTAs per instance: about one wave over the SMs in all
     kern<<<dim3((unsigned)(per > 0 ? per : 1), 1, (unsigned)n), kThreads, smem, st>>>(d);
@@ -865,7 +865,7 @@ template <class T, class RankT, int ITEMS, int CL>
 cudaError_t launch_cluster_multi(const SortTask* d, int n, cudaStream_t st) {
     const size_t smem = cluster_smem_bytes<T, ITEMS>();
     auto kern = sort_cluster_multi<T, RankT, ITEMS, CL>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     const int per = (num_sms() / CL + n - 1) / n;  // clusters per instance
     kern<<<dim3((unsigned)(CL * (per > 0 ? per : 1)), 1, (unsigned)n), kThreads, smem, st>>>(d);

@@ -574,7 +574,7 @@ cudaError_t launch_bucket(const T* keys, int G, int P, bool desc, const SortBuff
     const int cap = ITEMS > 0 ? G : window_cap<NT>(G);
     const size_t smem = bucket_smem<T, NT, ITEMS>(G, cap);
     auto kern = sort_bucket_kernel<T, NT, ITEMS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);
@@ -595,7 +595,7 @@ cudaError_t launch_bucket_multi(const SortTask* d, const SortTask* h, int n, cud
         smem = s > smem ? s : smem;
     }
     auto kern = sort_bucket_multi<T, NT, ITEMS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem);

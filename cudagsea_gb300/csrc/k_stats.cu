@@ -860,11 +860,8 @@ cudaError_t launch_stats_ragged(const T* es, int K, int64_t ld, const int64_t* c
         const DenseDims d{K, dense_hist_blocks<T>(K, ld, sms), ld, p_fwer};
         if (d.rows > 0 && d.step2_blocks() <= INT32_MAX) {
             const size_t smem = dense_hist_smem<T>(K);
-            cudaError_t e = cudaFuncSetAttribute(stats_dense3_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(stats_dense4_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)dense_q_smem(K));
+            cudaError_t e = allow_smem(stats_dense3_kernel<T>, smem);
+            if (e == cudaSuccess) e = allow_smem(stats_dense4_kernel<T>, dense_q_smem(K));
             if (e != cudaSuccess) return e;
             const int64_t clear = (d.init() + 255) / 256;  // blocks that clear, at most one to an SM more
             const int b1 = d.set_blocks() > sms ? d.set_blocks() : (int)(clear < sms ? std::max<int64_t>(clear, d.set_blocks()) : sms);
@@ -907,7 +904,7 @@ cudaError_t launch_stats_ragged(const T* es, int K, int64_t ld, const int64_t* c
         const int64_t want = 2 * (int64_t)sms, chunks = (hist_cols - 1 + kHistCols - 1) / kHistCols;
         const int64_t x = K < want ? K : want, y = std::min<int64_t>(std::max<int64_t>(1, 2 * want / x), chunks);
         auto kern = stats_fdr_hist_kernel<T>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = allow_smem(kern, smem);
         if (e != cudaSuccess) return e;
         kern<<<dim3((unsigned)x, (unsigned)(y > 0 ? y : 1)), kHistThreads, smem, st>>>(
             es, K, ld, counts, hist_cols, fac, sorted_pos, sorted_neg, hpos, hneg, totals, staged);
@@ -952,11 +949,8 @@ cudaError_t launch_stats_multi(const StatsTask<T>* d_tasks, const StatsTask<T>* 
     }
     if (b2 > INT32_MAX) return cudaErrorInvalidValue;
     const unsigned z = (unsigned)n;
-    cudaError_t e = cudaFuncSetAttribute(stats_dense3_multi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(stats_dense4_multi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)dense_q_smem(Kmax));
+    cudaError_t e = allow_smem(stats_dense3_multi<T>, smem);
+    if (e == cudaSuccess) e = allow_smem(stats_dense4_multi<T>, dense_q_smem(Kmax));
     if (e != cudaSuccess) return e;
     stats_dense1_multi<T><<<dim3((unsigned)b1, 1, z), 256, 0, st>>>(d_tasks);
     stats_dense2_multi<T><<<dim3((unsigned)b2, 1, z), 128, 0, st>>>(d_tasks);
