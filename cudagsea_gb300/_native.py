@@ -22,7 +22,7 @@ STATUS = {
     8: "GSEA_ERR_INJECTED", 9: "GSEA_ERR_INVALID_INPUT",
 }
 
-BUF_EXPRS, BUF_LABEL_MASKS, BUF_KEYS, BUF_RANKS, BUF_ORDER, BUF_ES, BUF_STATS, BUF_SORTED = range(8)
+BUF_EXPRS, BUF_LABEL_MASKS, BUF_KEYS, BUF_RANKS, BUF_ORDER, BUF_ES, BUF_STATS, BUF_SORTED, BUF_SORT_LEFT = range(9)
 FORM_PLAIN, FORM_CHOSEN, FORM_CHOSEN_FP64 = 0, 1, 2
 STAGES = ("permute", "metric", "sort", "es", "stats")
 

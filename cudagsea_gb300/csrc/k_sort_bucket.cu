@@ -9,10 +9,14 @@
 // or two keys per bucket, and the rest is a handful of compares:
 //   1. a coarse histogram of the top bits of the 32-bit radix image (sign,
 //      exponent, one or two mantissa bits: a half or quarter octave per bin),
-//      over every fourth key, gives each bin as many buckets as it holds
+//      over a quarter of the keys, gives each bin as many buckets as it holds
 //      keys; inside a bin the remaining bits interpolate linearly.  The map
 //      key -> bucket never decreases, whatever the histogram, so only the
-//      bucket sizes depend on the sampling;
+//      bucket sizes depend on the sampling.  The quarter is eight genes of
+//      every 32, so that it does not depend on how the table orders its genes
+//      (sampled(); one row of threads in four saw none of the wide genes of a
+//      table ordered by scale, and every permutation of it was declined: 1,000
+//      of 20,000 genes ordered so 539 -> 208 us);
 //   2. the keys of every bucket are counted (16-bit counters, two to a word)
 //      and the counts scanned;
 //   3. (key, gene) pairs go to their bucket's slots in any order;
@@ -43,8 +47,6 @@
 // the latency of shared memory between the barriers bound it (22 M warp
 // instructions per 152 permutations of 20,000 genes at 62% issue activity;
 // DRAM traffic is the keys once).
-#include <type_traits>
-
 #include "common.cuh"
 #include "kernels.h"
 
@@ -55,7 +57,7 @@ constexpr int kBig = 64;        // pairs of a bucket ranked by compares
 constexpr int kMaxBig = 16;     // tie buckets of a permutation
 constexpr int kMaxCompares = 16;  // compares per gene on average
 constexpr int kMaxWindows = 16;
-constexpr int kSample = 4;      // one key in four enters the coarse histogram
+constexpr int kSample = 4;      // one key in four enters the coarse histogram (beyond one row of threads)
 
 template <int NT>
 constexpr int coarse_bits() { return NT >= 1024 ? 11 : 10; }
@@ -74,11 +76,18 @@ __device__ __forceinline__ uint32_t image32(double v, bool descending) {
     return descending ? ~u : u;
 }
 
+// The keys of the coarse histogram: gene g = i * NT + t (row i of the block's
+// threads) with (t / 8) % kSample == i % kSample -- a sector of 32 bytes
+// of each 128 in fp32, so that a pass over them loads no more than it uses, and
+// another one in the next row.  Up to NT genes all of them.
+__host__ __device__ __forceinline__ int sampled_row(int t) { return (t >> 3) & (kSample - 1); }
 // buckets of a permutation: kSample times the sampled keys (16-bit indices)
-__host__ __device__ __forceinline__ int bucket_count(int G, int NT, int sample) {
-    int n = 0;
-    for (int i = 0; i * NT < G; i += sample) n += G - i * NT < NT ? G - i * NT : NT;
-    n *= sample;
+__host__ __device__ __forceinline__ int bucket_count(int G, int NT) {
+    if (G <= NT) return G;
+    const int rows = G / NT, rest = G - rows * NT;
+    int last = (rest & 31) - 8 * (rows & (kSample - 1));  // of the last, partial row
+    last = last < 0 ? 0 : last > 8 ? 8 : last;
+    const int n = kSample * (rows * (NT / kSample) + 8 * (rest >> 5) + last);
     return n < 65534 ? n : 65534;
 }
 
@@ -137,8 +146,8 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
     constexpr int CB = coarse_bits<NT>();
     constexpr int NC = 1 << CB;
     constexpr int BPT = NC / NT;           // coarse bins per thread
-    constexpr int SAMPLE = REGS && ITEMS < kSample ? 1 : kSample;
     static_assert(NC % NT == 0, "whole coarse bins per thread");
+    static_assert(ITEMS % kSample == 0 && NT % 32 == 0, "sampled rows");
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_scan[3][32];
     __shared__ BigBucket s_big[kMaxBig];
@@ -146,7 +155,7 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
     __shared__ uint32_t s_wb[kMaxWindows + 1], s_wp[kMaxWindows + 1];  // windows: first bucket, first slot
 
     const int tid = threadIdx.x;
-    const int NB = bucket_count(G, NT, SAMPLE);
+    const int NB = bucket_count(G, NT);
     const Layout L(G, NB, cap, REGS, CB);
     uint2* const H = reinterpret_cast<uint2*>(smem);  // coarse bin: first bucket, buckets
     uint32_t* const C = reinterpret_cast<uint32_t*>(smem + L.c);  // bucket counters, two 16-bit halves a word
@@ -190,32 +199,30 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
             }
         }
         // f(image, gene) for every gene of the thread
-        auto each = [&](auto&& f, auto step) {
+        auto each = [&](auto&& f) {
             if constexpr (REGS) {
 #pragma unroll
-                for (int i = 0; i < NREG; i += decltype(step)::value) {
+                for (int i = 0; i < NREG; i++) {
                     const int g = tid + i * NT;
                     if (g < G) f(a[i], g);
                 }
             } else {
                 constexpr int U = 4;  // loads in flight
-                for (int g0 = tid; g0 < G; g0 += U * NT * decltype(step)::value) {
+                for (int g0 = tid; g0 < G; g0 += U * NT) {
                     T v[U];
 #pragma unroll
                     for (int u = 0; u < U; u++) {
-                        const int g = g0 + u * NT * decltype(step)::value;
+                        const int g = g0 + u * NT;
                         v[u] = g < G ? kp[g] : T(0);
                     }
 #pragma unroll
                     for (int u = 0; u < U; u++) {
-                        const int g = g0 + u * NT * decltype(step)::value;
+                        const int g = g0 + u * NT;
                         if (g < G) f(image32(v[u], descending), g);
                     }
                 }
             }
         };
-        using Every = std::integral_constant<int, 1>;
-        using Sampled = std::integral_constant<int, SAMPLE>;
 
         // 1. coarse histogram -> first bucket and number of buckets per bin
 #pragma unroll
@@ -223,7 +230,36 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
         for (int w = tid; w < CW; w += NT) C[w] = 0u;
         if (tid == 0) s_nbig = s_pairs = s_bad = 0u;
         __syncthreads();
-        each([&](uint32_t k, int) { atomicAdd(&H[k >> (32 - CB)].y, (uint32_t)SAMPLE); }, Sampled{});
+        {
+            const int row = sampled_row(tid);
+            if constexpr (REGS) {
+                if (G <= NT) {
+                    if (tid < G) atomicAdd(&H[a[0] >> (32 - CB)].y, 1u);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < NREG; i += kSample) {
+                        const uint32_t k01 = row & 1 ? a[i + 1] : a[i], k23 = row & 1 ? a[i + 3] : a[i + 2];
+                        if (tid + (i + row) * NT < G)
+                            atomicAdd(&H[(row & 2 ? k23 : k01) >> (32 - CB)].y, (uint32_t)kSample);
+                    }
+                }
+            } else {
+                constexpr int U = 4;  // loads in flight
+                for (int g0 = tid + row * NT; g0 < G; g0 += U * kSample * NT) {
+                    T v[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int g = g0 + u * kSample * NT;
+                        v[u] = g < G ? kp[g] : T(0);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        if (g0 + u * kSample * NT < G)
+                            atomicAdd(&H[image32(v[u], descending) >> (32 - CB)].y, (uint32_t)kSample);
+                    }
+                }
+            }
+        }
         __syncthreads();
         {
             uint32_t c[BPT], sum = 0, total;
@@ -258,7 +294,7 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
             each([&](uint32_t k, int) {
                 const uint32_t b = bucket_of(k);
                 atomicAdd(&C[b >> 1], 1u << ((b & 1u) << 4));
-            }, Every{});
+            });
         }
         __syncthreads();
         uint32_t slots;  // pairs with a slot: those of buckets ranked by compares
@@ -336,7 +372,7 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
                         mine = min(mine, (uint32_t)g);
                         atomicOr(&bitmap[g >> 5], 1u << (g & 31));
                     }
-                }, Every{});
+                });
                 if (mine != 0xffffffffu) atomicMin(&s_first, mine);
                 __syncthreads();
                 const T ref = kp[s_first];
@@ -344,7 +380,7 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
                 bool differs = false;
                 each([&](uint32_t k, int g) {
                     if (bucket_of(k) == big) differs |= RadixKey<T>::from(kp[g], descending) != kref;
-                }, Every{});
+                });
                 if (differs) s_bad = 1u;
                 __syncthreads();
                 const bool bad = s_bad != 0u;
@@ -424,7 +460,7 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
                     const uint32_t slot = ((atomicSub(&C[b >> 1], 1u << sh) >> sh) & 0xffffu) - 1u - p_lo;
                     skey[slot] = k;
                     sgene[slot] = (uint16_t)g;
-                }, Every{});
+                });
             }
             if constexpr (AHEAD) {
                 const int pn = p + gx;
@@ -542,7 +578,7 @@ constexpr int kSmemCap = 232448 - 1024;  // a CTA's shared memory, less the stat
 // and the bitmap leave (the ranks by gene are turned round over all of it)
 template <int NT>
 int window_cap(int G) {
-    const int left = kSmemCap - (int)Layout(G, bucket_count(G, NT, kSample), 0, false, coarse_bits<NT>()).bytes - 16;
+    const int left = kSmemCap - (int)Layout(G, bucket_count(G, NT), 0, false, coarse_bits<NT>()).bytes - 16;
     const int cap = left / 6;
     return cap < G + kBig ? cap : G + kBig;
 }
@@ -558,8 +594,7 @@ __global__ void __launch_bounds__(NT, min_blocks<NT>()) sort_bucket_multi(const 
 
 template <class T, int NT, int ITEMS>
 size_t bucket_smem(int G, int cap) {
-    constexpr int SAMPLE = ITEMS > 0 && ITEMS < kSample ? 1 : kSample;
-    return Layout(G, bucket_count(G, NT, SAMPLE), cap, ITEMS > 0, coarse_bits<NT>()).bytes;
+    return Layout(G, bucket_count(G, NT), cap, ITEMS > 0, coarse_bits<NT>()).bytes;
 }
 
 int sm_count() {

@@ -217,7 +217,10 @@ typedef enum {
     GSEA_BUF_ORDER = 4,       /* [P_batch][G] uint32, gene at each position    */
     GSEA_BUF_ES = 5,          /* [K][P] T                                      */
     GSEA_BUF_STATS = 6,       /* [5][K] T                                      */
-    GSEA_BUF_SORTED = 7       /* [P_batch][G] T, |metric| at each position     */
+    GSEA_BUF_SORTED = 7,      /* [P_batch][G] T, |metric| at each position     */
+    GSEA_BUF_SORT_LEFT = 8    /* [permutations of the last batch] uint8, non-zero: the bucket sort left the
+                                 permutation to a radix sort (none without a bucket sort: more than
+                                 65,535 genes, sort_variant 2)                  */
 } gsea_buffer;
 int gsea_plan_buffer(gsea_plan plan, int which, void** dev_ptr, size_t* bytes);
 /* synchronise and copy min(bytes, buffer size) bytes of a plan buffer to host */
