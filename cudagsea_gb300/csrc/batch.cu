@@ -216,8 +216,10 @@ int build_multi(gsea_batch_s* b, Multi<gsea::StatsTask<T>>& stats) {
             st.num_perms = (int)c.num_perms;
             st.descending = c.ascending ? 0 : 1;
             st.cap = gsea::sort_bucket_cap(st.G);
-            st.hard = static_cast<uint8_t*>(p->sort_scratch) +
-                      (p->sort_scratch_bytes - gsea::sort_mark_bytes(st.num_perms));
+            const bool bucket = p->tuning.sort_variant != 3;  // an instance tuned to the radix sort alone: all of it
+            st.hard = bucket ? static_cast<uint8_t*>(p->sort_scratch) +
+                                   (p->sort_scratch_bytes - gsea::sort_mark_bytes(st.num_perms))
+                             : nullptr;
             auto add = [&](std::vector<Multi<gsea::SortTask>>& to, std::map<int, size_t>& at, int key) {
                 auto it = at.find(key);
                 if (it == at.end()) {
@@ -227,7 +229,7 @@ int build_multi(gsea_batch_s* b, Multi<gsea::StatsTask<T>>& stats) {
                 }
                 to[it->second].h.push_back(st);
             };
-            add(b->bucket_sorts, bucket_at, gsea::sort_bucket_multi_class(st.G));
+            if (bucket) add(b->bucket_sorts, bucket_at, gsea::sort_bucket_multi_class(st.G));
             add(b->sorts, sort_at, cls);
         }
         const int rows = gsea::stats_multi_rows<T>((int)c.num_sets, c.num_perms);

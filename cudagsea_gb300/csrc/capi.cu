@@ -750,7 +750,7 @@ int gsea_plan_buffer(gsea_plan p, int which, void** dev_ptr, size_t* bytes) {
         case GSEA_BUF_STATS: ptr = p->stats; n = T * 5 * (size_t)p->cfg.num_sets; break;
         case GSEA_BUF_SORTED: ptr = p->sorted; n = T * G * pb; break;
         case GSEA_BUF_SORT_LEFT:
-            if (p->ranks16 && p->tuning.sort_variant != 2 && gsea::sort_bucket_class((int)p->cfg.num_genes) != 0) {
+            if (p->ranks16 && p->tuning.sort_variant < 2 && gsea::sort_bucket_class((int)p->cfg.num_genes) != 0) {
                 n = (size_t)((p->cfg.num_perms - 1) % p->pb + 1);
                 ptr = static_cast<unsigned char*>(p->sort_scratch) + p->sort_scratch_bytes - gsea::sort_mark_bytes((int)n);
             }

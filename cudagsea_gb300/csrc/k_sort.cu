@@ -834,11 +834,11 @@ cudaError_t launch_radix(const T* keys, int G, int P, bool desc, const SortBuffe
 
 template <class T, class RankT>
 cudaError_t launch_sort_t(const T* keys, int G, int P, bool desc, SortBuffers o, cudaStream_t st) {
-    if (o.variant == 1 && G > regs_max_genes<T>()) return cudaErrorInvalidValue;
+    if ((o.variant == 1 || o.variant == 3) && G > regs_max_genes<T>()) return cudaErrorInvalidValue;
     if (o.scratch_bytes < sort_scratch_bytes<T>(G, P)) return cudaErrorInvalidValue;
     const uint8_t* only = nullptr;
     if constexpr (sizeof(RankT) == 2) {
-        if (o.variant != 2 && sort_bucket_class(G) != 0) {
+        if (o.variant < 2 && sort_bucket_class(G) != 0) {
             // one mark per permutation, at the end of the scratch
             o.hard = static_cast<uint8_t*>(o.scratch) + (o.scratch_bytes - sort_mark_bytes(P));
             const cudaError_t e = launch_sort_bucket<T>(keys, G, P, desc, o, st);

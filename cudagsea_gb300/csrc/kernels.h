@@ -55,7 +55,9 @@ struct SortBuffers {
     uint32_t* order;      // optional
     void* scratch;        // per-CTA ping-pong buffers for the tiled variant, one mark per permutation
     size_t scratch_bytes;
-    int variant = 0;      // 0 automatic, 1 on-chip sorts (bucket, then register radix; fp32 G <= 40,960, fp64 G <= 20,480), 2 tiled
+    // 0 automatic, 1 on-chip sorts (bucket, then register radix; fp32 G <= 40,960, fp64 G <= 20,480), 2 tiled, 3 the
+    // register radix sort alone (the G of 1)
+    int variant = 0;
     int* error_flag = nullptr;  // set to 1 when a bounded wait of the tiled sort expires
     uint8_t* hard = nullptr;    // set by launch_sort: permutations the bucket sort left to the radix sort
 };
@@ -163,7 +165,7 @@ struct SortTask {
     void* ranks;        // [P][G] uint16
     void* sorted;       // [P][G] T
     uint32_t* order;    // [P][G] or null
-    uint8_t* hard;      // [P] permutations left to the radix sort
+    uint8_t* hard;      // [P] permutations left to the radix sort; null: all of them
     int G;
     int num_perms;
     int descending;

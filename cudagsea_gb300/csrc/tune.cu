@@ -8,7 +8,8 @@
 // Tunables (every choice computes identical results):
 //   metric      plain fp32 packed form: 4 or 8 permutations per thread;
 //               tensor-core form: 128- or 256-permutation tiles (the GEMM's N)
-//   sort        register-resident radix sort or the tiled one
+//   sort        bucket sort (with a radix sort behind it), the tiled radix sort,
+//               or the register-resident radix sort alone
 //   enrichment  8 / 16 / 24 / 32 warps per CTA; the permutation's ranks and
 //               weights staged in shared memory, its ranks only, its
 //               weights only, or read from L2
@@ -107,9 +108,12 @@ int autotune_t(gsea_plan_s* p, int64_t n64, unsigned stages, gsea_tuning* best_o
     sb.scratch_bytes = p->sort_scratch_bytes;
     sb.error_flag = p->dev_error;
     float sbest = 1e30f;
-    // beyond the register radix sorts (variant 1) the automatic choice is the
-    // bucket sort with the tiled one behind it
-    std::vector<int> sc = {G <= (c.precision == 64 ? 20480 : 40960) ? 1 : 0, 2};
+    // beyond the register radix sorts (variants 1 and 3) the automatic choice
+    // is the bucket sort with the tiled one behind it.  Variant 3 wins on tables
+    // whose keys crowd into a few values: the bucket sort declines them all
+    const bool regs = G <= (c.precision == 64 ? 20480 : 40960);
+    std::vector<int> sc = {regs ? 1 : 0, 2};
+    if (regs) sc.push_back(3);
     if (!(stages & kSort)) sc = {best.sort_variant};
     for (int v : sc) {
         sb.variant = v;
@@ -165,7 +169,7 @@ int autotune_t(gsea_plan_s* p, int64_t n64, unsigned stages, gsea_tuning* best_o
 bool valid(const gsea_tuning* t) {
     return (t->metric_pb == 0 || t->metric_pb == 4 || t->metric_pb == 8) &&
            (t->chosen_tile == 0 || t->chosen_tile == 128 || t->chosen_tile == 256) &&
-           (t->sort_variant >= 0 && t->sort_variant <= 2) &&
+           (t->sort_variant >= 0 && t->sort_variant <= 3) &&
            (t->es_warps == 0 || t->es_warps == 8 || t->es_warps == 16 || t->es_warps == 24 ||
             t->es_warps == 32) &&
            (t->es_stage >= -1 && t->es_stage <= 3);

@@ -220,7 +220,7 @@ typedef enum {
     GSEA_BUF_SORTED = 7,      /* [P_batch][G] T, |metric| at each position     */
     GSEA_BUF_SORT_LEFT = 8    /* [permutations of the last batch] uint8, non-zero: the bucket sort left the
                                  permutation to a radix sort (none without a bucket sort: more than
-                                 65,535 genes, sort_variant 2)                  */
+                                 65,535 genes, sort_variant 2 or 3)             */
 } gsea_buffer;
 int gsea_plan_buffer(gsea_plan plan, int which, void** dev_ptr, size_t* bytes);
 /* synchronise and copy min(bytes, buffer size) bytes of a plan buffer to host */
@@ -286,8 +286,9 @@ typedef struct gsea_tuning {
     int32_t sort_variant; /* 1 on-chip sorts: a bucket sort, and for the permutations it declines the
                              register radix sort (fp32, G <= 40,960: one CTA up to 20,480, a two-CTA
                              cluster exchanging through distributed shared memory beyond; fp64,
-                             G <= 20,480: one CTA up to 10,240, a two-CTA cluster beyond), 2 tiled;
-                             0: the bucket sort up to 65,535 genes with 1 or 2 behind it */
+                             G <= 20,480: one CTA up to 10,240, a two-CTA cluster beyond), 2 tiled,
+                             3 the register radix sort alone (the G of 1);
+                             0: the bucket sort up to 65,535 genes with a radix sort behind it */
     int32_t es_warps;     /* warps per CTA of the enrichment kernel: 8, 16, 24 or 32 (24: with
                              es_stage 2 or 3 only) */
     int32_t es_stage;     /* 1 stage the permutation's ranks and weights in shared memory, 2 its ranks
@@ -325,7 +326,9 @@ int gsea_plan_autotune(gsea_plan plan, int64_t sample_perms, gsea_tuning* best, 
  *      replay that graph (gsea_batch_set_inputs or gsea_batch_autotune make
  *      the next execute capture again).  gsea_batch_autotune tunes every
  *      instance's plain metric (rounds of a warp, which pick its
- *      launch group) and the enrichment launch per size class.            */
+ *      launch group), its sort (an instance whose keys crowd into a few
+ *      values skips the bucket sort) and the enrichment launch per size
+ *      class.                                                             */
 typedef struct gsea_batch_s* gsea_batch;
 /* streams: size of the stream pool (0 = 16) over which an execute spreads
  * the sort classes and the enrichment size classes */
