@@ -855,7 +855,7 @@ cudaError_t launch_regs_multi(const SortTask* d, int n, cudaStream_t st) {
     auto kern = sort_regs_multi<T, RankT, ITEMS>;
     cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
-    const int per = (num_sms() + n - 1) / n;  // CTAs per instance: about one wave over the SMs in all
+    const int per = (2 * num_sms() + n - 1) / n;  // CTAs per instance: about two waves over the SMs in all
     kern<<<dim3((unsigned)(per > 0 ? per : 1), 1, (unsigned)n), kThreads, smem, st>>>(d);
     launches_add(1);
     return cudaGetLastError();
@@ -867,7 +867,7 @@ cudaError_t launch_cluster_multi(const SortTask* d, int n, cudaStream_t st) {
     auto kern = sort_cluster_multi<T, RankT, ITEMS, CL>;
     cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
-    const int per = (num_sms() / CL + n - 1) / n;  // clusters per instance
+    const int per = (2 * num_sms() / CL + n - 1) / n;  // clusters per instance
     kern<<<dim3((unsigned)(CL * (per > 0 ? per : 1)), 1, (unsigned)n), kThreads, smem, st>>>(d);
     launches_add(1);
     return cudaGetLastError();
@@ -875,16 +875,17 @@ cudaError_t launch_cluster_multi(const SortTask* d, int n, cudaStream_t st) {
 
 }  // namespace
 
-// radix sorts of a batch (what its bucket sorts declined): few classes, a
-// batch launches each of them
+// radix sorts of a batch (what its bucket sorts declined)
 int sort_multi_class(int G, bool fp64) {
     if (G <= 0 || G > 65535) return 0;
     if (!fp64) {
-        if (G <= kThreads * 8) return 8;
-        if (G <= kThreads * 20) return 20;
+        for (int items : {4, 8, 12, 16, 20})
+            if (G <= kThreads * items) return items;
+        if (G <= 2 * kThreads * 16) return 116;
         if (G <= 2 * kThreads * 20) return 120;
         return 0;
     }
+    if (G <= kThreads * 4) return 204;
     if (G <= kThreads * 10) return 210;
     if (G <= 2 * kThreads * 10) return 310;
     return 0;
@@ -896,13 +897,18 @@ cudaError_t launch_sort_multi(const SortTask* d_tasks, int n, int cls, bool fp64
     using R = uint16_t;  // batch instances have at most 65,536 genes
     if (!fp64) {
         switch (cls) {
+            case 4: return launch_regs_multi<float, R, 4>(d_tasks, n, st);
             case 8: return launch_regs_multi<float, R, 8>(d_tasks, n, st);
+            case 12: return launch_regs_multi<float, R, 12>(d_tasks, n, st);
+            case 16: return launch_regs_multi<float, R, 16>(d_tasks, n, st);
             case 20: return launch_regs_multi<float, R, 20>(d_tasks, n, st);
+            case 116: return launch_cluster_multi<float, R, 16, 2>(d_tasks, n, st);
             case 120: return launch_cluster_multi<float, R, 20, 2>(d_tasks, n, st);
             default: return cudaErrorInvalidValue;
         }
     }
     switch (cls) {
+        case 204: return launch_cluster_multi<double, R, 4, 1>(d_tasks, n, st);
         case 210: return launch_cluster_multi<double, R, 10, 1>(d_tasks, n, st);
         case 310: return launch_cluster_multi<double, R, 10, 2>(d_tasks, n, st);
         default: return cudaErrorInvalidValue;

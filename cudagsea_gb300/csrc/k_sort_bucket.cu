@@ -26,9 +26,20 @@
 // Buckets of more than kBig pairs are ties in practice (constant or absent
 // genes give one common key): if all their keys are equal they are ranked by
 // gene through a bitmap, without compares.  A permutation with a large bucket
-// of distinct keys, too many large buckets, or too many compares in all
-// (keys crowded into a few values) is marked in hard[] and left to the radix
-// sort launched after this kernel.
+// of distinct keys, more tie buckets than pay (max_ties), or too many compares in all
+// is marked in hard[] and left to the radix sort launched after this kernel.
+//
+// Keys crowded into a few values (counts under a difference of means) are left
+// too, and found early: the counters of step 2 are fought over there, and a
+// class mean's rounding makes neighbouring floats of one value, so that
+// their buckets are large and distinct.  Threads compare keys of their own;
+// with more than a dozen equal pairs (zeros, infinities and NaN apart), which
+// stand for some 50 genes to a value whatever the number of genes, step 2 is
+// not begun, and after two such permutations in a row a CTA looks at every
+// fourth only.  Radix sort alone, found at the end, found early (counts, 60
+// samples): 1,000 permutations of 20,000 genes 395, 480, 418 us; 2,000 of 3,000 200,
+// 253, 218; 400 of 40,000 510, 562, 522; ten groups of 300 equal genes among 20,000
+// 415, 752, 435.
 //
 // fp64 keys: the 32-bit image is the key rounded down to a float-like
 // pattern (11-bit exponent clamped to 8 bits, 23 mantissa bits), which never
@@ -54,7 +65,12 @@ namespace gsea {
 namespace {
 
 constexpr int kBig = 64;        // pairs of a bucket ranked by compares
-constexpr int kMaxBig = 16;     // tie buckets of a permutation
+// tie buckets of a permutation that are still faster than the radix sort: one
+// takes 9 us of 1,000 permutations of 1,000 genes (where the radix sort takes
+// 194), 20 at 3,000 (200), 65 at 7,000 (250), 75 to 150 at 20,000 (395), 50 to 150 of
+// 300 at 60,000 (690)
+template <int NT, int ITEMS>
+constexpr int max_ties() { return NT == 256 ? 16 : ITEMS == 20 ? 2 : 4; }
 constexpr int kMaxCompares = 16;  // compares per gene on average
 constexpr int kMaxWindows = 16;
 constexpr int kSample = 4;      // one key in four enters the coarse histogram (beyond one row of threads)
@@ -150,8 +166,9 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
     static_assert(ITEMS % kSample == 0 && NT % 32 == 0, "sampled rows");
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_scan[3][32];
+    constexpr int kMaxBig = max_ties<NT, ITEMS>();
     __shared__ BigBucket s_big[kMaxBig];
-    __shared__ uint32_t s_nbig, s_pairs, s_bad, s_first;
+    __shared__ uint32_t s_nbig, s_pairs, s_bad, s_first, s_alike;
     __shared__ uint32_t s_wb[kMaxWindows + 1], s_wp[kMaxWindows + 1];  // windows: first bucket, first slot
 
     const int tid = threadIdx.x;
@@ -172,24 +189,40 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
         const uint32_t b = h.x + __umulhi(a << CB, h.y);
         return b < (uint32_t)NB ? b : (uint32_t)NB - 1u;
     };
+    // images a table may have many of without being crowded: constant and absent
+    // genes have 0 or NaN, those absent from one class an infinity in the ratios
+    auto common = [&](uint32_t k) {
+        const uint32_t u = descending ? ~k : k;
+        return u == 0x80000000u || u == 0x7fffffffu || u == 0xffffffffu || u == 0xff800000u || u == 0x007fffffu;
+    };
     constexpr int NREG = REGS ? ITEMS : 1;
     constexpr bool AHEAD = REGS && sizeof(T) == 4;  // the next permutation's keys are loaded early
     T ahead[AHEAD ? NREG : 1];
-    if constexpr (AHEAD) {
-        if (bx < num_perms) {
-#pragma unroll
-            for (int i = 0; i < NREG; i++) {
-                const int g = tid + i * NT;
-                ahead[i] = g < G ? keys[(int64_t)bx * G + g] : T(0);
-            }
-        }
-    }
+    bool loaded = false;  // the keys of the permutation at hand
     for (int w = tid; w < BW; w += NT) bitmap[w] = 0u;
 
+    int left = 0;  // permutations left in a row
     for (int p = bx; p < num_perms; p += gx) {
+        // crowded keys are a matter of the table, not of the permutation: after
+        // two in a row only every fourth is looked at
+        if (left >= 2 && (left & 3) != 0) {
+            if (tid == 0) hard[p] = 1;
+            left++;
+            continue;
+        }
         const T* const kp = keys + (int64_t)p * G;
         const int64_t base = (int64_t)p * G;
         uint32_t a[NREG];
+        if constexpr (AHEAD) {
+            if (!loaded) {
+#pragma unroll
+                for (int i = 0; i < NREG; i++) {
+                    const int g = tid + i * NT;
+                    ahead[i] = g < G ? kp[g] : T(0);
+                }
+            }
+            loaded = false;
+        }
         if constexpr (REGS) {
 #pragma unroll
             for (int i = 0; i < NREG; i++) {
@@ -228,7 +261,7 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
 #pragma unroll
         for (int j = 0; j < BPT; j++) H[tid + j * NT].y = 0u;
         for (int w = tid; w < CW; w += NT) C[w] = 0u;
-        if (tid == 0) s_nbig = s_pairs = s_bad = 0u;
+        if (tid == 0) s_nbig = s_pairs = s_bad = s_alike = 0u;
         __syncthreads();
         {
             const int row = sampled_row(tid);
@@ -257,6 +290,13 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
                         if (g0 + u * kSample * NT < G)
                             atomicAdd(&H[image32(v[u], descending) >> (32 - CB)].y, (uint32_t)kSample);
                     }
+                    bool alike = false;
+#pragma unroll
+                    for (int u = 0; u < U; u += 2) {
+                        const uint32_t k = image32(v[u], descending);
+                        alike |= g0 + (u + 1) * kSample * NT < G && k == image32(v[u + 1], descending) && !common(k);
+                    }
+                    if (alike) atomicAdd(&s_alike, 1u);
                 }
             }
         }
@@ -268,6 +308,18 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
                 c[j] = H[tid * BPT + j].y;
                 sum += c[j];
             }
+            if constexpr (REGS) {  // here the block waits for the scan
+                bool alike = false;
+#pragma unroll
+                for (int i = 0; i < NREG; i += 4) alike |= a[i] == a[i + 1];
+                if (__any_sync(kFullMask, alike)) {
+                    alike = false;
+#pragma unroll
+                    for (int i = 0; i < NREG; i += 4)
+                        alike |= tid + (i + 1) * NT < G && a[i] == a[i + 1] && !common(a[i]);
+                    if (alike) atomicAdd(&s_alike, 1u);
+                }
+            }
             uint32_t run = block_exclusive<NT>(sum, s_scan[0], total);
 #pragma unroll
             for (int j = 0; j < BPT; j++) {
@@ -276,6 +328,12 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
             }
         }
         __syncthreads();
+        if (s_alike > (REGS ? 12u : 8u)) {  // crowded keys; of G / 4 or G / 8 pairs (uniform)
+            if (tid == 0) hard[p] = 1;
+            left++;
+            __syncthreads();  // the flags are cleared next
+            continue;
+        }
         // 2. pairs per bucket, scanned.  With the keys in registers a pair
         // keeps its bucket and the count before it (its place in the bucket)
         // and C becomes the buckets' first slots; else one past their last
@@ -414,19 +472,11 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
         }
         if (tid == 0) hard[p] = give_up ? 1 : 0;
         if (give_up) {
+            left++;
             __syncthreads();  // the counters and flags are cleared next
-            if constexpr (AHEAD) {
-                const int pn = p + gx;
-                if (pn < num_perms) {
-#pragma unroll
-                    for (int i = 0; i < NREG; i++) {
-                        const int g = tid + i * NT;
-                        ahead[i] = g < G ? keys[(int64_t)pn * G + g] : T(0);
-                    }
-                }
-            }
             continue;
         }
+        left = 0;
         if (!REGS) __syncthreads();  // the windows' bounds
         for (int win = 0; win < windows; win++) {
             const uint32_t b_lo = REGS ? 0u : s_wb[win], b_hi = REGS ? (uint32_t)NB : s_wb[win + 1];
@@ -464,7 +514,8 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
             }
             if constexpr (AHEAD) {
                 const int pn = p + gx;
-                if (pn < num_perms) {
+                loaded = pn < num_perms;
+                if (loaded) {
 #pragma unroll
                     for (int i = 0; i < NREG; i++) {
                         const int g = tid + i * NT;
