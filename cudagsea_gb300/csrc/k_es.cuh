@@ -639,9 +639,9 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
             };
             Acc<float> Wm;
             const int2 rec = __ldg(sets.rec + k);  // first group of the set's list, members
-            const uint2* __restrict__ const list = sets.list + (int64_t)rec.x * 32 + lane;
+            const uint2* __restrict__ const list = sets.list + (int64_t)(rec.x < 0 ? ~rec.x : rec.x) * 32 + lane;
             const int full = rec.y >> 7, rem = rec.y & 127;
-            if (rec.y >= 0) {
+            if (F64 || rec.x >= 0) {
 #pragma unroll 1
                 for (int i = 0; i < full; i++) {
                     const uint2 q = __ldg(list + 32 * i);
@@ -698,14 +698,13 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
             } else {
                 int n;
                 bool largest;
-                const int at = rec.y < 0 ? -1
-                                         : find_extremum<WPL>(
-                                               bmw, lane * WPL,
-                                               [&](uint32_t r4) -> float {
-                                                   if constexpr (STAGE == 1 || STAGE == 3) return weight_at(s_wf, r4);
-                                                   else return (float)weight_at(wt, r4);
-                                               },
-                                               decay, G, lane, Wm, n, largest);
+                const int at = find_extremum<WPL>(
+                    bmw, lane * WPL,
+                    [&](uint32_t r4) -> float {
+                        if constexpr (STAGE == 1 || STAGE == 3) return weight_at(s_wf, r4);
+                        else return (float)weight_at(wt, r4);
+                    },
+                    decay, G, lane, Wm, n, largest);
                 if (at < 0) {  // warp-uniform
                     score = set_score_positions_f64<WPL>(bmw, lane * WPL, wt, decay, G, lane);
                     clear_words<WPL>(bmw);

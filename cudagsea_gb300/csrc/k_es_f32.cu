@@ -7,7 +7,8 @@ int es_size_class(int G) { return es_wpl(G, G <= 65536); }
 
 namespace {
 // The sets' marking lists (EsSets): one warp per set writes its groups and
-// finds duplicates and unknown ids in a bitmap of the genes.  A set's list
+// finds duplicates and unknown ids in a bitmap of the genes, from which the
+// list of a set that has any is written again.  A set's list
 // starts at group floor(offset / 128) + k, which leaves every set room for
 // its last, partial group without a scan over the sets.
 constexpr int kListWarps = 4;
@@ -25,7 +26,7 @@ es_lists_kernel(const int64_t* __restrict__ off, const int32_t* __restrict__ gen
     const int64_t a = off[k];
     const int64_t m = off[k + 1] - a;
     const int64_t first = a / 128 + k;
-    bool bad = m > INT_MAX || first > INT_MAX;
+    bool bad = false;
     for (int64_t base = 0; base < m; base += 128) {
         uint32_t e[4];
 #pragma unroll
@@ -46,7 +47,27 @@ es_lists_kernel(const int64_t* __restrict__ off, const int32_t* __restrict__ gen
         list[(first + base / 128) * 32 + lane] = make_uint2(e[0] | (e[1] << 16), e[2] | (e[3] << 16));
     }
     bad = __any_sync(kFullMask, bad);
-    if (lane == 0) rec[k] = make_int2(bad ? 0 : (int)first, bad ? -1 : (int)m);
+    int n = (int)m;  // fewer than 2^31 members to a set
+    if (bad) {  // its genes once, ascending (what stays behind them in the last group are valid ids)
+        __syncwarp();
+        uint16_t* const entries = reinterpret_cast<uint16_t*>(list + first * 32);
+        n = 0;
+        for (int w0 = 0; w0 < words; w0 += 32) {
+            uint32_t bits = w0 + lane < words ? bm[w0 + lane] : 0u;
+            const int c = __popc(bits);
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(kFullMask, incl, o);
+                if (lane >= o) incl += y;
+            }
+            for (int at = n + incl - c; bits; at++, bits &= bits - 1u)
+                entries[(at >> 7) * 128 + (at & 31) * 4 + ((at >> 5) & 3)] =
+                    (uint16_t)((w0 + lane) * 32 + __ffs(bits) - 1);
+            n += __shfl_sync(kFullMask, incl, 31);
+        }
+    }
+    if (lane == 0) rec[k] = make_int2(bad ? ~(int)first : (int)first, n);
 }
 }  // namespace
 

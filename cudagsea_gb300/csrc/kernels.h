@@ -83,8 +83,10 @@ struct EsTuning {
 // The gene sets of a plan: the caller's CSR (offsets [K+1], genes) and the
 // lists the kernel marks from (launch_es_lists; G <= 65,536).  Set k's list
 // starts at group rec[k].x: groups of 128 16-bit gene ids, entry 4*lane + i
-// of a group the set's member 32*i + lane of it; rec[k].y members, or -1 when
-// the set lists a gene twice or an unknown id (the CSR is then read).
+// of a group the set's member 32*i + lane of it; rec[k].y members.  Of a set
+// that lists a gene twice or an unknown id rec[k].x is ~group and the list has
+// its genes once, ascending; fp32, whose sums keep the caller's order, reads
+// the CSR of such a set.
 struct EsSets {
     const int64_t* off;
     const int32_t* genes;
