@@ -705,12 +705,26 @@ __device__ __forceinline__ void es_one_perm(const RankT* rk, const T* wt, int G,
                 // duplicates or unknown ids: the caller's list, each member checked
                 const int64_t a = sets.off[k];
                 const int m = (int)(sets.off[k + 1] - a);  // a set lists fewer than 2^31 members
-                for (int idx = lane; idx < m; idx += 32) {
-                    const int g = __ldg(sets.genes + a + idx);
-                    if (g >= 0 && g < G) {
-                        const uint32_t r = rk[g];
-                        const uint32_t bit = __funnelshift_r(0x80000000u, 0u, r);
-                        if (!(atomicOr(rank_word<WPL>(bm, r), bit) & bit)) Wm.add(weight(r));
+                for (int64_t base = 0; base < m; base += 128) {
+                    int g[4];
+                    uint32_t r[4];
+                    float w[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int64_t idx = base + lane + 32 * i;
+                        g[i] = idx < m ? __ldg(sets.genes + a + idx) : -1;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        r[i] = rk[g[i] >= 0 && g[i] < G ? g[i] : 0];
+                        w[i] = weight(r[i]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        if (g[i] >= 0 && g[i] < G) {
+                            const uint32_t bit = __funnelshift_r(0x80000000u, 0u, r[i]);
+                            if (!(atomicOr(rank_word<WPL>(bm, r[i]), bit) & bit)) Wm.add(w[i]);
+                        }
                     }
                 }
             }
