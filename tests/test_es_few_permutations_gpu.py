@@ -1,0 +1,41 @@
+"""Few sets and fewer permutations than CTAs: the automatic enrichment launch
+gives the scores of the asked ones and is not slower than 32 warps."""
+import numpy as np
+import pytest
+
+from cudagsea_gb300 import api, synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("perms", [1, 151, 152, 303, 304, 305, 700])
+def test_same_scores_on_either_side_of_the_rule(gpu, perms):
+    d = synthetic.make(1200, 12, 30, perms, seed=perms, n_class_b=6, set_max=200)
+    out = []
+    for t in (None, dict(es_warps=32, es_stage=1), dict(es_warps=16, es_stage=1)):
+        p = api.Plan(1200, 12, 30, perms, "naive_diff_of_classes")
+        if t:
+            p.set_tuning(**t)
+        p.set_inputs(d.exprs, d.labels, d.set_offsets, d.set_genes)
+        p.execute()
+        out.append(p.read()[0])
+        p.close()
+    assert out[0].tobytes() == out[1].tobytes() == out[2].tobytes()
+
+
+def test_few_permutations_are_not_slower(gpu):
+    d = synthetic.make(1000, 12, 200, 130, seed=4, n_class_b=6, set_max=500)
+    p = api.Plan(1000, 12, 200, 130, "naive_diff_of_classes")
+    p.set_inputs(d.exprs, d.labels, d.set_offsets, d.set_genes)
+    p.set_profiling(True)
+    best = []
+    for t in ({}, dict(es_warps=32, es_stage=1)):
+        p.set_tuning(**t)
+        ts = []
+        for _ in range(25):
+            p.execute()
+            ts.append(p.stage_times()["es"])
+        best.append(float(np.sort(ts)[:12].mean()))
+    p.close()
+    # 1.21 times as long with pairs of CTAs
+    assert best[0] < 1.12 * best[1], best
