@@ -308,7 +308,9 @@ sort_bucket_body(int bx, int gx, const T* __restrict__ keys, int G, int num_perm
                 c[j] = H[tid * BPT + j].y;
                 sum += c[j];
             }
-            if constexpr (REGS) {  // here the block waits for the scan
+            // here the block waits for the scan; up to 2,048 genes the rest costs
+            // no more than the look (15 us of 2,000 permutations of 1,000)
+            if constexpr (REGS && NT > 256) {
                 bool alike = false;
 #pragma unroll
                 for (int i = 0; i < NREG; i += 4) alike |= a[i] == a[i + 1];

@@ -322,8 +322,8 @@ cudaError_t launch_adaptive_counts(int K, const int32_t* active, AdaptiveCtl* ct
 // counts[k] = v for every set, and the decision record cleared (rounds = 1)
 cudaError_t launch_adaptive_reset(int K, int64_t v, int64_t* counts, AdaptiveCtl* ctl, cudaStream_t st);
 
-// Lets a kernel be launched with `smem` bytes of dynamic shared memory: every
-// launch sets the same limit, all the device allows, whatever it needs itself.
+// Lets a kernel be launched with `smem` bytes of dynamic shared memory: the
+// limit is only ever set to all the device allows, whatever the launch needs.
 // The limit belongs to the kernel and not to the launch: set to each launch's
 // own need, two host threads with plans of different sizes took it from under
 // each other, and a launch was refused.
@@ -332,7 +332,9 @@ inline cudaError_t allow_smem(void (*kern)(P...), size_t smem) {
     cudaFuncAttributes a;
     int dev = 0, most = 0;
     cudaError_t e = cudaFuncGetAttributes(&a, kern);
-    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (a.maxDynamicSharedSizeBytes >= 0 && smem <= (size_t)a.maxDynamicSharedSizeBytes) return cudaSuccess;
+    e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
     const int room = most - (int)a.sharedSizeBytes;
