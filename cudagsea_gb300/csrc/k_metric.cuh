@@ -678,15 +678,19 @@ int metric_warps(int64_t units, int64_t groups, int S) {
     return w;
 }
 
-// Rounds of a warp: as tuned, but where the tile stays in shared memory as
-// many as leave four waves of blocks (2,000 genes x 40 samples x 1,024
-// permutations: the copies and their latency once per block, not per round).
+// Rounds of a warp: as tuned, but in fp32 where the tile stays in shared memory
+// two, if that leaves some sixteen blocks an SM: the copies once for both.  More
+// rounds make long blocks and an uneven end: onepass T test, 7,411 genes x 57 x
+// 2,000, 1, 2, 4, 8 rounds 159, 153, 158, 169 us; two-pass signal to noise, 20,000
+// x 40 x 1,000, 245, 237, 252, 271; log2 ratio, 60,963 x 16 x 338, 130, 133, 140, 155.
+// fp64 waits for its pipe and not for the copies: difference of classes, 20,000 x
+// 60 x 400, 1,196, 1,254, 1,338, 1,426.
 template <int ACC, class T>
 int metric_rounds(int64_t tiles, int64_t num_perms, int S, int tuned) {
-    if (S > 2 * kChunk) return tuned;
+    if (sizeof(T) == 8 || S > 2 * kChunk) return tuned;
     const int64_t blocks = tiles * num_perms / (metric_q<T>() * kMaxWarps);
     const int64_t r = blocks / (16 * (int64_t)metric_sms());
-    return r < tuned ? tuned : r > 16 ? 16 : (int)r;
+    return r < tuned ? tuned : r > 2 ? 2 : (int)r;
 }
 
 template <int ACC, class T>
