@@ -455,10 +455,14 @@ __device__ __noinline__ double set_score_positions_f64(const uint32_t* bmw, int 
 }
 
 // fp64, direct procedure: the walk in fp32, to find the hit the score is
-// taken at.  The fp32 candidates are off by less than 1e-6 (weights, their
-// sum, its reciprocal, the decay and the candidate itself, each rounded to
-// fp32, values at most 1 and the prefix compensated), so an extremum ahead of
-// every other candidate by kMargin is the extremum.  Returns the rank of the
+// taken at; no fp32 value enters the score.  A candidate here is off by less
+// than 10 roundings of 2^-24, 6e-7: of the weights, their compensated sum, its
+// reciprocal (two), the product, the decay, the misses times it, their sum and
+// the shift by the lanes before, of values at most 1.  An extremum ahead of
+// every other candidate by kMargin, three times what two of them can be off, is
+// the extremum.  The scores are as exact as those of the walk in double, or more
+// so, having fewer roundings: against 128-bit sums over 2,000 to 60,000 genes
+// 5.0e-17 rms and 2.4e-16 at most, 7.4e-17 and 3.4e-16 walked in double.  Returns the rank of the
 // hit (the largest value: after it, the smallest: before it), or -1 where the
 // lead is smaller, the end of the list would win, or the weights are outside
 // fp32's range.  `wf(r4)`: the weight at rank r4 / 4 as a float.

@@ -56,3 +56,28 @@ def test_nan_weights_cost_no_walk_in_double(gpu):
     plain, some = es_us(absent(20000, 304, 0.0, K=300)), es_us(absent(20000, 304, 0.05, K=300))
     # walked twice in double it took 2.9 times as long
     assert some < 1.5 * plain, (some, plain)
+
+
+@pytest.mark.parametrize("G", [64, 400, 6000, 20000, 50000])
+def test_leads_around_the_margin_of_the_search(gpu, G):
+    """Members at equal steps and weights that fall slowly: the running sum is
+    flat around its extremum, and the leads of neighbouring hits pass from far
+    above to far below what the walk in fp32 can tell.  The wrong hit would show
+    in the score, which is held to the tolerance of double sums."""
+    for slope in (1e-1, 1e-2, 1e-3, 1e-4, 1e-5, 1e-6, 1e-7):
+        sets = [np.arange(a, G, step) for step in (2, 3, 7) for a in (0, step - 1)]
+        sets.append(np.r_[np.arange(0, G // 2, 3), np.arange(G // 2, G, 5)])
+        d = synthetic.make(G, 2, 1, 3, seed=1, n_class_b=1, set_min=1, set_max=1)
+        keys = 1.0 + slope * np.linspace(0.5, -0.5, G) * (1 + 0.01 * np.sin(np.arange(G)))
+        x = np.zeros((2, G))
+        x[d.labels == 0] = keys  # one sample a class: the metric is its value
+        d.exprs = x
+        d.set_offsets = np.r_[0, np.cumsum([s.size for s in sets])].astype(np.int64)
+        d.set_genes = np.concatenate(sets).astype(np.int32)
+        r = run_plan(d, "naive_diff_of_classes", double=True)
+        sk, order = check_sort(r["keys"], r["order"], r["ranks"], r["sorted"])
+        es_o = oracle.es(sk, order, d.set_offsets, d.set_genes)
+        same = H.es_close(r["es"], es_o, True) | H.es_close(r["es"], -es_o, True) & (
+            np.abs(es_o) < 1e-9)  # both signs where the score is a rounding error
+        assert same.all(), (slope, r["es"][~same][:3], es_o[~same][:3])
+        r["plan"].close()
