@@ -832,10 +832,11 @@ int gsea_run(const gsea_config* cfg, const void* exprs, const uint8_t* labels, c
     gsea_plan p = nullptr;
     int rc = validate_config(cfg);
     if (rc) return rc;
-    // room for the sets with the plan's other buffers, if the offsets are in
-    // order (upload_sets refuses them otherwise)
+    // room for the sets with the plan's other buffers, if the call has all its
+    // arrays and the offsets are in order (what is refused after this is
+    // refused without their room)
     int64_t nnz = 0;
-    if (set_offsets && std::is_sorted(set_offsets, set_offsets + cfg->num_sets + 1) && set_offsets[0] == 0)
+    if (exprs && labels && set_genes && set_offsets && std::is_sorted(set_offsets, set_offsets + cfg->num_sets + 1) && set_offsets[0] == 0)
         nnz = set_offsets[cfg->num_sets];
     if ((rc = create_plan(cfg, nnz, &p))) return rc;
     p->use_graph = false;  // one pass: capturing it costs 110 us more than its launches

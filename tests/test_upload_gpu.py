@@ -63,3 +63,18 @@ def test_batch_instance_without_sets_is_refused(gpu, monkeypatch):
     ref, _ = api.gsea(large.exprs, large.labels, large.set_offsets, large.set_genes, 40, "naive_diff_of_classes")
     assert np.array_equal(es, ref)
     b.close()
+
+
+@pytest.mark.parametrize("missing", ["exprs", "labels", "set_genes"])
+def test_one_shot_refuses_missing_arrays_before_it_makes_room(gpu, missing):
+    """Offsets that ask for more than the device has, and an array missing: the
+    missing array is the answer, not the memory."""
+    small, _ = problems()
+    a = dict(exprs=np.ascontiguousarray(small.exprs, np.float32), labels=np.ascontiguousarray(small.labels, np.uint8),
+             set_offsets=np.ascontiguousarray(small.set_offsets, np.int64),
+             set_genes=np.ascontiguousarray(small.set_genes, np.int32))
+    a["set_offsets"][-1] = 1 << 40
+    a[missing] = None
+    args = [N.ptr(v) if v is not None else None for v in a.values()]
+    es = np.empty((8, 40), np.float32)
+    assert N.lib().gsea_run_f32(args[0], 600, 12, args[1], args[2], args[3], 8, 40, 0, 0, N.ptr(es), None, None) == 1
