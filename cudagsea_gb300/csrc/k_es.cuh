@@ -1109,15 +1109,18 @@ cudaError_t launch_es_t(const RankT* ranks, const T* sorted_abs, int G, int P, c
     // the other stages its permutation or waits for its last sets.  50 sets x
     // 1,024 permutations, 2,000 genes: 86 -> 82 us (passes in turn 128 -> 119),
     // 12,000 genes 88 -> 82; 250 sets 287 -> 281, 300 sets 373 -> 373, 600 sets
-    // 367 -> 379.  Only with a permutation to each CTA: below that both halves
-    // stage the same ones (200 sets, 1,000 genes, 130 permutations 57 us with 32
-    // warps, 69 with pairs; 12,000 genes 41 and 49; 304 permutations the same).
+    // 367 -> 379.  With fewer permutations than SMs both halves stage the same
+    // ones (200 sets, 1,000 genes, 130 permutations 57 us with 32 warps, 69 with
+    // pairs; 12,000 genes 41 and 49; 152 permutations 57 and 59, 39 and 41): only
+    // where the sets are so few that the smaller CTAs, which run beside another
+    // pass's kernels, matter more (66 sets x 272, 3,551 genes, passes of several
+    // plans in turn: 52 us with 32 warps, 46 with pairs).
     if constexpr (pairs_up<T, 16, 1>()) {
         int all = 0, reserved = 0;
         cudaDeviceGetAttribute(&all, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
         cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
         const size_t pair = 2 * (es_smem_bytes<T, RankT, 16, 1>(G) + 64 + (size_t)reserved);
-        if (K <= 256 && P >= 2 * sms && !tune.warps && tune.stage < 0 && wpl < 40 && pair <= (size_t)all) GSEA_ES(16, 1);
+        if ((K <= 64 || (K <= 256 && P >= sms)) && !tune.warps && tune.stage < 0 && wpl < 40 && pair <= (size_t)all) GSEA_ES(16, 1);
     }
     for (int pass = 0; pass < 2; pass++)
     for (const Cand& c : cands) {

@@ -8,12 +8,13 @@ from cudagsea_gb300 import api, synthetic
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("perms", [1, 151, 152, 303, 304, 305, 700])
-def test_same_scores_on_either_side_of_the_rule(gpu, perms):
-    d = synthetic.make(1200, 12, 30, perms, seed=perms, n_class_b=6, set_max=200)
+@pytest.mark.parametrize("perms", [1, 151, 152, 153, 303, 305, 700])
+@pytest.mark.parametrize("K", [30, 64, 65])
+def test_same_scores_on_either_side_of_the_rule(gpu, perms, K):
+    d = synthetic.make(1200, 12, K, perms, seed=perms, n_class_b=6, set_max=200)
     out = []
     for t in (None, dict(es_warps=32, es_stage=1), dict(es_warps=16, es_stage=1)):
-        p = api.Plan(1200, 12, 30, perms, "naive_diff_of_classes")
+        p = api.Plan(1200, 12, K, perms, "naive_diff_of_classes")
         if t:
             p.set_tuning(**t)
         p.set_inputs(d.exprs, d.labels, d.set_offsets, d.set_genes)
