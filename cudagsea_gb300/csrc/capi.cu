@@ -475,8 +475,9 @@ int create_plan(const gsea_config* cfg, int64_t nnz, gsea_plan* out) {
     const size_t per_perm = (size_t)G * (2 * p->tsize + (p->ranks16 ? 2 : 4)) + 4 * (size_t)p->words;
     int64_t pb = cfg->perm_batch > 0 ? cfg->perm_batch : (int64_t)(kBatchBudget / per_perm);
     if (pb < 1) pb = 1;
-    // the metric kernels' second grid dimension is one block per 4 or 8
-    // permutations of a batch and may not exceed 65,535
+    // the metric kernels' second grid dimension, at most 65,535 blocks, is the
+    // batch's groups of two (fp32) or four permutations by the warps of a block:
+    // two warps at least in the largest batch (metric_warps)
     constexpr int64_t kMaxBatch = (int64_t)4 * 65535;
     if (pb > kMaxBatch) pb = kMaxBatch;
     if (pb > P) pb = P;

@@ -45,7 +45,7 @@
 // double sums over the set's members.  Where fp32 cannot tell which hit (or
 // which sign) wins, the set is walked again in double throughout (20,000 genes,
 // 1,000 sets x 1,000 permutations: 7,978 us walked in double, where the FP64
-// pipe takes 80 cycles an instruction, 2,962 so, where it waits for the double
+// pipe takes 80 cycles an instruction, 2,890 so, where it waits for the double
 // weights, a sector each from L2).
 //
 // What bounds it: issue slots (1,000 sets x 1,000 permutations at 20,000

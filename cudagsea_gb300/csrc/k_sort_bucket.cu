@@ -53,8 +53,8 @@
 // L2) for each window.
 //
 // Measured (GB300, the sort stage, radix sorts before -> this): 1,000
-// permutations of 20,000 genes fp32 417 -> 204 us, fp64 1,724 -> 350 us; 300 x
-// 60,000 fp32 713 -> 297 us; 1,024 x 2,000 fp32 105 -> 32 us.  Issue slots and
+// permutations of 20,000 genes fp32 417 -> 197 us, fp64 1,724 -> 346 us; 300 x
+// 60,000 fp32 713 -> 287 us; 1,024 x 2,000 fp32 105 -> 32 us.  Issue slots and
 // the latency of shared memory between the barriers bound it (22 M warp
 // instructions per 152 permutations of 20,000 genes at 62% issue activity;
 // DRAM traffic is the keys once).

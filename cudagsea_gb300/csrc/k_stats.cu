@@ -151,15 +151,16 @@ __device__ __forceinline__ void stats_fwer_kernel_body(int bx, int K, int64_t P,
 }
 
 // ---------------------------------------------------------------------------
-// FDR counts, exact and O(K*P*log K).  Each side is handled as "key >= key*":
+// FDR counts, exact, O(K*P) but for a short search in a slot of the observed
+// keys (ObservedKeys).  Each side is handled as "key >= key*":
 // positive side keys are the scores themselves (observed NES >= 0, null
 // scores >= 0), negative side keys their negations (scores <= 0); a zero is on
 // both sides, NaN on neither.
 //   1. stats_fdr_obs_kernel: for every set, L = #{same-side observed keys <
 //      its key} and the observed count #{>= key}; the observed keys are
 //      scattered into ascending order at L + (#equal keys of lower index).
-//   2. stats_fdr_hist_kernel: every null score is binary-searched into the
-//      sorted observed keys of its side: t = #{observed keys <= it}, H[t]++.
+//   2. stats_fdr_hist_kernel: every null score is looked up among the sorted
+//      observed keys of its side: t = #{observed keys <= it}, counted in H[t].
 //   3. stats_fdr_suffix_kernel: S[i] = sum_{t >= i} H[t].
 //   4. stats_fdr_final_kernel: #{null keys >= key*} = S[L + 1] (a null key v
 //      satisfies v >= key* exactly when t(v) >= L + 1).

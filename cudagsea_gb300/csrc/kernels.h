@@ -19,7 +19,9 @@ template <class T>
 cudaError_t launch_metric(int metric, const T* exprs, int G, int S, const uint32_t* masks,
                           int words, int num_perms, int64_t nA, int64_t nB, T* keys,
                           const int* fast_ok, cudaStream_t st, int pb = 0);
-// (pb: permutations a warp takes, 4 or 8 in two rounds; 0 = 4)
+// (pb: groups of permutations a warp takes in turn, 4 (0) one, 8 two; a group is
+// two permutations in fp32, four in fp64.  fp32 with at most 64 samples takes two
+// of many permutations whatever was tuned)
 
 // Batched instances: one launch of the metric over every instance of a group
 // (blockIdx.z = instance), keys bit-identical to launch_metric's.  Instances

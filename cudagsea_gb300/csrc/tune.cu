@@ -6,7 +6,7 @@
 // enrichment_scores.cuh:218-256 launches 32 threads per permutation).
 //
 // Tunables (every choice computes identical results):
-//   metric      plain fp32 packed form: 4 or 8 permutations per thread;
+//   metric      plain form: one or two groups of permutations to a warp;
 //               tensor-core form: 128- or 256-permutation tiles (the GEMM's N)
 //   sort        bucket sort (with a radix sort behind it), the tiled radix sort,
 //               or the register-resident radix sort alone

@@ -262,7 +262,7 @@ int gsea_stats_device(const void* es, int64_t num_sets, int64_t num_perms, int p
  * memory is a fixed 4 MiB array inside the library, held by every GPU that
  * loads it; sizes whose scratch exceeds it are rejected with
  * GSEA_ERR_INVALID_ARGUMENT.  The scratch is sizeof(T)*(3K+2P) + 8*(4K+12)
- * + 320 bytes, plus the FDR histogram's per-block rows (up to 1 MiB:
+ * + 320 bytes, plus room that holds the FDR histogram (up to 1 MiB:
  * floor(2^20 / (4W)) * 4W + 16 bytes, W = 2K + 6) when K <= 6,142 (fp32) /
  * 4,095 (fp64); gsea_stats_scratch_bytes gives the exact figure.  The first
  * call on a device -- and the first after that device's context was reset
